@@ -99,6 +99,13 @@ static void set_derived_constants(GridDesc &g)
     g.c2f = (float)g.c2;
     g.igm1 = 1.0 / g.gm1;
     g.ig2 = 1.0 / (2 * g.gamma);
+    g.g16 = g.gamma / 16;
+    g.c1x8 = 8 * g.c1;
+    g.c2x16 = 16 * g.c2;
+    g.c1h = 0.5 * g.c1;
+    g.ggm1 = g.gamma * g.gm1;
+    g.gm1x2 = 2 * g.gm1;
+    g.ig4 = 1.0 / (4 * g.gamma);
     g.igm1f = (float)g.igm1;
     g.ig2f = (float)g.ig2;
     g.idx = 1.0 / g.dx;

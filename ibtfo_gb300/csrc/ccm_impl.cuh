@@ -117,8 +117,12 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
     }
     __syncthreads();
 
-    GasConst<T> K = (PREC == 2) ? GasConst<T>(g.gf, g.gm1f, g.c1f, g.c2f, g.igm1f, g.ig2f)
-                                : GasConst<T>(g.gamma, g.gm1, g.c1, g.c2, g.igm1, g.ig2);
+    const GasConst<T> K = [&] {
+        if constexpr (PREC == 2)
+            return GasConst<float>(g.gf, g.gm1f, g.c1f, g.c2f, g.igm1f, g.ig2f);
+        else
+            return GasConst<double>(g);
+    }();
     const T hx2 = s.sC[2], hy2 = s.sC[3];
     // X faces of the tile's rows (sF rows 1..TY; a warp reads one row of sU:
     // columns 0..TX-1 first, the last column after) and all Y faces
@@ -144,7 +148,10 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
             }
             const bool lo = low_order_cell(s.sT[r + 1][fc]) || low_order_cell(s.sT[r + 1][fc + 1]) ||
                             low_order_cell(s.sT[r + 1][fc + 2]) || low_order_cell(s.sT[r + 1][fc + 3]);
-            ccm_face<T, 1, SCH, RIE, LIM>(c0, c1, c2, c3, K, hx2, lo, f);
+            if constexpr (PREC == 2)
+                ccm_face<1, SCH, RIE, LIM>(c0, c1, c2, c3, K, hx2, lo, f);
+            else
+                ccm_face64<1, SCH, RIE, LIM>(c0, c1, c2, c3, K, hx2, lo, f);
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 s.sF[k][r][fc] = f[k];
@@ -163,7 +170,10 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
             }
             const bool lo = low_order_cell(s.sT[r][c + 2]) || low_order_cell(s.sT[r + 1][c + 2]) ||
                             low_order_cell(s.sT[r + 2][c + 2]) || low_order_cell(s.sT[r + 3][c + 2]);
-            ccm_face<T, 2, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, lo, f);
+            if constexpr (PREC == 2)
+                ccm_face<2, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, lo, f);
+            else
+                ccm_face64<2, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, lo, f);
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 s.sG[k][r][c] = f[k];
@@ -228,12 +238,13 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
                     const double x = s.sU[k][r + 2][c + 2] - lx * (s.sF[k][r + 1][c + 1] - s.sF[k][r + 1][c]);
                     v[k] = x - ly * (s.sG[k][r + 1][c] - s.sG[k][r][c]);
                 }
+                Cell64 cl = cell64(v);
                 if constexpr (safeguarded(RIE))
-                    pressure_floor(v);
+                    pressure_floor64(v, cl);
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     V[k * P + o] = v[k];
-                cell_stats_fast(v, K, g.dxdy, cs);
+                cell_stats_fast(v, cl, K, g.dxdy, cs);
             }
         }
         else if (i < g.ng + g.n_x && j < g.ng + g.n_y && t == CELL_CUT)
@@ -251,7 +262,10 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     Uc[k] = s.sU[k][r + 2][c + 2];
-                ccm_wall_flux<T, RIE>(Uc, (T)(nLx / L), (T)(nLy / L), K, Wt);
+                if constexpr (PREC == 2)
+                    ccm_wall_flux<RIE>(Uc, (T)(nLx / L), (T)(nLy / L), K, Wt);
+                else
+                    ccm_wall_flux64<RIE>(Uc, nLx / L, nLy / L, K, Wt);
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     W[k] = (double)Wt[k];
@@ -270,7 +284,10 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
             // is provisional (divided by a small alpha) until it is mixed
             if constexpr (safeguarded(RIE))
                 if (al >= 0.5)
-                    pressure_floor(v);
+                {
+                    Cell64 cl = cell64(v);
+                    pressure_floor64(v, cl);
+                }
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 state_st(Vd, k, o, v[k], g);

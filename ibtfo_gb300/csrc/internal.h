@@ -75,6 +75,8 @@ struct GridDesc
     // gas constants precomputed on the host (no per-thread divisions):
     // gamma - 1, (gamma+1)/(2 gamma), (gamma-1)/(2 gamma), and their FP32 copies
     double gm1, c1, c2, igm1, ig2; // ..., 1/(gamma - 1), 1/(2 gamma)
+    // gamma / 16, 8 c1, 16 c2, c1 / 2, gamma (gamma - 1), 2 (gamma - 1), 1/(4 gamma)
+    double g16, c1x8, c2x16, c1h, ggm1, gm1x2, ig4;
     float gf, gm1f, c1f, c2f, igm1f, ig2f;
     // 1/dx, 1/dy, dx*dy and FP32 copies of the reciprocals
     double idx, idy, dxdy;

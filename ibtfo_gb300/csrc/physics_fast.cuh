@@ -1,11 +1,12 @@
-// Physics with fewer floating-point instructions, templated on the
-// arithmetic type: T = double for the `fp64_fast` precision, T = float for
-// the FP32 compensated precision form.
+// Physics with fewer floating-point instructions, for the FP32 compensated
+// precision form (T = float), and what it shares with the fp64_fast form
+// (T = double), whose faces are in physics_fast64.cuh: the gas constants,
+// reciprocals, square roots, limiters and reconstruction.
 //
 // Same algorithm and branches as physics.cuh (the reference's), evaluated
 // with shared reciprocals, precomputed gamma constants, fused multiply-adds
-// (these units are compiled with contraction on) and the limiter's sign and
-// magnitude tests done on integer bit patterns.  For T = double the results
+// (these units are compiled with contraction on) and, in FP64, the limiter's
+// sign and magnitude tests done on integer bit patterns.  For T = double the results
 // differ from the reference in rounding only: relative differences of order
 // 1e-15 per step, inside the plain path's 1e-12 parity bar (checked by the GPU
 // parity tests for this precision).  Degenerate inputs (zero or non-finite
@@ -29,8 +30,26 @@ struct GasConst
     }
 };
 
-// 1/x: hardware seed + two Newton steps (within an ulp of the rounded value)
-__device__ __forceinline__ double rcp_t(double x)
+// FP64: with the multiples the faces of physics_fast64.cuh use
+template <>
+struct GasConst<double>
+{
+    double g, gm1, c1, c2, igm1, ig2;
+    double g16, c1x8, c2x16; // gamma / 16, 8 c1, 16 c2
+    double c1h, ggm1;        // c1 / 2, gamma (gamma - 1)
+    double gm1x2, ig4;       // 2 (gamma - 1), 1/(4 gamma)
+    template <typename G>
+    __device__ __forceinline__ explicit GasConst(const G &d)
+        : g(d.gamma), gm1(d.gm1), c1(d.c1), c2(d.c2), igm1(d.igm1), ig2(d.ig2), g16(d.g16), c1x8(d.c1x8),
+          c2x16(d.c2x16), c1h(d.c1h), ggm1(d.ggm1), gm1x2(d.gm1x2), ig4(d.ig4)
+    {
+    }
+};
+
+// 1/x of a double from the hardware estimate of the double's high word and
+// two Newton steps: four FP64 instructions (zero, subnormal, non-finite x,
+// results outside the normal range, and very small or large x)
+__device__ __forceinline__ double rcp_newton2(double x)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -38,6 +57,34 @@ __device__ __forceinline__ double rcp_t(double x)
     y = fma(y, e, y);
     e = fma(-x, y, 1.0);
     return fma(y, e, y);
+}
+// 1/x in two FP64 instructions, for a part whose FP64 pipe runs at 1/64 of
+// the FP32 one: the significand m = mh + ml (24 + 23 bits) as two floats, the
+// FP32 estimate y = 1/mh, its residual e = 1 - (mh + ml) y in FP32 (exact to
+// 2^-46), and y + y e put together as a double by integer arithmetic is 1/x to
+// about 2^-44; one Newton step in FP64 squares that.  Within an ulp of the
+// rounded value, as before; the FP64 faces went from 121 to 80 instructions
+// with this, sqrt_t and the flux form of physics_fast64.cuh.
+__device__ __forceinline__ double rcp_t(double x)
+{
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const unsigned ex = (unsigned)(hi >> 20) & 0x7ffu;
+    if (ex - 2u > 2040u)
+        return rcp_newton2(x);
+    const float mh = __int_as_float(0x3f800000 | ((hi << 3) & 0x007ffff8) | (int)(lo >> 29));
+    const float ml = __int_as_float(0x3f800000 | (int)((lo >> 6) & 0x007fffffu)) - 1.0f; // units of 2^-23
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(mh));
+    y = fminf(fmaxf(y, 0.5f), 1.0f); // one binade, so that the correction below is in its units
+    const float e = fmaf(ml * -0x1p-23f, y, fmaf(-mh, y, 1.0f));
+    const int n = __float2int_rn((y * e) * 0x1p52f); // |y e| < 2^-21
+    // y as a double of exponent 1023 - ex more, plus n units of 2^-52
+    const unsigned long long b = ((unsigned long long)(unsigned)__float_as_int(y) << 29) +
+                                 ((unsigned long long)(long long)(896 + 1023 - (int)ex) << 52) +
+                                 (unsigned long long)(2LL * n);
+    const double y0 = __longlong_as_double((long long)(b | ((unsigned long long)(hi & 0x80000000) << 32)));
+    return fma(y0, fma(-x, y0, 1.0), y0);
 }
 // FP32 form: hardware reciprocal seed + one Newton step (within ~1 ulp; no
 // correctly-rounded slow path), and the hardware square root approximation
@@ -49,14 +96,14 @@ __device__ __forceinline__ float rcp_t(float x)
     const float e = fmaf(-x, y, 1.0f);
     return fmaf(y, e, y);
 }
-// sqrt(x) for positive normal finite x from the hardware reciprocal square
-// root estimate y0 = (1 + e)/sqrt(x), |e| <= 2^-20 (measured on GB300): one
+// sqrt(x) of a double from the hardware reciprocal square root estimate
+// y0 = (1 + e)/sqrt(x), |e| <= 2^-20 (measured on GB300): one
 // Newton step folded into t = x y0 gives s0 = t (1 + r/2), r = 1 - x y0^2,
 // with relative error 1.5 e^2; one residual correction s1 = s0 + (y0/2)(x -
 // s0^2) leaves 1.5 e^3 (< 2^-59), so s1 is within about an ulp of sqrt(x).
 // Seven FP64 operations; zero, negative, subnormal and non-finite x take the
 // library square root.
-__device__ __forceinline__ double sqrt_t(double x)
+__device__ __forceinline__ double sqrt_newton2(double x)
 {
     const long long ix = __double_as_longlong(x);
     if (ix < 0x0010000000000000LL || ix >= 0x7ff0000000000000LL)
@@ -68,6 +115,33 @@ __device__ __forceinline__ double sqrt_t(double x)
     const double s0 = fma(0.5 * t, r, t);
     const double d = fma(-s0, s0, x);
     return fma(0.5 * y, d, s0);
+}
+// sqrt(x) in two FP64 instructions, as rcp_t: x = 4^k (mh + ml), mh in [1, 4);
+// with the FP32 estimate y = 1/sqrt(mh) and s = mh y, the FP32 residual
+// r = mh + ml - s^2 gives s + y r / 2 = sqrt(mh + ml) to about 2^-43, put
+// together as a double by integer arithmetic; the residual correction in
+// FP64 squares that (x far from the ends of the exponent range, so that
+// x - s^2 stays normal; others take the form above).
+__device__ __forceinline__ double sqrt_t(double x)
+{
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    if ((unsigned)(hi - (128 << 20)) >= (unsigned)(1790 << 20))
+        return sqrt_newton2(x);
+    const int E = (hi >> 20) - 1023, odd = E & 1, k = E >> 1;
+    const float mh = __int_as_float((0x3f800000 + (odd << 23)) | ((hi << 3) & 0x007ffff8) | (int)(lo >> 29));
+    const float ml = __int_as_float(0x3f800000 | (int)((lo >> 6) & 0x007fffffu)) - 1.0f; // units of 2^-23 (odd: 2^-22)
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(mh));
+    const float s = fminf(fmaxf(mh * y, 1.0f), 2.0f); // one binade
+    const float r = fmaf(ml, odd ? 0x1p-22f : 0x1p-23f, fmaf(-s, s, mh));
+    const int n = __float2int_rn((y * r) * 0x1p50f); // |y r / 2| < 2^-20, in units of 2^-51
+    const unsigned long long b = ((unsigned long long)(unsigned)__float_as_int(s) << 29) +
+                                 ((unsigned long long)(long long)(896 + k) << 52) + (unsigned long long)(2LL * n);
+    const double s0 = __longlong_as_double((long long)b);
+    const double h = __longlong_as_double((long long)(((unsigned long long)(unsigned)__float_as_int(y) << 29) +
+                                                      ((unsigned long long)(long long)(895 - k) << 52))); // ~ 1/(2 s0)
+    return fma(h, fma(-s0, s0, x), s0);
 }
 __device__ __forceinline__ float sqrt_t(float x)
 {
@@ -403,14 +477,6 @@ __device__ __forceinline__ bool pressure_floor_energy(const T U[4], T &E)
     return true;
 }
 
-template <typename T>
-__device__ __forceinline__ void pressure_floor(T U[4])
-{
-    T e;
-    if (pressure_floor_energy(U, e))
-        U[3] = e;
-}
-
 template <typename T, int SCH, int RIE, int LIM>
 __device__ __forceinline__ void x_face_fast(const T c0[4], const T c1[4], const T c2[4], const T c3[4],
                                             const GasConst<T> &K, T h2, T F[4])
@@ -422,9 +488,7 @@ __device__ __forceinline__ void x_face_fast(const T c0[4], const T c1[4], const 
     if constexpr (safeguarded(RIE))
         if (SCH != GODUNOV)
             positivity_fallback(c1, c2, UL, UR);
-    if constexpr (RIE == PVRS)
-        pvrs_x(UL, UR, (double)K.g, F); // double only (FP32 form rejects PVRS)
-    else if constexpr (RIE == SW)
+    if constexpr (RIE == SW)
         sw_fast<T, 1>(UL, UR, K, F);
     else if constexpr (RIE == HLLCT)
         hllc_toro<T, 1>(UL, UR, K, F);
@@ -436,7 +500,7 @@ __device__ __forceinline__ void x_face_fast(const T c0[4], const T c1[4], const 
 
 template <typename T, int SCH, int RIE, int LIM>
 __device__ __forceinline__ int y_face_fast(const T c0[4], const T c1[4], const T c2[4], const T c3[4],
-                                           const GasConst<T> &K, T h2, T G[4], T *stray)
+                                           const GasConst<T> &K, T h2, T G[4])
 {
     T UD[4], UU[4];
     face_states_fast<T, SCH, LIM>(c0, c1, c2, c3, UD, UU);
@@ -445,9 +509,7 @@ __device__ __forceinline__ int y_face_fast(const T c0[4], const T c1[4], const T
     if constexpr (safeguarded(RIE))
         if (SCH != GODUNOV)
             positivity_fallback(c1, c2, UD, UU);
-    if constexpr (RIE == PVRS)
-        return pvrs_y(UD, UU, (double)K.g, G, stray);
-    else if constexpr (RIE == SW)
+    if constexpr (RIE == SW)
     {
         sw_fast<T, 2>(UD, UU, K, G);
         return 0;
@@ -489,10 +551,11 @@ __device__ __forceinline__ void ccm_solve(const T UL[4], const T UR[4], const Ga
 // across it.  first_order: a stencil cell is cut or solid, so the face takes
 // the two cell averages (no slopes, no predictor); a reconstructed pair that
 // is not physical also falls back to the cell averages (positivity_fallback).
-template <typename T, int NRM, int SCH, int RIE, int LIM>
-__device__ __forceinline__ void ccm_face(const T c0[4], const T c1[4], const T c2[4], const T c3[4],
-                                         const GasConst<T> &K, T h2, bool first_order, T F[4])
+template <int NRM, int SCH, int RIE, int LIM>
+__device__ __forceinline__ void ccm_face(const float c0[4], const float c1[4], const float c2[4], const float c3[4],
+                                         const GasConst<float> &K, float h2, bool first_order, float F[4])
 {
+    using T = float;
     T UL[4], UR[4];
     if (first_order || SCH == GODUNOV)
     {
@@ -518,9 +581,10 @@ __device__ __forceinline__ void ccm_face(const T c0[4], const T c1[4], const T c
 // reversed), solved in the wall's frame.  Only its normal-momentum flux (the
 // wall pressure p_w) is kept: W = (0, p_w nx, p_w ny, 0), so no mass, energy
 // or tangential momentum crosses the wall whichever branch the solver takes.
-template <typename T, int RIE>
-__device__ __forceinline__ void ccm_wall_flux(const T U[4], T nx, T ny, const GasConst<T> &K, T W[4])
+template <int RIE>
+__device__ __forceinline__ void ccm_wall_flux(const float U[4], float nx, float ny, const GasConst<float> &K, float W[4])
 {
+    using T = float;
     const T mn = U[1] * nx + U[2] * ny, mt = -U[1] * ny + U[2] * nx;
     const T UL[4] = {U[0], mn, mt, U[3]};
     const T UR[4] = {U[0], -mn, mt, U[3]};

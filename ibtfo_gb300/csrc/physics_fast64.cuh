@@ -1,0 +1,396 @@
+// The fp64_fast faces: the algorithms of physics_fast.cuh in the fewest FP64
+// instructions.
+//
+// What bounds the FP64 sweeps is the FP64 pipe (two thread instructions per
+// SM and clock, one sixty-fourth of the FP32 rate), so an FP64 instruction
+// costs as much as 64 integer or FP32 ones.  Three things follow:
+//   * reciprocals and square roots start from a 44-bit estimate made on the
+//     FP32 and integer pipes (rcp_t, sqrt_t in physics_fast.cuh) and need two
+//     FP64 instructions each;
+//   * comparisons and the positivity tests read bit patterns;
+//   * the fluxes are written so that no full flux of either side is formed:
+//     with S_L = u_L - c_L and S_R = u_R + c_R the HLL flux is
+//       F = w_L (F_L - S_L U_L) + w_R (F_R - S_R U_R),
+//       F_K - S_K U_K = (u_K - S_K) U_K + p_K (0, 1, 0, u_K),
+//     where u_K - S_K is the root c_K just taken (20 instructions instead of
+//     32), and Steger-Warming's sums over the three waves are regrouped
+//     around T = 2 (gamma - 1) l1 + l3 + l4 (41 per state instead of 77).
+// Instructions per MUSCL + minmod face, reconstruction included: HLL 80
+// (121 before), Steger-Warming 102 (200 before), HLL_Toro 83 (about 165
+// before: the positivity test repeated four reciprocals).
+// Measured on GB300, ms per step: see the dispatch in capi.cu and the sweep
+// kernels of sweep_impl.cuh.
+#pragma once
+
+#include "physics_fast.cuh"
+
+namespace ibtfo {
+
+// x >= 0 and x <= 0 as IEEE comparisons give them (false for NaN), on the integer pipe
+__device__ __forceinline__ bool ge0(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return (b >= 0 && b <= 0x7ff0000000000000LL) || b == (long long)0x8000000000000000ULL;
+}
+__device__ __forceinline__ bool le0(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b == 0 || (b < 0 && b <= (long long)0xfff0000000000000ULL);
+}
+
+// a state with its primitive variables across a face of normal NRM
+struct Prim64
+{
+    double r, ir, mn, mt, E, un, ei, p; // ei = E - rho (u^2 + v^2) / 2, p = (gamma - 1) ei
+};
+
+template <int NRM>
+__device__ __forceinline__ Prim64 prim64(const double U[4], const GasConst<double> &K)
+{
+    Prim64 s;
+    s.r = U[0];
+    s.mn = U[NRM];
+    s.mt = U[3 - NRM];
+    s.E = U[3];
+    s.ir = rcp_t(s.r);
+    s.un = s.mn * s.ir;
+    s.ei = fma(-0.5, fma(s.mn, s.un, s.mt * (s.mt * s.ir)), s.E);
+    s.p = K.gm1 * s.ei;
+    return s;
+}
+
+// flux of one state normal to the face; m_t u_n is the tangential momentum flux
+template <int NRM>
+__device__ __forceinline__ void flux64(const Prim64 &s, double F[4])
+{
+    F[0] = s.mn;
+    F[NRM] = fma(s.mn, s.un, s.p);
+    F[3 - NRM] = s.mt * s.un;
+    F[3] = (s.E + s.p) * s.un;
+}
+
+// The HLL combination (header) of two states with wave speeds S_L = u_L - cL
+// and S_R = u_R + cR
+template <int NRM>
+__device__ __forceinline__ void hll_combine64(const Prim64 &L, const Prim64 &R, double cL, double cR, double S_L,
+                                              double S_R, double F[4])
+{
+    if (ge0(S_L))
+        flux64<NRM>(L, F);
+    else if (le0(S_R))
+        flux64<NRM>(R, F);
+    else
+    {
+        const double inv = rcp_t(S_R - S_L);
+        const double wl = S_R * inv, wr = S_L * inv; // w_L and -w_R
+        const double A = wl * cL, B = wr * cR, Pl = wl * L.p, Pr = wr * R.p;
+        F[0] = fma(A, L.r, B * R.r);
+        F[NRM] = fma(A, L.mn, fma(B, R.mn, Pl - Pr));
+        F[3 - NRM] = fma(A, L.mt, B * R.mt);
+        F[3] = fma(A, L.E, fma(B, R.E, fma(Pl, L.un, -(Pr * R.un))));
+    }
+}
+
+// HLL face flux (HLL/Riemann_solver.cpp:131-169 X, :202-235 Y).  For Y,
+// returns false when S_D >= 0 (the reference keeps the X-face flux).
+// With q_K = gamma / (16 rho_K), a_K / 4 = sqrt(q_K p_K) and
+// W = 2 p* = p_L + p_R + (u_L - u_R) (rho_L + rho_R) (a_L + a_R) / 4:
+// c_K = sqrt((gamma / rho_K) (c1 p* + c2 p_K)) = sqrt(q_K (8 c1 W + 16 c2 p_K)).
+template <int NRM>
+__device__ __forceinline__ bool hll64(const double UL[4], const double UR[4], const GasConst<double> &K, double F[4])
+{
+    const Prim64 L = prim64<NRM>(UL, K), R = prim64<NRM>(UR, K);
+    const double qL = K.g16 * L.ir, qR = K.g16 * R.ir;
+    const double W = fma(L.un - R.un, (L.r + R.r) * (sqrt_t(qL * L.p) + sqrt_t(qR * R.p)), L.p + R.p);
+    const double t = K.c1x8 * W;
+    const double cL = sqrt_t(qL * fma(K.c2x16, L.p, t));
+    const double S_L = L.un - cL;
+    if (NRM == 2 && ge0(S_L))
+        return false;
+    const double cR = sqrt_t(qR * fma(K.c2x16, R.p, t));
+    hll_combine64<NRM>(L, R, cL, cR, S_L, R.un + cR, F);
+    return true;
+}
+
+// w > 2 p for w >= 0 (false where either is NaN): doubles of one sign order
+// like their bits, and doubling a normal number adds one to its exponent
+__device__ __forceinline__ bool exceeds_twice(double w, double p)
+{
+    const long long bw = __double_as_longlong(w), bp = __double_as_longlong(p);
+    return bw > bp + 0x0010000000000000LL;
+}
+
+// HLL with Toro's wave-speed estimates (hll_plain: p* >= 0, q_K = 1 for p* <= p_K)
+template <int NRM>
+__device__ __forceinline__ void hll_toro64(const Prim64 &L, const Prim64 &R, const GasConst<double> &K, double F[4])
+{
+    const double gL = K.g * L.ir, gR = K.g * R.ir;
+    const double aL = sqrt_t(gL * L.p), aR = sqrt_t(gR * R.p);
+    double W = fma(0.25 * (L.un - R.un), (L.r + R.r) * (aL + aR), L.p + R.p); // 2 p*
+    const long long bw = __double_as_longlong(W);
+    W = (bw > 0 && bw <= 0x7ff0000000000000LL) ? W : 0.0;
+    const double t = K.c1h * W;
+    double cL = aL, cR = aR;
+    if (exceeds_twice(W, L.p))
+        cL = sqrt_t(gL * fma(K.c2, L.p, t));
+    if (exceeds_twice(W, R.p))
+        cR = sqrt_t(gR * fma(K.c2, R.p, t));
+    hll_combine64<NRM>(L, R, cL, cR, L.un - cL, R.un + cR, F);
+}
+
+// Contact-restoring HLLC with Toro's wave speeds (hllc_toro), from the primitive variables
+template <int NRM>
+__device__ __forceinline__ void hllc_toro64(const Prim64 &L, const Prim64 &R, const GasConst<double> &K, double F[4])
+{
+    const double gL = K.g * L.ir, gR = K.g * R.ir;
+    const double aL = sqrt_t(gL * L.p), aR = sqrt_t(gR * R.p);
+    double W = fma(0.25 * (L.un - R.un), (L.r + R.r) * (aL + aR), L.p + R.p);
+    const long long bw = __double_as_longlong(W);
+    W = (bw > 0 && bw <= 0x7ff0000000000000LL) ? W : 0.0;
+    const double t = K.c1h * W;
+    double cL = aL, cR = aR;
+    if (exceeds_twice(W, L.p))
+        cL = sqrt_t(gL * fma(K.c2, L.p, t));
+    if (exceeds_twice(W, R.p))
+        cR = sqrt_t(gR * fma(K.c2, R.p, t));
+    const double S_L = L.un - cL, S_R = R.un + cR;
+    if (ge0(S_L))
+    {
+        flux64<NRM>(L, F);
+        return;
+    }
+    if (le0(S_R))
+    {
+        flux64<NRM>(R, F);
+        return;
+    }
+    // rho_K (S_K - u_K): -rho_L c_L and rho_R c_R
+    const double mL = L.r * (S_L - L.un), mR = R.r * (S_R - R.un);
+    const double S_s = (R.p - L.p + L.un * mL - R.un * mR) * rcp_t(mL - mR);
+    const bool left = ge0(S_s);
+    const Prim64 s = left ? L : R;
+    const double S = left ? S_L : S_R, m = left ? mL : mR;
+    const double fac = m * rcp_t(S - S_s);
+    double Fk[4];
+    flux64<NRM>(s, Fk);
+    F[0] = Fk[0] + S * (fac - s.r);
+    F[NRM] = Fk[NRM] + S * (fac * S_s - s.mn);
+    F[3 - NRM] = Fk[3 - NRM] + S * (fac * (s.mt * s.ir) - s.mt);
+    F[3] = Fk[3] + S * (fac * (s.E * s.ir + (S_s - s.un) * (S_s + s.p * rcp_t(m))) - s.E);
+}
+
+// One side of the Steger-Warming splitting (StegerWarming/Riemann_solver.cpp:
+// 173-234 X, :262-325 Y), added to F.  With L_k = lambda_k +- sqrt(lambda_k^2
+// + delta^2) (twice the reference's), T = 2 (gamma - 1) L1 + L3 + L4,
+// X = a (L4 - L3), w = rho / (4 gamma) and h - |u|^2 / 2 = a^2 / (gamma - 1):
+//   F = w (T, u_n T + X, u_t T, |u|^2 / 2 T + a^2 / (gamma - 1) (L3 + L4) + u_n X)
+template <int NRM, int SIGN>
+__device__ __forceinline__ void sw_split64(const double U[4], const GasConst<double> &K, double F[4])
+{
+    const double ir = rcp_t(U[0]);
+    const double un = U[NRM] * ir, ut = U[3 - NRM] * ir;
+    const double q2 = fma(un, un, ut * ut);          // |u|^2
+    const double e = fma(-0.5, q2, U[3] * ir);       // internal energy per unit mass
+    const double a2 = K.ggm1 * e, a = sqrt_t(a2);
+    const double d2 = 1e-12; // delta = 1e-6 (:193)
+    auto lam = [&](double x) {
+        const double r = sqrt_t(fma(x, x, d2));
+        return SIGN > 0 ? x + r : x - r;
+    };
+    const double l1 = lam(un), l3 = lam(un - a), l4 = lam(un + a);
+    const double s = l3 + l4, T = fma(K.gm1x2, l1, s), X = a * (l4 - l3);
+    const double w = K.ig4 * U[0];
+    const double wT = w * T, wX = w * X;
+    const double g2 = fma(0.5 * q2, wT, fma(un, wX, w * (s * (K.g * e))));
+    F[0] = (SIGN > 0) ? wT : F[0] + wT;
+    F[NRM] = (SIGN > 0) ? fma(un, wT, wX) : F[NRM] + fma(un, wT, wX);
+    F[3 - NRM] = (SIGN > 0) ? ut * wT : fma(ut, wT, F[3 - NRM]);
+    F[3] = (SIGN > 0) ? g2 : F[3] + g2;
+}
+
+// MHM predictor with h2 = dt / (2 h) (mhm_predict_fast)
+template <int NRM>
+__device__ __forceinline__ void mhm_predict64(double UL[4], double UR[4], const GasConst<double> &K, double h2)
+{
+    const Prim64 L = prim64<NRM>(UL, K), R = prim64<NRM>(UR, K);
+    double FL[4], FR[4];
+    flux64<NRM>(L, FL);
+    flux64<NRM>(R, FR);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+    {
+        const double d = FL[k] - FR[k];
+        UL[k] = fma(h2, d, UL[k]);
+        UR[k] = fma(h2, d, UR[k]);
+    }
+}
+
+// x > f |E| for a threshold f < 2^-(DROP + 0.1), settled on the high words
+// where x / |E| is well above it: a high word is a number's exponent and the
+// leading bits of its significand, so that a difference above -(DROP << 20)
+// means x / |E| > 2^-(DROP + 0.1); closer values are compared in FP64
+template <int DROP>
+__device__ __forceinline__ bool above_fraction(double x, double E, double f)
+{
+    const int hx = __double2hiint(x), hE = __double2hiint(E) & 0x7fffffff;
+    if (hx >= 0x00100000 && hx < 0x7ff00000 && hE < 0x7ff00000 && hx - hE >= -(DROP << 20))
+        return true;
+    return x > f * fabs(E);
+}
+// positive density and an internal energy above 1e-6 E (physical())
+__device__ __forceinline__ bool physical64(const Prim64 &s)
+{
+    const long long b = __double_as_longlong(s.r);
+    return b > 0 && b <= 0x7ff0000000000000LL && above_fraction<18>(s.ei, s.E, 1e-6);
+}
+
+// velocity and internal energy of a cell's state
+struct Cell64
+{
+    double ir, u, v, ei;
+};
+__device__ __forceinline__ Cell64 cell64(const double U[4])
+{
+    Cell64 c;
+    c.ir = rcp_t(U[0]);
+    c.u = U[1] * c.ir;
+    c.v = U[2] * c.ir;
+    c.ei = fma(-0.5, fma(U[1], c.u, U[2] * c.v), U[3]);
+    return c;
+}
+
+// the pressure floor (pressure_floor_energy) of an updated cell: raises U[3]
+// and c.ei where the internal energy is below 1e-5 E
+__device__ __forceinline__ void pressure_floor64(double U[4], Cell64 &c)
+{
+    if (above_fraction<15>(c.ei, U[3], 1e-5) || !(U[0] > 0.0))
+        return;
+    const double f = 1e-5 * fabs(U[3]);
+    if (c.ei >= f)
+        return;
+    U[3] = (U[3] - c.ei) + f;
+    c.ei = f;
+}
+
+// The primitive variables of a face's pair; a pair that is not physical
+// between two cells that are takes the two cell averages
+// (positivity_fallback).  The cells are looked at only then.
+template <int NRM, bool SAFE>
+__device__ __forceinline__ void face_prims64(const double c1[4], const double c2[4], const double UL[4],
+                                             const double UR[4], const GasConst<double> &K, Prim64 &L, Prim64 &R)
+{
+    L = prim64<NRM>(UL, K);
+    R = prim64<NRM>(UR, K);
+    if (SAFE && !(physical64(L) && physical64(R)))
+    {
+        const Prim64 a = prim64<NRM>(c1, K), b = prim64<NRM>(c2, K);
+        if (physical64(a) && physical64(b))
+        {
+            L = a;
+            R = b;
+        }
+    }
+}
+
+// The flux from the pair (UL, UR) of a face between cells c1 and c2; false:
+// the Y face keeps its slot's X-face flux (HLL only).  SAFE: the positivity
+// fallback applies (the Toro keys, and every cut-cell solver).
+template <int NRM, int RIE, bool SAFE>
+__device__ __forceinline__ bool solve64(const double c1[4], const double c2[4], double UL[4], double UR[4],
+                                        const GasConst<double> &K, double F[4])
+{
+    if constexpr (RIE == SW)
+    {
+        if (SAFE)
+        {
+            Prim64 L = prim64<NRM>(UL, K), R = prim64<NRM>(UR, K);
+            if (!(physical64(L) && physical64(R)))
+            {
+                L = prim64<NRM>(c1, K), R = prim64<NRM>(c2, K);
+                if (physical64(L) && physical64(R))
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        UL[k] = c1[k], UR[k] = c2[k];
+            }
+        }
+        sw_split64<NRM, 1>(UL, K, F);
+        sw_split64<NRM, -1>(UR, K, F);
+        return true;
+    }
+    else if constexpr (RIE == HLLT || RIE == HLLCT)
+    {
+        Prim64 L, R;
+        face_prims64<NRM, SAFE>(c1, c2, UL, UR, K, L, R);
+        if constexpr (RIE == HLLT)
+            hll_toro64<NRM>(L, R, K, F);
+        else
+            hllc_toro64<NRM>(L, R, K, F);
+        return true;
+    }
+    else
+        return hll64<NRM>(UL, UR, K, F);
+}
+
+// One face of the FP64 sweeps, normal NRM; returns the components of a Y face
+// that keep the X-face flux of its slot (HLL: all, PVRS: the energy, whose
+// stray value *stray receives)
+template <int SCH, int RIE, int LIM, int NRM>
+__device__ __forceinline__ int face64(const double c0[4], const double c1[4], const double c2[4], const double c3[4],
+                                      const GasConst<double> &K, double h2, double F[4], double *stray)
+{
+    double UL[4], UR[4];
+    face_states_fast<double, SCH, LIM>(c0, c1, c2, c3, UL, UR);
+    if (SCH == MHM)
+        mhm_predict64<NRM>(UL, UR, K, h2);
+    if constexpr (RIE == PVRS)
+    {
+        if (NRM == 2)
+            return pvrs_y(UL, UR, K.g, F, stray);
+        pvrs_x(UL, UR, K.g, F);
+        return 0;
+    }
+    else
+        return solve64<NRM, RIE, safeguarded(RIE) && SCH != GODUNOV>(c1, c2, UL, UR, K, F) ? 0 : 0xF;
+}
+
+// One face of the FP64 cut-cell sweeps (ccm_face)
+template <int NRM, int SCH, int RIE, int LIM>
+__device__ __forceinline__ void ccm_face64(const double c0[4], const double c1[4], const double c2[4],
+                                           const double c3[4], const GasConst<double> &K, double h2, bool first_order,
+                                           double F[4])
+{
+    double UL[4], UR[4];
+    if (first_order || SCH == GODUNOV)
+    {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+        {
+            UL[k] = c1[k];
+            UR[k] = c2[k];
+        }
+    }
+    else
+    {
+        face_states_fast<double, SCH, LIM>(c0, c1, c2, c3, UL, UR);
+        if (SCH == MHM)
+            mhm_predict64<NRM>(UL, UR, K, h2);
+    }
+    // first-order pairs are the cell averages: the fallback changes nothing there
+    solve64<NRM, RIE, SCH != GODUNOV>(c1, c2, UL, UR, K, F);
+}
+
+// The wall flux of the FP64 cut-cell sweeps (ccm_wall_flux)
+template <int RIE>
+__device__ __forceinline__ void ccm_wall_flux64(const double U[4], double nx, double ny, const GasConst<double> &K,
+                                                double W[4])
+{
+    const double mn = U[1] * nx + U[2] * ny, mt = -U[1] * ny + U[2] * nx;
+    double UL[4] = {U[0], mn, mt, U[3]}, UR[4] = {U[0], -mn, mt, U[3]}, F[4];
+    solve64<1, RIE, false>(UL, UR, UL, UR, K, F);
+    W[0] = 0.0;
+    W[1] = F[1] * nx;
+    W[2] = F[1] * ny;
+    W[3] = 0.0;
+}
+
+} // namespace ibtfo

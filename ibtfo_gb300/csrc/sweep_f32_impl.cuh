@@ -190,8 +190,7 @@ __device__ __forceinline__ void sweep_tile32(SweepSmem32<TX, TY> &s, const GridD
                 c2[k] = s.sU[k][r + 2][c + 2];
                 c3[k] = s.sU[k][r + 3][c + 2];
             }
-            float stray = 0.0f;
-            int keep = y_face_fast<float, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, f, &stray);
+            int keep = y_face_fast<float, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, f);
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 s.sG[k][r][c] = f[k];

@@ -22,7 +22,7 @@
 
 #include "internal.h"
 #include "physics.cuh"
-#include "physics_fast.cuh"
+#include "physics_fast64.cuh"
 #include "tile_faces.cuh"
 #include "tma.cuh"
 
@@ -239,16 +239,13 @@ __device__ __forceinline__ void cell_stats(const double v[4], double gam, double
     cs.nans += any_nan4(v);
 }
 
-// the same statistics with a shared reciprocal (fp64_fast)
-__device__ __forceinline__ void cell_stats_fast(const double v[4], const GasConst<double> &K, double dxdy,
-                                                CellStats &cs)
+// the same statistics from the cell's velocity and internal energy (fp64_fast)
+__device__ __forceinline__ void cell_stats_fast(const double v[4], const Cell64 &c, const GasConst<double> &K,
+                                                double dxdy, CellStats &cs)
 {
-    const double ir = rcp_t(v[0]);
-    const double u = v[1] * ir, w = v[2] * ir;
-    const double p = K.gm1 * fma(-0.5, fma(v[1], u, v[2] * w), v[3]);
-    cs.a2max = max_nonneg(cs.a2max, K.g * ir * p);
-    cs.umax = max_nonneg(cs.umax, fabs(u));
-    cs.vmax = max_nonneg(cs.vmax, fabs(w));
+    cs.a2max = max_nonneg(cs.a2max, K.ggm1 * (c.ir * c.ei));
+    cs.umax = max_nonneg(cs.umax, fabs(c.u));
+    cs.vmax = max_nonneg(cs.vmax, fabs(c.v));
     cs.mass += v[0] * dxdy;
     cs.nans += any_nan4(v);
 }
@@ -343,7 +340,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
     __syncthreads();
 
     const double gam = g.gamma;
-    const GasConst<double> K(gam, g.gm1, g.c1, g.c2, g.igm1, g.ig2);
+    const GasConst<double> K(g);
     const double hx2 = FASTPHYS ? s.sC[2] : 0.0, hy2 = FASTPHYS ? s.sC[3] : 0.0; // MHM predictor of physics_fast
     // X faces of the tile's rows (sF rows 1..TY) and all Y faces; the X faces
     // of the row below the tile (sF row 0) follow below, where needed
@@ -366,7 +363,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
                 c3[k] = s.sU[k][r + 1][fc + 3];
             }
             if (FASTPHYS)
-                x_face_fast<double, SCH, RIE, LIM>(c0, c1, c2, c3, K, hx2, f);
+                face64<SCH, RIE, LIM, 1>(c0, c1, c2, c3, K, hx2, f, nullptr);
             else
                 x_face<SCH, RIE, LIM>(c0, c1, c2, c3, gam, dt, g.dx, f);
 #pragma unroll
@@ -386,7 +383,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
                 c3[k] = s.sU[k][r + 3][c + 2];
             }
             double stray = 0.0;
-            int keep = FASTPHYS ? y_face_fast<double, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, f, &stray)
+            int keep = FASTPHYS ? face64<SCH, RIE, LIM, 2>(c0, c1, c2, c3, K, hy2, f, &stray)
                                 : y_face<SCH, RIE, LIM>(c0, c1, c2, c3, gam, dt, g.dy, f, &stray);
             if constexpr (RIE == PVRS)
             {
@@ -429,7 +426,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
             c3[k] = s.sU[k][r + 1][fc + 3];
         }
         if (FASTPHYS)
-            x_face_fast<double, SCH, RIE, LIM>(c0, c1, c2, c3, K, hx2, f);
+            face64<SCH, RIE, LIM, 1>(c0, c1, c2, c3, K, hx2, f, nullptr);
         else
             x_face<SCH, RIE, LIM>(c0, c1, c2, c3, gam, dt, g.dx, f);
 #pragma unroll
@@ -464,17 +461,25 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
                     v[k] = x - dt * (gp - gm) / g.dy;
                 }
             }
+            Cell64 cl;
+            if constexpr (FASTPHYS)
+                if (safeguarded(RIE) || stage == 0)
+                    cl = cell64(v);
             if constexpr (safeguarded(RIE))
-                pressure_floor(v);
+                pressure_floor64(v, cl);
             if (stage == 2)
+            {
                 rk2_average(V, (long long)j * pitch + i, P, v);
+                if constexpr (FAST)
+                    cl = cell64(v);
+            }
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 V[k * P + (long long)j * pitch + i] = v[k];
             if (stage == 1)
                 continue;
             if (FAST)
-                cell_stats_fast(v, K, g.dxdy, cs);
+                cell_stats_fast(v, cl, K, g.dxdy, cs);
             else
                 cell_stats(v, gam, g.dx, g.dy, cs);
         }
