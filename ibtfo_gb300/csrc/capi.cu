@@ -88,6 +88,22 @@ void set_last_error(const char *msg) { g_err = msg; }
             return cuda_fail(e_, #call);              \
     } while (0)
 
+// a divisor of the strict sweeps that the whole case shares
+static Divisor case_divisor(double b)
+{
+    Divisor d{};
+    uint64_t bits;
+    std::memcpy(&bits, &b, sizeof(bits));
+    d.b = b;
+    d.B = (bits & (SIG_HIDDEN - 1)) | SIG_HIDDEN;
+    d.Y = (uint64_t)(((unsigned __int128)1 << 114) / d.B);
+    d.sign = bits & (1ull << 63);
+    d.ex = (int)((bits >> 52) & 0x7ff);
+    if (d.ex == 0x7ff)
+        d.ex = 0;
+    return d;
+}
+
 static void set_derived_constants(GridDesc &g)
 {
     g.gm1 = g.gamma - 1;
@@ -106,6 +122,12 @@ static void set_derived_constants(GridDesc &g)
     g.ggm1 = g.gamma * g.gm1;
     g.gm1x2 = 2 * g.gm1;
     g.ig4 = 1.0 / (4 * g.gamma);
+    g.gp1 = g.gamma + 1;
+    g.hgm1g = (g.gamma - 1) / 2 / g.gamma;
+    g.by_g = case_divisor(g.gamma);
+    g.by_gm1 = case_divisor(g.gm1);
+    g.by_dx = case_divisor(g.dx);
+    g.by_dy = case_divisor(g.dy);
     g.igm1f = (float)g.igm1;
     g.ig2f = (float)g.ig2;
     g.idx = 1.0 / g.dx;

@@ -8,6 +8,8 @@
 #include <string>
 #include <vector>
 
+#include "int64math.cuh"
+
 namespace ibtfo {
 
 enum Boundary { BC_REGULAR = 0, BC_IDW = 1, BC_LINEAR = 2, BC_RIEMANNGFM = 3, BC_BCGFM = 4, BC_HBCGFM = 5, BC_CCM = 6 };
@@ -77,6 +79,9 @@ struct GridDesc
     double gm1, c1, c2, igm1, ig2; // ..., 1/(gamma - 1), 1/(2 gamma)
     // gamma / 16, 8 c1, 16 c2, c1 / 2, gamma (gamma - 1), 2 (gamma - 1), 1/(4 gamma)
     double g16, c1x8, c2x16, c1h, ggm1, gm1x2, ig4;
+    // gamma + 1 and (gamma - 1) / 2 / gamma as the reference evaluates them, and the divisors of the strict sweeps
+    double gp1, hgm1g;
+    Divisor by_g, by_gm1, by_dx, by_dy;
     float gf, gm1f, c1f, c2f, igm1f, ig2f;
     // 1/dx, 1/dy, dx*dy and FP32 copies of the reciprocals
     double idx, idy, dxdy;

@@ -11,6 +11,9 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "int64math.cuh"
+#include "internal.h"
+
 namespace ibtfo {
 
 enum Scheme { MUSCL = 0, MHM = 1, GODUNOV = 2, LAX = 3 };
@@ -20,8 +23,35 @@ enum Riemann { HLL = 0, HLLC = 1, PVRS = 2, SW = 3, HLLCT = 4, HLLT = 5 };
 constexpr bool safeguarded(int rie) { return rie == HLLCT || rie == HLLT; }
 enum Limiter { MINMOD = 0, VANLEER = 1 };
 
+// x >= 0 and x <= 0 as IEEE comparisons give them (false for NaN), on the integer pipe
+__device__ __forceinline__ bool ge0(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return (b >= 0 && b <= 0x7ff0000000000000LL) || b == (long long)0x8000000000000000ULL;
+}
+__device__ __forceinline__ bool le0(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b == 0 || (b < 0 && b <= (long long)0xfff0000000000000ULL);
+}
+
+// The bits of |x|, masked on the high word: masking a double's 64 bits at
+// once is taken for fabs, which is an FP64 addition on this part (12 of a
+// face's 24 additions, before).
+__device__ __forceinline__ long long magnitude_bits(double x)
+{
+    return ((long long)(__double2hiint(x) & 0x7fffffff) << 32) | (unsigned)__double2loint(x);
+}
+__device__ __forceinline__ double magnitude(double x)
+{
+    return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
+}
+
 // pow(x, 0.5): +0 for a zero of either sign (as pow gives), sqrt otherwise
-__device__ __forceinline__ double pow_half(double x) { return (x == 0.0) ? 0.0 : sqrt(x); }
+__device__ __forceinline__ double pow_half(double x)
+{
+    return (__double_as_longlong(x) << 1) == 0 ? 0.0 : sqrt_rn(x);
+}
 
 // Src/Base/Slope_limiter/minmod/Slope_limiter.H:4:
 //   ((a*b) > 0) ? ((a/b > 1) ? b : a) : 0
@@ -36,9 +66,9 @@ __device__ __forceinline__ double pow_half(double x) { return (x == 0.0) ? 0.0 :
 //   non-NaN doubles order like their bit patterns.
 __device__ __forceinline__ double lim_minmod(double a, double b)
 {
-    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    const long long ma = ia & 0x7fffffffffffffffLL, mb = ib & 0x7fffffffffffffffLL;
-    bool pos = ((ia ^ ib) >= 0) && ma != 0 && mb != 0 && ma <= 0x7ff0000000000000LL && mb <= 0x7ff0000000000000LL;
+    const long long ma = magnitude_bits(a), mb = magnitude_bits(b);
+    bool pos = ((__double2hiint(a) ^ __double2hiint(b)) >= 0) && ma != 0 && mb != 0 && ma <= 0x7ff0000000000000LL &&
+               mb <= 0x7ff0000000000000LL;
     if (pos)
     {
         const int ea = (int)(ma >> 52), eb = (int)(mb >> 52);
@@ -53,18 +83,22 @@ __device__ __forceinline__ double lim_minmod(double a, double b)
 __device__ __forceinline__ double lim_vanleer(double a, double P, double Q)
 {
     double b = P - Q;
-    double r = (a + 1e-7) / (b + 1e-7);
-    return (r > 0) ? ((r * r + r) * P - Q / (r * r + 1)) : 0.0;
+    double r = divide_rn(a + 1e-7, divisor(b + 1e-7));
+    return (r > 0) ? ((r * r + r) * P - divide_rn(Q, divisor(r * r + 1))) : 0.0;
 }
 
-// 0.5 * limiter(hi - lo, P - Q)
+// limiter(hi - lo, P - Q), and half of it
+template <int LIM>
+__device__ __forceinline__ double limited(double hi, double lo, double P, double Q)
+{
+    if (LIM == VANLEER)
+        return lim_vanleer(hi - lo, P, Q);
+    return lim_minmod(hi - lo, P - Q);
+}
 template <int LIM>
 __device__ __forceinline__ double half_slope(double hi, double lo, double P, double Q)
 {
-    double a = hi - lo;
-    if (LIM == VANLEER)
-        return 0.5 * lim_vanleer(a, P, Q);
-    return 0.5 * lim_minmod(a, P - Q);
+    return 0.5 * limited<LIM>(hi, lo, P, Q);
 }
 
 // Face states of one interface from the four cells c0..c3 along the sweep
@@ -85,8 +119,9 @@ __device__ __forceinline__ void face_states(const double c0[4], const double c1[
         }
         else
         {
-            UL[k] = c1[k] + half_slope<LIM>(c1[k], c0[k], c2[k], c1[k]);
-            UR[k] = c2[k] - half_slope<LIM>(c3[k], c2[k], c2[k], c1[k]);
+            // c +- RN(0.5 s): halving is exact, so one fused operation rounds as the two do
+            UL[k] = fma(0.5, limited<LIM>(c1[k], c0[k], c2[k], c1[k]), c1[k]);
+            UR[k] = fma(-0.5, limited<LIM>(c3[k], c2[k], c2[k], c1[k]), c2[k]);
         }
     }
 }
@@ -117,96 +152,91 @@ __device__ __forceinline__ void flux_y(const double U[4], double g, double G[4])
     G[3] = (U[3] + p) * v;
 }
 
+// The states of a face as the strict solvers use them: every quotient by rho
+// shares one reciprocal (divide_rn gives the IEEE quotient).  Conserve2FluxX /
+// Conserve2FluxY (Conserve2Flux.cpp:66-74, :101-109) evaluated from them.
+struct StrictPrim
+{
+    double rho, u, v, p, E;
+    Divisor by_rho;
+};
+__device__ __forceinline__ StrictPrim strict_prim(const double U[4], const GridDesc &g)
+{
+    StrictPrim s;
+    s.rho = U[0];
+    s.by_rho = divisor(U[0]);
+    s.u = divide_rn(U[1], s.by_rho);
+    s.v = divide_rn(U[2], s.by_rho);
+    s.E = U[3];
+    s.p = g.gm1 * (U[3] - 0.5 * s.rho * (s.u * s.u + s.v * s.v));
+    return s;
+}
+template <int NRM>
+__device__ __forceinline__ void strict_flux(const StrictPrim &s, double F[4])
+{
+    const double q = (NRM == 1) ? s.u : s.v;
+    F[0] = s.rho * q;
+    F[NRM] = s.rho * q * q + s.p;
+    F[3 - NRM] = s.rho * s.u * s.v;
+    F[3] = (s.E + s.p) * q;
+}
+
 // MHM half-step predictor on the two states of one interface,
 // MHM_Scheme.cpp:73-93 (X, h = dx) and :160-180 (Y, h = dy):
-// U += 0.5 * (F(U_L) - F(U_R)) * dt / h for both states.
-template <int YDIR>
-__device__ __forceinline__ void mhm_predict(double UL[4], double UR[4], double g, double dt, double h)
+// U += 0.5 * (F(U_L) - F(U_R)) * dt / h for both states (the halving commutes
+// with the roundings that follow it).
+template <int NRM>
+__device__ __forceinline__ void mhm_predict(double UL[4], double UR[4], const GridDesc &g, double dt)
 {
+    const Divisor &by_h = (NRM == 1) ? g.by_dx : g.by_dy;
     double FL[4], FR[4];
-    if (YDIR)
-    {
-        flux_y(UL, g, FL);
-        flux_y(UR, g, FR);
-    }
-    else
-    {
-        flux_x(UL, g, FL);
-        flux_x(UR, g, FR);
-    }
+    strict_flux<NRM>(strict_prim(UL, g), FL);
+    strict_flux<NRM>(strict_prim(UR, g), FR);
 #pragma unroll
     for (int k = 0; k < 4; k++)
     {
-        double d = 0.5 * (FL[k] - FR[k]) * dt / h;
-        UL[k] = UL[k] + d;
-        UR[k] = UR[k] + d;
+        const double q = divide_rn((FL[k] - FR[k]) * dt, by_h);
+        UL[k] = fma(0.5, q, UL[k]);
+        UR[k] = fma(0.5, q, UR[k]);
     }
 }
 
 // ----------------------------------------------------------------- HLL
 
-// HLL/Riemann_solver.cpp:131-169 (X).  Returns the face flux.
-__device__ __forceinline__ void hll_x(const double UL[4], const double UR[4], double g, double F[4])
+// HLL/Riemann_solver.cpp:131-169 (X), :202-235 (Y).  Y: returns false when
+// S_D >= 0 (the reference then stores nothing and the slot keeps the X-face
+// flux, :224-227).  The reference's halvings are exact and are moved past the
+// roundings they commute with:
+//   p_star = 0.5 (p_L + p_R) + 0.5 (u_L - u_R) (0.5 (rho_L + rho_R) 0.5 (a_L + a_R)),
+//   (g + 1) p_star / 2 / g / p_K + (g - 1) / 2 / g
+template <int NRM>
+__device__ __forceinline__ bool strict_hll(const double UL[4], const double UR[4], const GridDesc &g, double F[4])
 {
-    double rho_L = UL[0], rho_R = UR[0];
-    double u_L = UL[1] / rho_L;
-    double v_L = UL[2] / rho_L;
-    double p_L = (g - 1) * (UL[3] - 0.5 * rho_L * (u_L * u_L + v_L * v_L));
-    double u_R = UR[1] / rho_R;
-    double v_R = UR[2] / rho_R;
-    double p_R = (g - 1) * (UR[3] - 0.5 * rho_R * (u_R * u_R + v_R * v_R));
-    double a_L = pow_half(g * p_L / rho_L);
-    double a_R = pow_half(g * p_R / rho_R);
-    double rho_bar = 0.5 * (rho_L + rho_R);
-    double a_bar = 0.5 * (a_L + a_R);
-    double p_star = 0.5 * (p_L + p_R) + 0.5 * (u_L - u_R) * (rho_bar * a_bar);
-    double S_L = u_L - a_L * sqrt((g + 1) * p_star / 2 / g / p_L + (g - 1) / 2 / g);
-    double S_R = u_R + a_R * sqrt((g + 1) * p_star / 2 / g / p_R + (g - 1) / 2 / g);
-    double FL[4], FR[4];
-    flux_x(UL, g, FL);
-    flux_x(UR, g, FR);
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-    {
-        if (S_L >= 0)
-            F[k] = FL[k];
-        else if (S_R <= 0)
-            F[k] = FR[k];
-        else
-            F[k] = (S_R * FL[k] - S_L * FR[k] + S_R * S_L * (UR[k] - UL[k])) / (S_R - S_L);
-    }
-}
-
-// HLL/Riemann_solver.cpp:202-235 (Y).  Returns false when S_D >= 0: the
-// reference then stores nothing and the slot keeps the X-face flux (:224-227).
-__device__ __forceinline__ bool hll_y(const double UD[4], const double UU[4], double g, double G[4])
-{
-    double rho_U = UU[0], rho_D = UD[0];
-    double u_U = UU[1] / rho_U;
-    double v_U = UU[2] / rho_U;
-    double p_U = (g - 1) * (UU[3] - 0.5 * rho_U * (u_U * u_U + v_U * v_U));
-    double u_D = UD[1] / rho_D;
-    double v_D = UD[2] / rho_D;
-    double p_D = (g - 1) * (UD[3] - 0.5 * rho_D * (u_D * u_D + v_D * v_D));
-    double a_U = pow_half(g * p_U / rho_U);
-    double a_D = pow_half(g * p_D / rho_D);
-    double rho_bar = 0.5 * (rho_U + rho_D);
-    double a_bar = 0.5 * (a_U + a_D);
-    double p_star = 0.5 * (p_U + p_D) + 0.5 * (v_D - v_U) * (rho_bar * a_bar);
-    double S_D = v_D - a_D * sqrt((g + 1) * p_star / 2 / g / p_D + (g - 1) / 2 / g);
-    double S_U = v_U + a_U * sqrt((g + 1) * p_star / 2 / g / p_U + (g - 1) / 2 / g);
-    if (S_D >= 0)
+    const StrictPrim L = strict_prim(UL, g), R = strict_prim(UR, g);
+    const double qL = (NRM == 1) ? L.u : L.v, qR = (NRM == 1) ? R.u : R.v;
+    const double aL = pow_half(divide_rn(g.gamma * L.p, L.by_rho));
+    const double aR = pow_half(divide_rn(g.gamma * R.p, R.by_rho));
+    const double z = (qL - qR) * ((L.rho + R.rho) * (aL + aR));
+    const double p_star = fma(0.125, z, 0.5 * (L.p + R.p));
+    const double t = divide_rn(g.gp1 * p_star, g.by_g);
+    const double S_L = qL - aL * sqrt_rn(fma(0.5, divide_rn(t, divisor(L.p)), g.hgm1g));
+    if (NRM == 2 && ge0(S_L))
         return false;
-    double GD[4], GU[4];
-    flux_y(UD, g, GD);
-    flux_y(UU, g, GU);
-#pragma unroll
-    for (int k = 0; k < 4; k++)
+    const double S_R = qR + aR * sqrt_rn(fma(0.5, divide_rn(t, divisor(R.p)), g.hgm1g));
+    if (ge0(S_L))
+        strict_flux<NRM>(L, F);
+    else if (le0(S_R))
+        strict_flux<NRM>(R, F);
+    else
     {
-        if (S_U <= 0)
-            G[k] = GU[k];
-        else
-            G[k] = (S_U * GD[k] - S_D * GU[k] + S_U * S_D * (UU[k] - UD[k])) / (S_U - S_D);
+        double FL[4], FR[4];
+        strict_flux<NRM>(L, FL);
+        strict_flux<NRM>(R, FR);
+        const Divisor by_w = divisor(S_R - S_L);
+        const double SS = S_R * S_L;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            F[k] = divide_rn(S_R * FL[k] - S_L * FR[k] + SS * (UR[k] - UL[k]), by_w);
     }
     return true;
 }
@@ -386,75 +416,38 @@ __device__ __forceinline__ int pvrs_y(const double UD[4], const double UU[4], do
 
 // ----------------------------------------------------------- Steger-Warming
 
-#define IBTFO_SW_LAM(x, sgn) (0.5 * ((x)sgn sqrt((x) * (x) + delta * delta)))
-
-// StegerWarming/Riemann_solver.cpp:173-234 (X): F = F+(U_L) + F-(U_R)
-__device__ __forceinline__ void sw_x(const double UL[4], const double UR[4], double g, double F[4])
+// StegerWarming/Riemann_solver.cpp:173-234 (X), :262-325 (Y): F = F+(U_L) + F-(U_R).
+// Halves (x / 2) are exact and move past the roundings they commute with.
+template <int NRM, int SIGN>
+__device__ __forceinline__ void strict_sw_split(const double U[4], const GridDesc &g, double f[4])
 {
-    double rho_L = UL[0], rho_R = UR[0];
-    double u_L = UL[1] / rho_L;
-    double v_L = UL[2] / rho_L;
-    double p_L = (g - 1) * (UL[3] - 0.5 * rho_L * (u_L * u_L + v_L * v_L));
-    double u_R = UR[1] / rho_R;
-    double v_R = UR[2] / rho_R;
-    double p_R = (g - 1) * (UR[3] - 0.5 * rho_R * (u_R * u_R + v_R * v_R));
-    double a_L = pow_half(g * p_L / rho_L);
-    double a_R = pow_half(g * p_R / rho_R);
-    double e_L = p_L / (g - 1) / rho_L;
-    double e_R = p_R / (g - 1) / rho_R;
-    double h_L = e_L + u_L * u_L / 2 + v_L * v_L / 2 + p_L / rho_L;
-    double h_R = e_R + u_R * u_R / 2 + v_R * v_R / 2 + p_R / rho_R;
+    const StrictPrim s = strict_prim(U, g);
+    const double a = pow_half(divide_rn(g.gamma * s.p, s.by_rho));
+    const double e = divide_rn(divide_rn(s.p, g.by_gm1), s.by_rho);
+    const double h = fma(0.5, s.v * s.v, fma(0.5, s.u * s.u, e)) + divide_rn(s.p, s.by_rho);
     const double delta = 1e-6;
-    double l1p = IBTFO_SW_LAM(u_L, +), l3p = IBTFO_SW_LAM((u_L - a_L), +), l4p = IBTFO_SW_LAM((u_L + a_L), +);
-    double l1n = IBTFO_SW_LAM(u_R, -), l3n = IBTFO_SW_LAM((u_R - a_R), -), l4n = IBTFO_SW_LAM((u_R + a_R), -);
-    double f1p = rho_L * (2 * (g - 1) * l1p + l3p + l4p) / 2 / g;
-    double f2p = rho_L * (2 * (g - 1) * u_L * l1p + (u_L - a_L) * l3p + (u_L + a_L) * l4p) / 2 / g;
-    double f3p = rho_L * (2 * (g - 1) * v_L * l1p + l3p * v_L + l4p * v_L) / 2 / g;
-    double f4p = rho_L * ((g - 1) * (u_L * u_L + v_L * v_L) * l1p + (h_L - a_L * u_L) * l3p + (h_L + a_L * u_L) * l4p) / 2 / g;
-    double f1n = rho_R * (2 * (g - 1) * l1n + l3n + l4n) / 2 / g;
-    double f2n = rho_R * (2 * (g - 1) * u_R * l1n + (u_R - a_R) * l3n + (u_R + a_R) * l4n) / 2 / g;
-    double f3n = rho_R * (2 * (g - 1) * v_R * l1n + l3n * v_R + l4n * v_R) / 2 / g;
-    double f4n = rho_R * ((g - 1) * (u_R * u_R + v_R * v_R) * l1n + (h_R - a_R * u_R) * l3n + (h_R + a_R * u_R) * l4n) / 2 / g;
-    F[0] = f1p + f1n;
-    F[1] = f2p + f2n;
-    F[2] = f3p + f3n;
-    F[3] = f4p + f4n;
+    auto lam = [&](double x) {
+        const double r = sqrt_rn(x * x + delta * delta);
+        return 0.5 * (SIGN > 0 ? x + r : x - r);
+    };
+    const double q = (NRM == 1) ? s.u : s.v, w = (NRM == 1) ? s.v : s.u;
+    const double l1 = lam(q), l3 = lam(q - a), l4 = lam(q + a);
+    f[0] = divide_rn(0.5 * (s.rho * (g.gm1x2 * l1 + l3 + l4)), g.by_g);
+    f[NRM] = divide_rn(0.5 * (s.rho * (g.gm1x2 * q * l1 + (q - a) * l3 + (q + a) * l4)), g.by_g);
+    f[3 - NRM] = divide_rn(0.5 * (s.rho * (g.gm1x2 * w * l1 + l3 * w + l4 * w)), g.by_g);
+    f[3] = divide_rn(0.5 * (s.rho * (g.gm1 * (s.u * s.u + s.v * s.v) * l1 + (h - a * q) * l3 + (h + a * q) * l4)),
+                     g.by_g);
 }
-
-// StegerWarming/Riemann_solver.cpp:262-325 (Y): G = G+(U_D) + G-(U_U)
-__device__ __forceinline__ void sw_y(const double UD[4], const double UU[4], double g, double G[4])
+template <int NRM>
+__device__ __forceinline__ void strict_sw(const double UL[4], const double UR[4], const GridDesc &g, double F[4])
 {
-    double rho_U = UU[0], rho_D = UD[0];
-    double u_U = UU[1] / rho_U;
-    double v_U = UU[2] / rho_U;
-    double p_U = (g - 1) * (UU[3] - 0.5 * rho_U * (u_U * u_U + v_U * v_U));
-    double u_D = UD[1] / rho_D;
-    double v_D = UD[2] / rho_D;
-    double p_D = (g - 1) * (UD[3] - 0.5 * rho_D * (u_D * u_D + v_D * v_D));
-    double a_U = pow_half(g * p_U / rho_U);
-    double a_D = pow_half(g * p_D / rho_D);
-    double e_U = p_U / (g - 1) / rho_U;
-    double e_D = p_D / (g - 1) / rho_D;
-    double h_U = e_U + u_U * u_U / 2 + v_U * v_U / 2 + p_U / rho_U;
-    double h_D = e_D + u_D * u_D / 2 + v_D * v_D / 2 + p_D / rho_D;
-    const double delta = 1e-6;
-    double m1p = IBTFO_SW_LAM(v_D, +), m3p = IBTFO_SW_LAM((v_D - a_D), +), m4p = IBTFO_SW_LAM((v_D + a_D), +);
-    double m1n = IBTFO_SW_LAM(v_U, -), m3n = IBTFO_SW_LAM((v_U - a_U), -), m4n = IBTFO_SW_LAM((v_U + a_U), -);
-    double g1p = rho_D * (2 * (g - 1) * m1p + m3p + m4p) / 2 / g;
-    double g2p = rho_D * (2 * (g - 1) * u_D * m1p + m3p * u_D + m4p * u_D) / 2 / g;
-    double g3p = rho_D * (2 * (g - 1) * v_D * m1p + (v_D - a_D) * m3p + (v_D + a_D) * m4p) / 2 / g;
-    double g4p = rho_D * ((g - 1) * (u_D * u_D + v_D * v_D) * m1p + (h_D - a_D * v_D) * m3p + (h_D + a_D * v_D) * m4p) / 2 / g;
-    double g1n = rho_U * (2 * (g - 1) * m1n + m3n + m4n) / 2 / g;
-    double g2n = rho_U * (2 * (g - 1) * u_U * m1n + m3n * u_U + m4n * u_U) / 2 / g;
-    double g3n = rho_U * (2 * (g - 1) * v_U * m1n + (v_U - a_U) * m3n + (v_U + a_U) * m4n) / 2 / g;
-    double g4n = rho_U * ((g - 1) * (u_U * u_U + v_U * v_U) * m1n + (h_U - a_U * v_U) * m3n + (h_U + a_U * v_U) * m4n) / 2 / g;
-    G[0] = g1p + g1n;
-    G[1] = g2p + g2n;
-    G[2] = g3p + g3n;
-    G[3] = g4p + g4n;
+    double fp[4], fn[4];
+    strict_sw_split<NRM, 1>(UL, g, fp);
+    strict_sw_split<NRM, -1>(UR, g, fn);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        F[k] = fp[k] + fn[k];
 }
-
-#undef IBTFO_SW_LAM
 
 // ---------------------------------------------------------------- PVRS stray store
 //
@@ -573,18 +566,18 @@ __device__ bool pvrs_stray_source(const double *__restrict__ U, long long P, int
 // One X face: states from four cells, MHM predictor, Riemann solver.
 template <int SCH, int RIE, int LIM>
 __device__ __forceinline__ void x_face(const double c0[4], const double c1[4], const double c2[4], const double c3[4],
-                                       double g, double dt, double dx, double F[4])
+                                       const GridDesc &g, double dt, double F[4])
 {
     double UL[4], UR[4];
     face_states<SCH, LIM>(c0, c1, c2, c3, UL, UR);
     if (SCH == MHM)
-        mhm_predict<0>(UL, UR, g, dt, dx);
+        mhm_predict<1>(UL, UR, g, dt);
     if (RIE == PVRS)
-        pvrs_x(UL, UR, g, F);
+        pvrs_x(UL, UR, g.gamma, F);
     else if (RIE == SW)
-        sw_x(UL, UR, g, F);
+        strict_sw<1>(UL, UR, g, F);
     else
-        hll_x(UL, UR, g, F);
+        strict_hll<1>(UL, UR, g, F);
 }
 
 // One Y face.  Returns the mask of components that keep the X-face flux of
@@ -592,20 +585,20 @@ __device__ __forceinline__ void x_face(const double c0[4], const double c1[4], c
 // branch at :547-550, none otherwise).
 template <int SCH, int RIE, int LIM>
 __device__ __forceinline__ int y_face(const double c0[4], const double c1[4], const double c2[4], const double c3[4],
-                                      double g, double dt, double dy, double G[4], double *stray)
+                                      const GridDesc &g, double dt, double G[4], double *stray)
 {
     double UD[4], UU[4];
     face_states<SCH, LIM>(c0, c1, c2, c3, UD, UU);
     if (SCH == MHM)
-        mhm_predict<1>(UD, UU, g, dt, dy);
+        mhm_predict<2>(UD, UU, g, dt);
     if (RIE == PVRS)
-        return pvrs_y(UD, UU, g, G, stray);
+        return pvrs_y(UD, UU, g.gamma, G, stray);
     if (RIE == SW)
     {
-        sw_y(UD, UU, g, G);
+        strict_sw<2>(UD, UU, g, G);
         return 0;
     }
-    return hll_y(UD, UU, g, G) ? 0 : 0xF;
+    return strict_hll<2>(UD, UU, g, G) ? 0 : 0xF;
 }
 
 } // namespace ibtfo

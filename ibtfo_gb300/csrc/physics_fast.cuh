@@ -46,45 +46,21 @@ struct GasConst<double>
     }
 };
 
-// 1/x of a double from the hardware estimate of the double's high word and
-// two Newton steps: four FP64 instructions (zero, subnormal, non-finite x,
-// results outside the normal range, and very small or large x)
-__device__ __forceinline__ double rcp_newton2(double x)
+// 1/x of a double on the integer pipes (int64math.cuh; no FP64 instruction,
+// four before).  Zero, subnormal and non-finite x, and results near the ends
+// of the exponent range: the hardware estimate of the double's high word and
+// two Newton steps.
+__device__ __forceinline__ double rcp_t(double x)
 {
+    const uint64_t b = double_bits(x);
+    if (rcp_range(b))
+        return rcp_int(b);
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     double e = fma(-x, y, 1.0);
     y = fma(y, e, y);
     e = fma(-x, y, 1.0);
     return fma(y, e, y);
-}
-// 1/x in two FP64 instructions, for a part whose FP64 pipe runs at 1/64 of
-// the FP32 one: the significand m = mh + ml (24 + 23 bits) as two floats, the
-// FP32 estimate y = 1/mh, its residual e = 1 - (mh + ml) y in FP32 (exact to
-// 2^-46), and y + y e put together as a double by integer arithmetic is 1/x to
-// about 2^-44; one Newton step in FP64 squares that.  Within an ulp of the
-// rounded value, as before; the FP64 faces went from 121 to 80 instructions
-// with this, sqrt_t and the flux form of physics_fast64.cuh.
-__device__ __forceinline__ double rcp_t(double x)
-{
-    const int hi = __double2hiint(x);
-    const unsigned lo = (unsigned)__double2loint(x);
-    const unsigned ex = (unsigned)(hi >> 20) & 0x7ffu;
-    if (ex - 2u > 2040u)
-        return rcp_newton2(x);
-    const float mh = __int_as_float(0x3f800000 | ((hi << 3) & 0x007ffff8) | (int)(lo >> 29));
-    const float ml = __int_as_float(0x3f800000 | (int)((lo >> 6) & 0x007fffffu)) - 1.0f; // units of 2^-23
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(mh));
-    y = fminf(fmaxf(y, 0.5f), 1.0f); // one binade, so that the correction below is in its units
-    const float e = fmaf(ml * -0x1p-23f, y, fmaf(-mh, y, 1.0f));
-    const int n = __float2int_rn((y * e) * 0x1p52f); // |y e| < 2^-21
-    // y as a double of exponent 1023 - ex more, plus n units of 2^-52
-    const unsigned long long b = ((unsigned long long)(unsigned)__float_as_int(y) << 29) +
-                                 ((unsigned long long)(long long)(896 + 1023 - (int)ex) << 52) +
-                                 (unsigned long long)(2LL * n);
-    const double y0 = __longlong_as_double((long long)(b | ((unsigned long long)(hi & 0x80000000) << 32)));
-    return fma(y0, fma(-x, y0, 1.0), y0);
 }
 // FP32 form: hardware reciprocal seed + one Newton step (within ~1 ulp; no
 // correctly-rounded slow path), and the hardware square root approximation
@@ -96,52 +72,13 @@ __device__ __forceinline__ float rcp_t(float x)
     const float e = fmaf(-x, y, 1.0f);
     return fmaf(y, e, y);
 }
-// sqrt(x) of a double from the hardware reciprocal square root estimate
-// y0 = (1 + e)/sqrt(x), |e| <= 2^-20 (measured on GB300): one
-// Newton step folded into t = x y0 gives s0 = t (1 + r/2), r = 1 - x y0^2,
-// with relative error 1.5 e^2; one residual correction s1 = s0 + (y0/2)(x -
-// s0^2) leaves 1.5 e^3 (< 2^-59), so s1 is within about an ulp of sqrt(x).
-// Seven FP64 operations; zero, negative, subnormal and non-finite x take the
-// library square root.
-__device__ __forceinline__ double sqrt_newton2(double x)
-{
-    const long long ix = __double_as_longlong(x);
-    if (ix < 0x0010000000000000LL || ix >= 0x7ff0000000000000LL)
-        return sqrt(x);
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double t = x * y;
-    const double r = fma(-t, y, 1.0);
-    const double s0 = fma(0.5 * t, r, t);
-    const double d = fma(-s0, s0, x);
-    return fma(0.5 * y, d, s0);
-}
-// sqrt(x) in two FP64 instructions, as rcp_t: x = 4^k (mh + ml), mh in [1, 4);
-// with the FP32 estimate y = 1/sqrt(mh) and s = mh y, the FP32 residual
-// r = mh + ml - s^2 gives s + y r / 2 = sqrt(mh + ml) to about 2^-43, put
-// together as a double by integer arithmetic; the residual correction in
-// FP64 squares that (x far from the ends of the exponent range, so that
-// x - s^2 stays normal; others take the form above).
+// sqrt(x) of a double on the integer pipes (no FP64 instruction, seven
+// before); zero, negative, subnormal and non-finite x take the library square
+// root.
 __device__ __forceinline__ double sqrt_t(double x)
 {
-    const int hi = __double2hiint(x);
-    const unsigned lo = (unsigned)__double2loint(x);
-    if ((unsigned)(hi - (128 << 20)) >= (unsigned)(1790 << 20))
-        return sqrt_newton2(x);
-    const int E = (hi >> 20) - 1023, odd = E & 1, k = E >> 1;
-    const float mh = __int_as_float((0x3f800000 + (odd << 23)) | ((hi << 3) & 0x007ffff8) | (int)(lo >> 29));
-    const float ml = __int_as_float(0x3f800000 | (int)((lo >> 6) & 0x007fffffu)) - 1.0f; // units of 2^-23 (odd: 2^-22)
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(mh));
-    const float s = fminf(fmaxf(mh * y, 1.0f), 2.0f); // one binade
-    const float r = fmaf(ml, odd ? 0x1p-22f : 0x1p-23f, fmaf(-s, s, mh));
-    const int n = __float2int_rn((y * r) * 0x1p50f); // |y r / 2| < 2^-20, in units of 2^-51
-    const unsigned long long b = ((unsigned long long)(unsigned)__float_as_int(s) << 29) +
-                                 ((unsigned long long)(long long)(896 + k) << 52) + (unsigned long long)(2LL * n);
-    const double s0 = __longlong_as_double((long long)b);
-    const double h = __longlong_as_double((long long)(((unsigned long long)(unsigned)__float_as_int(y) << 29) +
-                                                      ((unsigned long long)(long long)(895 - k) << 52))); // ~ 1/(2 s0)
-    return fma(h, fma(-s0, s0, x), s0);
+    const uint64_t b = double_bits(x);
+    return sqrt_range(b) ? sqrt_int(b) : sqrt_hardware(x);
 }
 __device__ __forceinline__ float sqrt_t(float x)
 {
@@ -157,10 +94,9 @@ __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(
 // underflow to zero as positive (only for |a|,|b| below ~1e-154 in double)
 __device__ __forceinline__ double minmod_t(double a, double b)
 {
-    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    const long long ma = ia & 0x7fffffffffffffffLL, mb = ib & 0x7fffffffffffffffLL;
-    const bool ok = ((ia ^ ib) >= 0) && ma != 0 && mb != 0 && ma <= 0x7ff0000000000000LL &&
-                    mb <= 0x7ff0000000000000LL;
+    const long long ma = magnitude_bits(a), mb = magnitude_bits(b);
+    const bool ok = ((__double2hiint(a) ^ __double2hiint(b)) >= 0) && ma != 0 && mb != 0 &&
+                    ma <= 0x7ff0000000000000LL && mb <= 0x7ff0000000000000LL;
     return ok ? ((ma > mb) ? b : a) : 0.0;
 }
 // FP32: the reference's form, a product and two compares on the FP32 pipes

@@ -4,9 +4,8 @@
 // What bounds the FP64 sweeps is the FP64 pipe (two thread instructions per
 // SM and clock, one sixty-fourth of the FP32 rate), so an FP64 instruction
 // costs as much as 64 integer or FP32 ones.  Three things follow:
-//   * reciprocals and square roots start from a 44-bit estimate made on the
-//     FP32 and integer pipes (rcp_t, sqrt_t in physics_fast.cuh) and need two
-//     FP64 instructions each;
+//   * reciprocals and square roots are taken on the integer and FP32 pipes
+//     (int64math.cuh), which the faces leave idle;
 //   * comparisons and the positivity tests read bit patterns;
 //   * the fluxes are written so that no full flux of either side is formed:
 //     with S_L = u_L - c_L and S_R = u_R + c_R the HLL flux is
@@ -25,18 +24,6 @@
 #include "physics_fast.cuh"
 
 namespace ibtfo {
-
-// x >= 0 and x <= 0 as IEEE comparisons give them (false for NaN), on the integer pipe
-__device__ __forceinline__ bool ge0(double x)
-{
-    const long long b = __double_as_longlong(x);
-    return (b >= 0 && b <= 0x7ff0000000000000LL) || b == (long long)0x8000000000000000ULL;
-}
-__device__ __forceinline__ bool le0(double x)
-{
-    const long long b = __double_as_longlong(x);
-    return b == 0 || (b < 0 && b <= (long long)0xfff0000000000000ULL);
-}
 
 // a state with its primitive variables across a face of normal NRM
 struct Prim64

@@ -149,6 +149,14 @@ struct CellStats
     int nans = 0;
 };
 
+// max(m, x) for m >= 0 as fmax gives it (NaN and negative x leave m), with
+// the compare on the integer pipe: non-negative doubles order like their bits
+__device__ __forceinline__ double max_nonneg(double m, double x)
+{
+    const long long bm = __double_as_longlong(m), bx = __double_as_longlong(x);
+    return (bx > bm && bx <= 0x7ff0000000000000LL) ? x : m;
+}
+
 // Block-wide FP64 reduction of the per-thread statistics, then
 // block_commit_finalize.
 template <int NT>
@@ -168,10 +176,10 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
     {
-        cs.amax = fmax(cs.amax, __shfl_xor_sync(0xffffffffu, cs.amax, o));
-        cs.a2max = fmax(cs.a2max, __shfl_xor_sync(0xffffffffu, cs.a2max, o));
-        cs.umax = fmax(cs.umax, __shfl_xor_sync(0xffffffffu, cs.umax, o));
-        cs.vmax = fmax(cs.vmax, __shfl_xor_sync(0xffffffffu, cs.vmax, o));
+        cs.amax = max_nonneg(cs.amax, __shfl_xor_sync(0xffffffffu, cs.amax, o));
+        cs.a2max = max_nonneg(cs.a2max, __shfl_xor_sync(0xffffffffu, cs.a2max, o));
+        cs.umax = max_nonneg(cs.umax, __shfl_xor_sync(0xffffffffu, cs.umax, o));
+        cs.vmax = max_nonneg(cs.vmax, __shfl_xor_sync(0xffffffffu, cs.vmax, o));
         cs.mass += __shfl_xor_sync(0xffffffffu, cs.mass, o);
         cs.nans += __shfl_xor_sync(0xffffffffu, cs.nans, o);
     }
@@ -194,32 +202,24 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
         n = rnan[0];
         for (int w = 1; w < NT / 32; w++)
         {
-            a = fmax(a, red[0][w]);
-            a2 = fmax(a2, red[4][w]);
-            u = fmax(u, red[1][w]);
-            v = fmax(v, red[2][w]);
+            a = max_nonneg(a, red[0][w]);
+            a2 = max_nonneg(a2, red[4][w]);
+            u = max_nonneg(u, red[1][w]);
+            v = max_nonneg(v, red[2][w]);
             m += red[3][w];
             n += rnan[w];
         }
-        a = fmax(a, sqrt(a2));
+        a = max_nonneg(a, sqrt_rn(a2));
     }
     block_commit_finalize<NT>(a, u, v, m, n, st, partial, g, step_accounting, set_start, nblocks, bid);
-}
-
-// max(m, x) for m >= 0 as fmax gives it (NaN and negative x leave m), with
-// the compare on the integer pipe: non-negative doubles order like their bits
-__device__ __forceinline__ double max_nonneg(double m, double x)
-{
-    const long long bm = __double_as_longlong(m), bx = __double_as_longlong(x);
-    return (bx > bm && bx <= 0x7ff0000000000000LL) ? x : m;
 }
 
 // any of four values NaN, tested on the integer pipe
 __device__ __forceinline__ int any_nan4(const double v[4])
 {
-    const long long inf = 0x7ff0000000000000LL, mask = 0x7fffffffffffffffLL;
-    return ((__double_as_longlong(v[0]) & mask) > inf || (__double_as_longlong(v[1]) & mask) > inf ||
-            (__double_as_longlong(v[2]) & mask) > inf || (__double_as_longlong(v[3]) & mask) > inf)
+    const long long inf = 0x7ff0000000000000LL;
+    return (magnitude_bits(v[0]) > inf || magnitude_bits(v[1]) > inf || magnitude_bits(v[2]) > inf ||
+            magnitude_bits(v[3]) > inf)
                ? 1
                : 0;
 }
@@ -229,12 +229,13 @@ __device__ __forceinline__ int any_nan4(const double v[4])
 __device__ __forceinline__ void cell_stats(const double v[4], double gam, double dx, double dy, CellStats &cs)
 {
     double rho = v[0];
-    double u = v[1] / v[0];
-    double w = v[2] / v[0];
+    const Divisor by_rho = divisor(rho);
+    double u = divide_rn(v[1], by_rho);
+    double w = divide_rn(v[2], by_rho);
     double p = (gam - 1) * (v[3] - 0.5 * rho * (u * u + w * w));
-    cs.a2max = max_nonneg(cs.a2max, gam * p / rho); // pow(gam p / rho, 0.5) taken once per block
-    cs.umax = max_nonneg(cs.umax, fabs(u));
-    cs.vmax = max_nonneg(cs.vmax, fabs(w));
+    cs.a2max = max_nonneg(cs.a2max, divide_rn(gam * p, by_rho)); // pow(gam p / rho, 0.5) taken once per block
+    cs.umax = max_nonneg(cs.umax, magnitude(u));
+    cs.vmax = max_nonneg(cs.vmax, magnitude(w));
     cs.mass += v[0] * dx * dy;
     cs.nans += any_nan4(v);
 }
@@ -244,8 +245,8 @@ __device__ __forceinline__ void cell_stats_fast(const double v[4], const Cell64 
                                                 double dxdy, CellStats &cs)
 {
     cs.a2max = max_nonneg(cs.a2max, K.ggm1 * (c.ir * c.ei));
-    cs.umax = max_nonneg(cs.umax, fabs(c.u));
-    cs.vmax = max_nonneg(cs.vmax, fabs(c.v));
+    cs.umax = max_nonneg(cs.umax, magnitude(c.u));
+    cs.vmax = max_nonneg(cs.vmax, magnitude(c.v));
     cs.mass += v[0] * dxdy;
     cs.nans += any_nan4(v);
 }
@@ -365,7 +366,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
             if (FASTPHYS)
                 face64<SCH, RIE, LIM, 1>(c0, c1, c2, c3, K, hx2, f, nullptr);
             else
-                x_face<SCH, RIE, LIM>(c0, c1, c2, c3, gam, dt, g.dx, f);
+                x_face<SCH, RIE, LIM>(c0, c1, c2, c3, g, dt, f);
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 s.sF[k][r][fc] = f[k];
@@ -384,7 +385,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
             }
             double stray = 0.0;
             int keep = FASTPHYS ? face64<SCH, RIE, LIM, 2>(c0, c1, c2, c3, K, hy2, f, &stray)
-                                : y_face<SCH, RIE, LIM>(c0, c1, c2, c3, gam, dt, g.dy, f, &stray);
+                                : y_face<SCH, RIE, LIM>(c0, c1, c2, c3, g, dt, f, &stray);
             if constexpr (RIE == PVRS)
             {
                 // the reference's PVRS stray store from cell 7 c' + 2 into this face's
@@ -428,7 +429,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
         if (FASTPHYS)
             face64<SCH, RIE, LIM, 1>(c0, c1, c2, c3, K, hx2, f, nullptr);
         else
-            x_face<SCH, RIE, LIM>(c0, c1, c2, c3, gam, dt, g.dx, f);
+            x_face<SCH, RIE, LIM>(c0, c1, c2, c3, g, dt, f);
 #pragma unroll
         for (int k = 0; k < 4; k++)
             s.sF[k][r][fc] = f[k];
@@ -457,8 +458,9 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
                 }
                 else
                 {
-                    double x = s.sU[k][r + 2][c + 2] - dt * (s.sF[k][r + 1][c + 1] - s.sF[k][r + 1][c]) / g.dx;
-                    v[k] = x - dt * (gp - gm) / g.dy;
+                    double x = s.sU[k][r + 2][c + 2] -
+                               divide_rn(dt * (s.sF[k][r + 1][c + 1] - s.sF[k][r + 1][c]), g.by_dx);
+                    v[k] = x - divide_rn(dt * (gp - gm), g.by_dy);
                 }
             }
             Cell64 cl;
