@@ -71,7 +71,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, (PREC == 2 && RIE == HLLT) ? 3 
             CellStats cs;
             sweep_tile64<SCH, RIE, LIM, 1, TX, TY, NT>(s, g, U, V, a.type, i0, j0, dt, cs, stage, tm, status,
                                                        interior);
-            block_reduce_finalize<NT>(cs, st, a.partial, g, true, false, (unsigned)bc.ntiles, e.y, stage == 1);
+            block_reduce_finalize<NT, TX, TY>(cs, st, {a.partial, (unsigned)bc.ntiles, false, e.y}, g, true, false,
+                                              (unsigned)bc.ntiles, stage == 1);
         }
     }
 }

@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) reduce_kernel(const ReduceArgs
             double v[4];
             for (int k = 0; k < 4; k++)
                 v[k] = state_ld(a.u, k, o, g);
-            cell_stats(v, g.gamma, g.dx, g.dy, cs);
+            cell_stats(v, g.gamma, g.dx, g.dy, cs, cs.mass);
         }
         else if (a.type[o] == CELL_CUT && a.alpha)
         {
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) reduce_kernel(const ReduceArgs
             for (int k = 0; k < 4; k++)
                 v[k] = state_ld(a.u, k, o, g);
             CellStats c1;
-            cell_stats(v, g.gamma, g.dx, g.dy, c1);
+            cell_stats(v, g.gamma, g.dx, g.dy, c1, c1.mass);
             cs.mass += a.alpha[o] * c1.mass;
             cs.nans += c1.nans;
             if (a.alpha[o] >= 0.5)
@@ -458,8 +458,9 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) reduce_kernel(const ReduceArgs
             }
         }
     }
-    block_reduce_finalize<TILE_X * TILE_Y>(cs, a.st, a.partial, g, false, a.set_start, gridDim.x * gridDim.y,
-                                           blockIdx.y * gridDim.x + blockIdx.x);
+    const unsigned nblocks = gridDim.x * gridDim.y;
+    block_reduce_finalize<TILE_X * TILE_Y>(cs, a.st, {a.partial, nblocks, false, blockIdx.y * gridDim.x + blockIdx.x},
+                                           g, false, a.set_start, nblocks);
 }
 
 void launch_reduce(const ReduceArgs &a, int, cudaStream_t s)

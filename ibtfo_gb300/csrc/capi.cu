@@ -21,39 +21,42 @@
 #include "physics.cuh"
 
 namespace ibtfo {
-SweepLaunch sweep_launcher_muscl(int riemann, int limiter);
-SweepLaunch sweep_launcher_mhm(int riemann, int limiter);
-SweepLaunch sweep_launcher_godunov(int riemann, int limiter);
-SweepLaunch sweep_launcher_muscl_fast(int riemann, int limiter, int ty);
-SweepLaunch sweep_launcher_mhm_fast(int riemann, int limiter, int ty);
-SweepLaunch sweep_launcher_godunov_fast(int riemann, int limiter, int ty);
-SweepLaunch sweep_launcher_muscl_f32(int riemann, int limiter, int ty);
-SweepLaunch sweep_launcher_mhm_f32(int riemann, int limiter, int ty);
-SweepLaunch sweep_launcher_godunov_f32(int riemann, int limiter, int ty);
+SweepLaunch sweep_launcher_muscl(int riemann, int limiter, bool fine);
+SweepLaunch sweep_launcher_mhm(int riemann, int limiter, bool fine);
+SweepLaunch sweep_launcher_godunov(int riemann, int limiter, bool fine);
+SweepLaunch sweep_launcher_muscl_fast(int riemann, int limiter, bool fine);
+SweepLaunch sweep_launcher_mhm_fast(int riemann, int limiter, bool fine);
+SweepLaunch sweep_launcher_godunov_fast(int riemann, int limiter, bool fine);
+SweepLaunch sweep_launcher_muscl_f32(int riemann, int limiter);
+SweepLaunch sweep_launcher_mhm_f32(int riemann, int limiter);
+SweepLaunch sweep_launcher_godunov_f32(int riemann, int limiter);
 SweepLaunch sweep_launcher_lax();
 
-// the sweep of a case's configuration over TILE_X x ty tiles (ty = TILE_Y,
-// or FAST_TILE_Y for the fp64_fast sweeps without PVRS and the FP32 sweeps)
-SweepLaunch sweep_launcher(int scheme, int riemann, int limiter, int precision, int ty)
+// the sweep of a case's configuration over its tiles of TILE_X columns, or
+// (fine; FP64 precisions except Lax) over FINE_X x FINE_Y tiles
+static SweepLaunch sweep_launcher(int scheme, int riemann, int limiter, int precision, bool fine)
 {
     const int r = (riemann == HLLC) ? HLL : riemann; // HLLC/Riemann_solver.cpp is HLL
     const bool fast = (precision == IBTFO_PRECISION_FP64_FAST);
     if (scheme == LAX)
-        return sweep_launcher_lax(); // strict FP64 for both FP64 keys
+        return fine ? nullptr : sweep_launcher_lax(); // strict FP64 for both FP64 keys
     if (precision == IBTFO_PRECISION_FP32_COMPENSATED)
     {
+        if (fine)
+            return nullptr;
         switch (scheme)
         {
-        case MHM: return sweep_launcher_mhm_f32(r, limiter, ty);
-        case GODUNOV: return sweep_launcher_godunov_f32(r, limiter, ty);
-        default: return sweep_launcher_muscl_f32(r, limiter, ty);
+        case MHM: return sweep_launcher_mhm_f32(r, limiter);
+        case GODUNOV: return sweep_launcher_godunov_f32(r, limiter);
+        default: return sweep_launcher_muscl_f32(r, limiter);
         }
     }
     switch (scheme)
     {
-    case MHM: return fast ? sweep_launcher_mhm_fast(r, limiter, ty) : sweep_launcher_mhm(r, limiter);
-    case GODUNOV: return fast ? sweep_launcher_godunov_fast(r, limiter, ty) : sweep_launcher_godunov(r, limiter);
-    default: return fast ? sweep_launcher_muscl_fast(r, limiter, ty) : sweep_launcher_muscl(r, limiter);
+    case MHM: return fast ? sweep_launcher_mhm_fast(r, limiter, fine) : sweep_launcher_mhm(r, limiter, fine);
+    case GODUNOV:
+        return fast ? sweep_launcher_godunov_fast(r, limiter, fine) : sweep_launcher_godunov(r, limiter, fine);
+    default: return fast ? sweep_launcher_muscl_fast(r, limiter, fine) : sweep_launcher_muscl(r, limiter, fine);
     }
 }
 
@@ -161,6 +164,13 @@ struct ibtfo_case
     CUtensorMap tmap[2];        // boxes of TILE_X x tile_y cells and their halo
     unsigned *tiles = nullptr;  // active sweep tiles (TILE_X x tile_y)
     int ntiles = 0;
+    // the device steps of a small grid sweep FINE_X x FINE_Y tiles (make_fine); 0: not in use
+    int nfine = 0, fine_tma = 0;
+    unsigned nparents = 0;      // 32x16 tiles the fine tiles' mass sums are grouped by
+    SweepLaunch fine_sweep = nullptr;
+    CUtensorMap fine_tmap[2];
+    unsigned *fine_tiles = nullptr, *fine_slot = nullptr;
+    double *fine_partial = nullptr;
     // the same tiles in row order: the row bands of the host-array step
     unsigned *band_list = nullptr;
     int nband_list = 0;
@@ -439,11 +449,11 @@ static ibtfo_status ring_to_host(ibtfo_case *c, double *u_out, cudaStream_t ks, 
 
 // Tensor maps of the two state buffers for the sweeps' bulk tensor copies:
 // (column, row, plane) with the row pitch and plane stride of the buffers,
-// box = a 32x8 tile plus its two-cell halo over the four planes (FP64, or
-// the FP32 form's hi planes).  A box starts at column i0 - 2 = 32 k + ng - 2,
+// box = a tx x ty tile plus its two-cell halo over the four planes (FP64, or
+// the FP32 form's hi planes).  A box starts at column i0 - 2 = tx k + ng - 2,
 // so the copies need ng == 2 for their 16-byte start alignment; other
 // ghost widths keep the element-wise staging.  0 when not available.
-static int make_state_tmaps(ibtfo_case *c)
+static int make_state_tmaps(const ibtfo_case *c, int tx, int ty, CUtensorMap tmap[2])
 {
     const GridDesc &g = c->g;
     if (g.ng != 2)
@@ -470,9 +480,9 @@ static int make_state_tmaps(ibtfo_case *c)
     const cuuint64_t dims[3] = {(cuuint64_t)g.M, (cuuint64_t)g.N, (cuuint64_t)(f32 ? 8 : 4)};
     const cuuint64_t strides[2] = {(cuuint64_t)g.pitch * elem, (cuuint64_t)g.plane * elem};
     const cuuint32_t estr[3] = {1, 1, 1};
-    const cuuint32_t box[3] = {TILE_X + 4, (cuuint32_t)c->tile_y + 4, 4};
+    const cuuint32_t box[3] = {(cuuint32_t)tx + 4, (cuuint32_t)ty + 4, 4};
     for (int b = 0; b < 2; b++)
-        if (encode(&c->tmap[b], f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, c->buf[b],
+        if (encode(&tmap[b], f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, c->buf[b],
                    dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return 0;
@@ -564,7 +574,8 @@ ibtfo_status ibtfo_destroy(ibtfo_case *c)
     // device-wide synchronisation (other cases keep running)
     cudaStream_t fs = c->own ? c->own : c->stream;
     void *bufs[] = {c->buf[0], c->buf[1], c->ic, c->staging, c->phi, c->nx, c->ny, c->type, c->ghosts,
-                    c->st, c->partial, c->ring_ic, c->tiles, c->band_list, c->alpha, c->ax, c->ay, c->mix_ex, c->mix_part,
+                    c->st, c->partial, c->ring_ic, c->tiles, c->band_list, c->fine_tiles, c->fine_slot,
+                    c->fine_partial, c->alpha, c->ax, c->ay, c->mix_ex, c->mix_part,
                     c->mix_links, c->mix_e};
     for (void *p : bufs)
         if (p)
@@ -638,9 +649,10 @@ ibtfo_status ibtfo_create(const ibtfo_config *cfg, ibtfo_case **out)
                         k.riemann != IBTFO_RIEMANN_PVRS
                     ? FAST_TILE_Y
                     : TILE_Y;
-    c->sweep = sweep_launcher(k.scheme, k.riemann, k.limiter, k.precision, c->tile_y);
-    if (k.boundary == IBTFO_BOUNDARY_CCM)
+    if (ccm)
         c->ccm = ccm_launcher(k.scheme, k.riemann, k.limiter, k.precision);
+    else
+        c->sweep = sweep_launcher(k.scheme, k.riemann, k.limiter, k.precision, false);
 
     const size_t plane_bytes = sizeof(double) * (size_t)g.plane;
     retain_pool_memory(c->device);
@@ -679,7 +691,7 @@ ibtfo_status ibtfo_create(const ibtfo_config *cfg, ibtfo_case **out)
         return s;
     }
     c->stream = c->own;
-    c->tma = make_state_tmaps(c);
+    c->tma = make_state_tmaps(c, TILE_X, c->tile_y, c->tmap);
     *out = c;
     return IBTFO_OK;
 }
@@ -709,6 +721,71 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
     CK(cudaMemcpy2DAsync(c->phi, sizeof(double) * g.pitch, phi, sizeof(double) * g.M, sizeof(double) * g.M, g.N,
                          cudaMemcpyHostToDevice, c->stream));
     return geometry_from_phi(c);
+}
+
+// Up to how many active 32x16 tiles the fp64_fast sweeps take 16x8 tiles.  A
+// 32x16 CTA lasts 45 us, most of it latency, and few of them leave SMs idle;
+// four 16x8 CTAs in its place spread over the SMs but solve 5% more faces and
+// reduce four times.  Measured (GB300, 152 SMs; us per step, 32x16 / 16x8
+// tiles): 48x24 cells 44 / 24, 256x128 (64 tiles) 46 / 30, channel 600x300
+// (100) 50 / 43, 400x200 (169) 60 / 54, channel 777x389 (190) 58 / 58, 512x256
+// (256) 70 / 69, channel 1000x500 (300) 76 / 86, 1200x600 (1444) 287 / 311.
+constexpr int FINE_PARENTS = 256;
+
+// The 16x8 tiles of a case's device steps (ibtfo_advance, ibtfo_step; the
+// row bands of the host-array step and batches keep the case's tiles): for
+// fp64_fast on grids of few tiles, and for the strict sweeps and the PVRS
+// solvers on every grid (32x8 / 16x8: strict HLL 48x24 41 / 31, 400x200 84 / 76,
+// 1200x600 511 / 482, channel 2048x1024 386 / 376 us per step; PVRS 1200x600
+// 2238 / 1889).  0, 2 (allocation) or 5 (CUDA error)
+static int make_fine(ibtfo_case *c)
+{
+    for (void *p : {(void *)c->fine_tiles, (void *)c->fine_slot, (void *)c->fine_partial})
+        if (p)
+            cudaFreeAsync(p, c->stream);
+    c->fine_tiles = c->fine_slot = nullptr;
+    c->fine_partial = nullptr;
+    c->nfine = 0;
+    if (c->ccm)
+        return 0;
+    c->fine_sweep = sweep_launcher(c->cfg.scheme, c->cfg.riemann, c->cfg.limiter, c->cfg.precision, true);
+    if (!c->fine_sweep)
+        return 0;
+    const GridDesc &g = c->g;
+    std::vector<unsigned> parents, fine;
+    int rc = active_tile_list(g, c->type, TILE_X, FAST_TILE_Y, parents, c->stream);
+    const bool fast = c->cfg.precision == IBTFO_PRECISION_FP64_FAST && c->cfg.riemann != IBTFO_RIEMANN_PVRS;
+    if (rc || (fast && parents.size() > FINE_PARENTS))
+        return rc;
+    rc = active_tile_list(g, c->type, FINE_X, FINE_Y, fine, c->stream);
+    if (rc)
+        return rc;
+    // a fine tile's mass sum: places per 32x16 tile, in the order of the
+    // list, so that the total adds up as over the 32x16 tiles (mass_partial)
+    const int ntx = (g.n_x + TILE_X - 1) / TILE_X, nty = (g.n_y + FAST_TILE_Y - 1) / FAST_TILE_Y;
+    std::vector<unsigned> place((size_t)ntx * nty, 0u), slot(fine.size());
+    for (size_t q = 0; q < parents.size(); q++)
+        place[(size_t)tile_jy(parents[q]) * ntx + tile_ix(parents[q])] = (unsigned)q;
+    constexpr int PX = TILE_X / FINE_X, PY = FAST_TILE_Y / FINE_Y;
+    for (size_t q = 0; q < fine.size(); q++)
+    {
+        const int ix = tile_ix(fine[q]), jy = tile_jy(fine[q]);
+        slot[q] = place[(size_t)(jy / PY) * ntx + ix / PX] * (PX * PY) + (unsigned)((jy % PY) * PX + ix % PX);
+    }
+    const size_t n = fine.size() * sizeof(unsigned), np = parents.size() * PX * PY * sizeof(double);
+    if (cudaMallocAsync(&c->fine_tiles, n, c->stream) != cudaSuccess ||
+        cudaMallocAsync(&c->fine_slot, n, c->stream) != cudaSuccess ||
+        cudaMallocAsync(&c->fine_partial, np, c->stream) != cudaSuccess)
+        return 2;
+    if (cudaMemcpyAsync(c->fine_tiles, fine.data(), n, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        cudaMemcpyAsync(c->fine_slot, slot.data(), n, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->fine_partial, 0, np, c->stream) != cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess)
+        return 5;
+    c->fine_tma = make_state_tmaps(c, FINE_X, FINE_Y, c->fine_tmap);
+    c->nparents = (unsigned)parents.size();
+    c->nfine = (int)fine.size();
+    return 0;
 }
 
 // normals, cell types, ghost list and tiles from the level set in c->phi
@@ -742,6 +819,8 @@ static ibtfo_status geometry_from_phi(ibtfo_case *c)
         rc = active_tiles(g, c->type, c->tile_y, &c->band_list, &c->nband_list, c->stream, &tile_list, true);
     if (rc == 0)
         rc = active_tiles(g, c->type, c->tile_y, &c->tiles, &c->ntiles, c->stream);
+    if (rc == 0)
+        rc = make_fine(c);
     if (rc == 0)
     {
         make_bands(c, tile_list);
@@ -912,6 +991,27 @@ static void enqueue_boundary(ibtfo_case *c)
     }
 }
 
+// one sweep of the device state: over the fine tiles where the case has them
+static void enqueue_sweep_stage(ibtfo_case *c, int guard, int stage)
+{
+    SweepArgs a = sweep_args(c, guard);
+    a.stage = stage;
+    count_launch();
+    if (!c->nfine)
+    {
+        c->sweep(a, c->ntiles, c->stream);
+        return;
+    }
+    a.tma = c->fine_tma;
+    a.tmap[0] = c->fine_tmap[0];
+    a.tmap[1] = c->fine_tmap[1];
+    a.tiles = c->fine_tiles;
+    a.slot = c->fine_slot;
+    a.nparents = c->nparents;
+    a.partial = c->fine_partial;
+    c->fine_sweep(a, c->nfine, c->stream);
+}
+
 // TimeAdvance: the sweep (and, for cut cells, the small-cell mixing after it)
 static void enqueue_advance(ibtfo_case *c, int guard)
 {
@@ -922,7 +1022,7 @@ static void enqueue_advance(ibtfo_case *c, int guard)
         a.alpha = c->alpha;
         a.ax = c->ax;
         a.ay = c->ay;
-        c->ccm(a, dim3(c->ntiles), dim3(TILE_X * TILE_Y), c->stream); // cut-cell cases: 32x8 tiles
+        c->ccm(a, c->ntiles, c->stream);
         count_launch();
         MixArgs m{};
         m.g = c->g;
@@ -938,8 +1038,7 @@ static void enqueue_advance(ibtfo_case *c, int guard)
         launch_mix(m, c->stream);
         return;
     }
-    c->sweep(sweep_args(c, guard), dim3(c->ntiles), dim3(TILE_X * TILE_Y), c->stream);
-    count_launch();
+    enqueue_sweep_stage(c, guard, 0);
 }
 
 // the sweep part of one iteration: Time = RK2, the first stage and its
@@ -949,14 +1048,9 @@ static void enqueue_sweeps(ibtfo_case *c, int guard)
 {
     if (c->cfg.time_advance == IBTFO_TIME_RK2)
     {
-        SweepArgs a = sweep_args(c, guard);
-        a.stage = 1;
-        c->sweep(a, dim3(c->ntiles), dim3(TILE_X * TILE_Y), c->stream);
-        count_launch();
+        enqueue_sweep_stage(c, guard, 1);
         enqueue_boundary(c);
-        a.stage = 2;
-        c->sweep(a, dim3(c->ntiles), dim3(TILE_X * TILE_Y), c->stream);
-        count_launch();
+        enqueue_sweep_stage(c, guard, 2);
         return;
     }
     enqueue_advance(c, guard);
@@ -1215,6 +1309,9 @@ ibtfo_status ibtfo_case_bytes(const ibtfo_config *k, long long *resident, long l
     if (k->boundary == IBTFO_BOUNDARY_CCM)
         r += 3 * 8 * plane;                               // cut cells: alpha and the two apertures
     r += plane + (long long)sizeof(DevState) + 8 * nblocks + 4 * nblocks + 2 * 2 * k->num_ghost_cell * 4 * 8;
+    // the fine tiles' lists and mass sums (FP64 precisions): a tile of 16x8 cells holds 16 bytes
+    if (k->precision != IBTFO_PRECISION_FP32_COMPENSATED && k->boundary != IBTFO_BOUNDARY_CCM)
+        r += 16LL * ((k->n_x + 31) / 32 * 2) * ((k->n_y + 15) / 16 * 2);
     // ghost records: at most every interior cell next to the outline, bounded
     // here by two layers around the domain perimeter per unit of perimeter
     if (k->boundary != IBTFO_BOUNDARY_REGULAR)
@@ -1761,7 +1858,7 @@ static ibtfo_status step_host_banded(ibtfo_case *c, const double *u_in, double *
         if (t1 > t0)
         {
             a.tile0 = t0;
-            c->sweep(a, dim3(t1 - t0), dim3(TILE_X * TILE_Y), s);
+            c->sweep(a, t1 - t0, s);
             count_launch();
         }
         CK(cudaEventRecord(c->ev_swept[k], s));

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     V[k * P + o] = v[k];
-                cell_stats_fast(v, cl, K, g.dxdy, cs);
+                cell_stats_fast(v, cl, K, g.dxdy, cs, cs.mass);
             }
         }
         else if (i < g.ng + g.n_x && j < g.ng + g.n_y && t == CELL_CUT)
@@ -325,17 +325,17 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
         }
     }
     if constexpr (PREC == 2)
-        block_reduce_finalize32<NT>(cs, st, a.partial, g, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x);
+        block_reduce_finalize32<NT>(cs, st, a.partial, g, gridDim.x, blockIdx.x);
     else
-        block_reduce_finalize<NT>(cs, st, a.partial, g, true, false, gridDim.x * gridDim.y,
-                                  blockIdx.y * gridDim.x + blockIdx.x);
+        block_reduce_finalize<NT>(cs, st, {a.partial, gridDim.x, false, blockIdx.x}, g, true, false, gridDim.x);
 }
 
 template <int SCH, int RIE, int LIM, int PREC>
-void launch_ccm_sweep(const CcmArgs &a, dim3 grid, dim3 block, cudaStream_t s)
+void launch_ccm_sweep(const CcmArgs &a, int grid, cudaStream_t s)
 {
     using T = typename std::conditional<PREC == 2, float, double>::type;
-    ccm_sweep_kernel<SCH, RIE, LIM, PREC><<<grid, block, sizeof(CcmSmem<T, TILE_X, ccm_tile_rows<PREC>()>), s>>>(a);
+    ccm_sweep_kernel<SCH, RIE, LIM, PREC>
+        <<<grid, TILE_X * TILE_Y, sizeof(CcmSmem<T, TILE_X, ccm_tile_rows<PREC>()>), s>>>(a);
 }
 
 // every Riemann solver and limiter of one scheme and precision: HLL_Toro,

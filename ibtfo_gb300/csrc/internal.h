@@ -128,6 +128,8 @@ struct SweepArgs
     int stage;               // 0: one step; Time = RK2: 1 the first stage, 2 the second stage and average
     int tile0;               // a step split over several launches: first tile of this launch
     int nblocks;             // ... and the tiles of the whole step (0: one launch, its grid)
+    const unsigned *slot;    // FINE_X x FINE_Y tiles: where each one's mass sum goes
+    unsigned nparents;       // ... and the 32x16 tiles they belong to
     int tma;                 // stage tiles with the tensor maps below (else element-wise loads)
     CUtensorMap tmap[2];     // buf0 / buf1 as (column, row, plane) tensors, box = tile + halo, 4 planes
 };
@@ -200,7 +202,7 @@ struct MixArgs
     double *e;        // exchange values, 4 per exchange
 };
 
-typedef void (*CcmLaunch)(const CcmArgs &, dim3 grid, dim3 block, cudaStream_t s);
+typedef void (*CcmLaunch)(const CcmArgs &, int grid, cudaStream_t s);
 CcmLaunch ccm_launcher(int scheme, int riemann, int limiter, int precision);
 void launch_mix(const MixArgs &a, cudaStream_t s);
 // geometry of a cut-cell case from the cell-centred level set: alpha, ax, ay,
@@ -210,7 +212,7 @@ int ccm_setup(const GridDesc &g, const double *d_phi, double *d_alpha, double *d
               MixExchange **d_ex, int *nex, MixParticipant **d_part, int *npart, int **d_links, double **d_e,
               cudaStream_t s);
 
-typedef void (*SweepLaunch)(const SweepArgs &, dim3 grid, dim3 block, cudaStream_t s);
+typedef void (*SweepLaunch)(const SweepArgs &, int grid, cudaStream_t s);
 
 // sweep tile (interior cells per CTA)
 constexpr int TILE_X = 32;
@@ -220,6 +222,9 @@ constexpr int TILE_Y = 8;
 // 2.16 faces per cell where a 32x8 tile solves 2.28, and stages 1.41 cells
 // per cell, not 1.69.  Every sweep CTA has TILE_X x TILE_Y threads.
 constexpr int FAST_TILE_Y = 16;
+// The FP64 sweeps' small tiles (capi.cu, make_fine): a 16x8 tile's 280 faces
+// are two passes of 160 threads, five CTAs per SM in 80 registers
+constexpr int FINE_X = 16, FINE_Y = 8, FINE_THREADS = 160;
 
 // A tile-list entry: the tile's column index in bits 0-15, its row index in
 // bits 16-30, and TILE_INTERIOR when every cell of the tile and of the
@@ -229,8 +234,6 @@ constexpr unsigned TILE_INTERIOR = 0x80000000u;
 __host__ __device__ __forceinline__ int tile_ix(unsigned t) { return (int)(t & 0xFFFFu); }
 __host__ __device__ __forceinline__ int tile_jy(unsigned t) { return (int)((t >> 16) & 0x7FFFu); }
 
-// the sweep of a configuration over TILE_X x ty tiles (capi.cu)
-SweepLaunch sweep_launcher(int scheme, int riemann, int limiter, int precision, int ty);
 void launch_fill(const FillArgs &a, cudaStream_t s);
 // ghost records [g0, g1) of a step in flight (FillArgs.pre_flip)
 void launch_fill_ghosts(const FillArgs &a, int g0, int g1, cudaStream_t s);

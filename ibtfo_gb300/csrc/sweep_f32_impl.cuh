@@ -484,7 +484,7 @@ __device__ __forceinline__ void block_reduce_finalize32(CellStats32 cs, DevState
     if (first_stage)
     {
         __syncthreads(); // every thread of the block has stored its cells
-        block_commit_finalize<NT>(0, 0, 0, 0, 0, st, partial, g, false, false, nblocks, bid, true);
+        block_commit_finalize<NT>(0, 0, 0, 0, 0, st, {partial, nblocks, false, bid}, g, false, false, nblocks, true);
         return;
     }
     __shared__ float red[5][NT / 32];
@@ -529,17 +529,17 @@ __device__ __forceinline__ void block_reduce_finalize32(CellStats32 cs, DevState
         vmax = (double)fv;
         mass = ((double)h + (double)l) * g.dxdy;
     }
-    block_commit_finalize<NT>(amax, umax, vmax, mass, n, st, partial, g, true, false, nblocks, bid);
+    block_commit_finalize<NT>(amax, umax, vmax, mass, n, st, {partial, nblocks, false, bid}, g, true, false, nblocks);
 }
 
-// one case: one 256-thread CTA per active tile of TILE_X x TY cells (32x8:
-// 40 registers, 6 CTAs per SM; 32x16: 5 CTAs per SM; the difference form of
-// HLL_Toro: 3 CTAs per SM, its 32x16 tile holding 62 KB of shared memory)
-template <int SCH, int RIE, int LIM, int TY>
-__global__ void __launch_bounds__(TILE_X *TILE_Y, RIE == HLLT ? 3 : (TY == TILE_Y ? 6 : 5))
+// one case: one 256-thread CTA per active tile of 32x16 cells (5 CTAs per SM;
+// the difference form of HLL_Toro: 3 CTAs per SM, its tile holding 62 KB of
+// shared memory)
+template <int SCH, int RIE, int LIM>
+__global__ void __launch_bounds__(TILE_X *TILE_Y, RIE == HLLT ? 3 : 5)
     sweep_f32_kernel(const __grid_constant__ SweepArgs a)
 {
-    constexpr int NT = TILE_X * TILE_Y;
+    constexpr int NT = TILE_X * TILE_Y, TY = FAST_TILE_Y;
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
     const GridDesc &g = a.g;
@@ -569,20 +569,20 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, RIE == HLLT ? 3 : (TY == TILE_
     block_reduce_finalize32<NT>(cs, st, a.partial, g, a.nblocks ? a.nblocks : gridDim.x, bid, a.stage == 1);
 }
 
-template <int SCH, int RIE, int LIM, int TY>
-void launch_sweep_f32(const SweepArgs &a, dim3 grid, dim3 block, cudaStream_t s)
+template <int SCH, int RIE, int LIM>
+void launch_sweep_f32(const SweepArgs &a, int grid, cudaStream_t s)
 {
-    sweep_f32_kernel<SCH, RIE, LIM, TY><<<grid, block, sizeof(Smem32<RIE, TILE_X, TY>), s>>>(a);
+    sweep_f32_kernel<SCH, RIE, LIM><<<grid, TILE_X * TILE_Y, sizeof(Smem32<RIE, TILE_X, FAST_TILE_Y>), s>>>(a);
 }
 
 // The launcher of one instantiation; a tile whose shared memory exceeds the
 // default 48 KB (the difference form's 32x16 tile) has the limit raised on the
 // current device, once per device, when a case picks the launcher (outside
 // any stream capture).
-template <int SCH, int RIE, int LIM, int TY>
+template <int SCH, int RIE, int LIM>
 SweepLaunch prepared_f32_launcher()
 {
-    constexpr int smem = (int)sizeof(Smem32<RIE, TILE_X, TY>);
+    constexpr int smem = (int)sizeof(Smem32<RIE, TILE_X, FAST_TILE_Y>);
     if (smem > 48 * 1024)
     {
         static std::atomic<unsigned long long> ready{0};
@@ -591,26 +591,25 @@ SweepLaunch prepared_f32_launcher()
         const unsigned long long bit = 1ull << (dev & 63);
         if (!(ready.load() & bit))
         {
-            cudaFuncSetAttribute(sweep_f32_kernel<SCH, RIE, LIM, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem);
+            cudaFuncSetAttribute(sweep_f32_kernel<SCH, RIE, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             ready.fetch_or(bit);
         }
     }
-    return &launch_sweep_f32<SCH, RIE, LIM, TY>;
+    return &launch_sweep_f32<SCH, RIE, LIM>;
 }
 
-// the launchers of one scheme over TILE_X x TY tiles (nullptr: PVRS, FP64 precisions only)
-template <int SCH, int TY>
+// the launchers of one scheme (nullptr: PVRS, FP64 precisions only)
+template <int SCH>
 SweepLaunch select_f32(int riemann, bool vl)
 {
     if (riemann == SW)
-        return vl ? &launch_sweep_f32<SCH, SW, VANLEER, TY> : &launch_sweep_f32<SCH, SW, MINMOD, TY>;
+        return vl ? &launch_sweep_f32<SCH, SW, VANLEER> : &launch_sweep_f32<SCH, SW, MINMOD>;
     if (riemann == HLLCT)
-        return vl ? &launch_sweep_f32<SCH, HLLCT, VANLEER, TY> : &launch_sweep_f32<SCH, HLLCT, MINMOD, TY>;
+        return vl ? &launch_sweep_f32<SCH, HLLCT, VANLEER> : &launch_sweep_f32<SCH, HLLCT, MINMOD>;
     if (riemann == HLLT)
-        return vl ? prepared_f32_launcher<SCH, HLLT, VANLEER, TY>() : prepared_f32_launcher<SCH, HLLT, MINMOD, TY>();
+        return vl ? prepared_f32_launcher<SCH, HLLT, VANLEER>() : prepared_f32_launcher<SCH, HLLT, MINMOD>();
     if (riemann == HLL)
-        return vl ? &launch_sweep_f32<SCH, HLL, VANLEER, TY> : &launch_sweep_f32<SCH, HLL, MINMOD, TY>;
+        return vl ? &launch_sweep_f32<SCH, HLL, VANLEER> : &launch_sweep_f32<SCH, HLL, MINMOD>;
     return nullptr;
 }
 

@@ -4,10 +4,9 @@
 
 namespace ibtfo {
 
-SweepLaunch sweep_launcher_godunov_f32(int riemann, int limiter, int ty)
+SweepLaunch sweep_launcher_godunov_f32(int riemann, int limiter)
 {
-    const bool vl = (limiter == VANLEER);
-    return ty == TILE_Y ? select_f32<GODUNOV, TILE_Y>(riemann, vl) : select_f32<GODUNOV, FAST_TILE_Y>(riemann, vl);
+    return select_f32<GODUNOV>(riemann, limiter == VANLEER);
 }
 
 } // namespace ibtfo

@@ -34,18 +34,39 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *addr, doub
     atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
+// the partial mass sums a step's last block adds up: `n` of them, or with
+// `fine` those of the FINE_X x FINE_Y tiles of each 32x16 tile (lower row
+// first), which are added in the tree of tile_mass_32x16
+struct MassPartials
+{
+    double *p;
+    unsigned n;    // 32x16 tiles (fine), or partials
+    bool fine;
+    unsigned at;   // where the block's own sum goes
+};
+
+__device__ __forceinline__ double mass_partial(const MassPartials &m, unsigned b)
+{
+    const volatile double *p = m.p;
+    if (!m.fine)
+        return p[b];
+    static_assert(TILE_X == 2 * FINE_X && FAST_TILE_Y == 2 * FINE_Y, "four fine tiles in a 32x16 tile");
+    const volatile double *q = p + 4 * (size_t)b;
+    return (q[0] + q[1]) + (q[2] + q[3]);
+}
+
 // Commit one block's (max a, max |u|, max |v|, mass, nan count), held by
 // thread 0, to the step's device state; the last of the case's `nblocks`
 // blocks to finish computes the next dt and advances the reference loop
 // accounting.  Deterministic: the mass partials are summed in a fixed order
-// (by block index `bid`) whichever block finishes last.  Called by every
+// (256 interleaved sums, then a tree) whichever block finishes last and
+// however many threads it has.  Called by every
 // thread of the block.  A first RK2 stage (`first_stage`) commits nothing:
 // its last block only hands the stage's buffer to the boundary pass.
 template <int NT>
 __device__ __forceinline__ void block_commit_finalize(double a, double u, double v, double m, int n, DevState *st,
-                                                      double *partial, const GridDesc &g, bool step_accounting,
-                                                      bool set_start, unsigned nblocks, unsigned bid,
-                                                      bool first_stage = false)
+                                                      const MassPartials &mp, const GridDesc &g, bool step_accounting,
+                                                      bool set_start, unsigned nblocks, bool first_stage = false)
 {
     __shared__ bool last;
     if (first_stage)
@@ -71,7 +92,7 @@ __device__ __forceinline__ void block_commit_finalize(double a, double u, double
         if (u > 0) atomic_max_nonneg(&st->umax_bits, u);
         if (v > 0) atomic_max_nonneg(&st->vmax_bits, v);
         if (n) atomicAdd(&st->nan_step, n);
-        partial[bid] = m;
+        mp.p[mp.at] = m;
         __threadfence();
         unsigned t = atomicAdd(&st->ticket, 1u);
         last = (t == nblocks - 1);
@@ -80,17 +101,21 @@ __device__ __forceinline__ void block_commit_finalize(double a, double u, double
     if (!last)
         return;
     __threadfence();
-    // fixed-order sum of the per-block mass partials
-    __shared__ double msum[NT];
-    double s = 0.0;
-    for (unsigned b = threadIdx.x; b < nblocks; b += NT)
-        s += ((volatile double *)partial)[b];
-    msum[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = NT / 2; h > 0; h >>= 1)
+    // fixed-order sum of the mass partials
+    constexpr int SUMS = 256;
+    __shared__ double msum[SUMS];
+    for (int q = threadIdx.x; q < SUMS; q += NT)
     {
-        if (threadIdx.x < h)
-            msum[threadIdx.x] += msum[threadIdx.x + h];
+        double s = 0.0;
+        for (unsigned b = q; b < mp.n; b += SUMS)
+            s += mass_partial(mp, b);
+        msum[q] = s;
+    }
+    __syncthreads();
+    for (int h = SUMS / 2; h > 0; h >>= 1)
+    {
+        for (int q = threadIdx.x; q < h; q += NT)
+            msum[q] += msum[q + h];
         __syncthreads();
     }
     if (threadIdx.x == 0)
@@ -143,9 +168,10 @@ __device__ __forceinline__ void rk2_average(const double *V, long long o, long l
 // The sound speed enters as its square (a2max); the block takes one square
 // root of the maximum, which equals the maximum of the roots (the root is
 // monotone and correctly rounded; NaN and negative squares drop out of both).
+// The mass of a 32x16 tile's lower and upper eight rows is kept apart.
 struct CellStats
 {
-    double amax = 0.0, a2max = 0.0, umax = 0.0, vmax = 0.0, mass = 0.0;
+    double amax = 0.0, a2max = 0.0, umax = 0.0, vmax = 0.0, mass = 0.0, mass_upper = 0.0;
     int nans = 0;
 };
 
@@ -157,61 +183,136 @@ __device__ __forceinline__ double max_nonneg(double m, double x)
     return (bx > bm && bx <= 0x7ff0000000000000LL) ? x : m;
 }
 
+// The mass of a 32x16 tile, added as a tree over its 8x8 blocks: in a block
+// the columns in pairs, fours and eights, then the rows likewise; then the
+// four blocks of each half, then the halves.  A sum of the same cells swept
+// as 16x8 tiles (mass_partial) has the same bits.  Warp w holds rows w (mass)
+// and w + 8 (mass_upper), lane c column c; thread 0 receives the sum.
+__device__ __forceinline__ double tile_mass_32x16(double lower, double upper)
+{
+    __shared__ double col[2][4][8], half[2];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+    {
+        lower += __shfl_xor_sync(0xffffffffu, lower, o);
+        upper += __shfl_xor_sync(0xffffffffu, upper, o);
+    }
+    if ((lane & 7) == 0)
+    {
+        col[0][lane >> 3][w] = lower;
+        col[1][lane >> 3][w] = upper;
+    }
+    __syncthreads();
+    if (w < 2)
+    {
+        double v = col[w][lane >> 3][lane & 7];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0)
+            half[w] = v;
+    }
+    __syncthreads();
+    return half[0] + half[1];
+}
+
+// The mass of a 16x8 tile: threads 0..127 hold its cells, row-major (a warp
+// two rows of 16); the others take no part.  Thread 0 receives the sum.
+__device__ __forceinline__ double tile_mass_16x8(double v)
+{
+    static_assert(FINE_X == 16 && FINE_Y == 8, "two 8x8 blocks");
+    __shared__ double part[2][4]; // block, pair of rows
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < 4)
+    {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) // the columns of a block
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+        v += __shfl_xor_sync(0xffffffffu, v, 16); // the warp's two rows
+        if ((lane & 7) == 0 && lane < 16)
+            part[lane >> 3][w] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0)
+        return 0.0;
+    return ((part[0][0] + part[0][1]) + (part[0][2] + part[0][3])) +
+           ((part[1][0] + part[1][1]) + (part[1][2] + part[1][3]));
+}
+
 // Block-wide FP64 reduction of the per-thread statistics, then
-// block_commit_finalize.
-template <int NT>
-__device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st, double *partial, const GridDesc &g,
-                                                      bool step_accounting, bool set_start, unsigned nblocks,
-                                                      unsigned bid, bool first_stage = false)
+// block_commit_finalize.  CELLS: the warps that hold updated cells come first
+// (a block with more threads than cells).
+template <int NT, int TX = 0, int TY = 0>
+__device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st, const MassPartials &mp,
+                                                      const GridDesc &g, bool step_accounting, bool set_start,
+                                                      unsigned nblocks, bool first_stage = false)
 {
     if (first_stage)
     {
         __syncthreads(); // every thread of the block has stored its cells
-        block_commit_finalize<NT>(0, 0, 0, 0, 0, st, partial, g, false, false, nblocks, bid, true);
+        block_commit_finalize<NT>(0, 0, 0, 0, 0, st, mp, g, false, false, nblocks, true);
         return;
     }
-    __shared__ double red[5][NT / 32];
-    __shared__ int rnan[NT / 32];
+    constexpr bool TREE = (TX == 32 && TY == 16 && NT == 256) || (TX == FINE_X && TY == FINE_Y);
+    constexpr int CELLS = TX * TY ? TX * TY : NT;
+    constexpr int NW = (CELLS < NT ? CELLS : NT) / 32; // warps with cells
+    __shared__ double red[5][NW];
+    __shared__ int rnan[NW];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double m = 0.0;
+    if constexpr (TREE && TX == 32)
+        m = tile_mass_32x16(cs.mass, cs.mass_upper);
+    if constexpr (TREE && TX == FINE_X)
+        m = tile_mass_16x8(cs.mass);
+    if constexpr (!TREE && TX * TY > NT)
+        cs.mass += cs.mass_upper;
+    if (wid < NW)
+    {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        cs.amax = max_nonneg(cs.amax, __shfl_xor_sync(0xffffffffu, cs.amax, o));
-        cs.a2max = max_nonneg(cs.a2max, __shfl_xor_sync(0xffffffffu, cs.a2max, o));
-        cs.umax = max_nonneg(cs.umax, __shfl_xor_sync(0xffffffffu, cs.umax, o));
-        cs.vmax = max_nonneg(cs.vmax, __shfl_xor_sync(0xffffffffu, cs.vmax, o));
-        cs.mass += __shfl_xor_sync(0xffffffffu, cs.mass, o);
-        cs.nans += __shfl_xor_sync(0xffffffffu, cs.nans, o);
-    }
-    if (lane == 0)
-    {
-        red[0][wid] = cs.amax;
-        red[1][wid] = cs.umax;
-        red[2][wid] = cs.vmax;
-        red[3][wid] = cs.mass;
-        red[4][wid] = cs.a2max;
-        rnan[wid] = cs.nans;
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            cs.amax = max_nonneg(cs.amax, __shfl_xor_sync(0xffffffffu, cs.amax, o));
+            cs.a2max = max_nonneg(cs.a2max, __shfl_xor_sync(0xffffffffu, cs.a2max, o));
+            cs.umax = max_nonneg(cs.umax, __shfl_xor_sync(0xffffffffu, cs.umax, o));
+            cs.vmax = max_nonneg(cs.vmax, __shfl_xor_sync(0xffffffffu, cs.vmax, o));
+            if (!TREE)
+                cs.mass += __shfl_xor_sync(0xffffffffu, cs.mass, o);
+            cs.nans += __shfl_xor_sync(0xffffffffu, cs.nans, o);
+        }
+        if (lane == 0)
+        {
+            red[0][wid] = cs.amax;
+            red[1][wid] = cs.umax;
+            red[2][wid] = cs.vmax;
+            red[3][wid] = cs.mass;
+            red[4][wid] = cs.a2max;
+            rnan[wid] = cs.nans;
+        }
     }
     __syncthreads();
-    double a = 0.0, u = 0.0, v = 0.0, m = 0.0;
+    double a = 0.0, u = 0.0, v = 0.0;
     int n = 0;
     if (threadIdx.x == 0)
     {
         double a2 = red[4][0];
-        a = red[0][0], u = red[1][0], v = red[2][0], m = red[3][0];
+        a = red[0][0], u = red[1][0], v = red[2][0];
         n = rnan[0];
-        for (int w = 1; w < NT / 32; w++)
+        if (!TREE)
+            m = red[3][0];
+        for (int w = 1; w < NW; w++)
         {
             a = max_nonneg(a, red[0][w]);
             a2 = max_nonneg(a2, red[4][w]);
             u = max_nonneg(u, red[1][w]);
             v = max_nonneg(v, red[2][w]);
-            m += red[3][w];
+            if (!TREE)
+                m += red[3][w];
             n += rnan[w];
         }
         a = max_nonneg(a, sqrt_rn(a2));
     }
-    block_commit_finalize<NT>(a, u, v, m, n, st, partial, g, step_accounting, set_start, nblocks, bid);
+    block_commit_finalize<NT>(a, u, v, m, n, st, mp, g, step_accounting, set_start, nblocks);
 }
 
 // any of four values NaN, tested on the integer pipe
@@ -226,7 +327,8 @@ __device__ __forceinline__ int any_nan4(const double v[4])
 
 // CFL and mass contributions of one fluid cell of the new state
 // (ComputeDt.cpp:38-45, CaculateMass.cpp:36)
-__device__ __forceinline__ void cell_stats(const double v[4], double gam, double dx, double dy, CellStats &cs)
+__device__ __forceinline__ void cell_stats(const double v[4], double gam, double dx, double dy, CellStats &cs,
+                                           double &mass)
 {
     double rho = v[0];
     const Divisor by_rho = divisor(rho);
@@ -236,18 +338,18 @@ __device__ __forceinline__ void cell_stats(const double v[4], double gam, double
     cs.a2max = max_nonneg(cs.a2max, divide_rn(gam * p, by_rho)); // pow(gam p / rho, 0.5) taken once per block
     cs.umax = max_nonneg(cs.umax, magnitude(u));
     cs.vmax = max_nonneg(cs.vmax, magnitude(w));
-    cs.mass += v[0] * dx * dy;
+    mass += v[0] * dx * dy;
     cs.nans += any_nan4(v);
 }
 
 // the same statistics from the cell's velocity and internal energy (fp64_fast)
 __device__ __forceinline__ void cell_stats_fast(const double v[4], const Cell64 &c, const GasConst<double> &K,
-                                                double dxdy, CellStats &cs)
+                                                double dxdy, CellStats &cs, double &mass)
 {
     cs.a2max = max_nonneg(cs.a2max, K.ggm1 * (c.ir * c.ei));
     cs.umax = max_nonneg(cs.umax, magnitude(c.u));
     cs.vmax = max_nonneg(cs.vmax, magnitude(c.v));
-    cs.mass += v[0] * dxdy;
+    mass += v[0] * dxdy;
     cs.nans += any_nan4(v);
 }
 
@@ -480,10 +582,12 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
                 V[k * P + (long long)j * pitch + i] = v[k];
             if (stage == 1)
                 continue;
+            // the rows of a tile's upper half are the threads' second cells
+            double &mass = (cell < NT) ? cs.mass : cs.mass_upper;
             if (FAST)
-                cell_stats_fast(v, cl, K, g.dxdy, cs);
+                cell_stats_fast(v, cl, K, g.dxdy, cs, mass);
             else
-                cell_stats(v, gam, g.dx, g.dy, cs);
+                cell_stats(v, gam, g.dx, g.dy, cs, mass);
         }
     }
     // a copy that missed the first wait is waited for once more (bounded);
@@ -492,17 +596,33 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
         mbar_inval(&bar);
 }
 
-// one case: one CTA of TILE_X x TILE_Y threads per active tile of TILE_X x TY
-// cells.  fp64_fast with HLL or Steger-Warming: 32x8 tiles in 64 registers
-// (4 CTAs per SM); 32x16 tiles in 85 registers (3 CTAs per SM, 59 KB of
+// threads of a sweep CTA: one per cell of a 32x8 tile, one for two cells of a 32x16 tile
+template <int TX>
+constexpr int sweep_threads()
+{
+    return TX == FINE_X ? FINE_THREADS : TILE_X * TILE_Y;
+}
+// CTAs per SM the registers are fitted to
+template <int RIE, int FAST, int TX>
+constexpr int sweep_ctas()
+{
+    if (RIE == PVRS)
+        return 1;
+    if (TX == FINE_X)
+        return 5;
+    return (FAST && (RIE == HLL || RIE == SW)) ? 3 : 1;
+}
+
+// one case: one CTA per active tile of TX x TY cells.  fp64_fast with HLL or
+// Steger-Warming: 32x16 tiles in 85 registers (3 CTAs per SM, 59 KB of
 // shared memory each), which measured 4% faster than 512 threads per tile.
-template <int SCH, int RIE, int LIM, int FAST, int TY>
-__global__ void __launch_bounds__(TILE_X *TILE_Y, (FAST && (RIE == HLL || RIE == SW)) ? (TY == TILE_Y ? 4 : 3) : 1)
+template <int SCH, int RIE, int LIM, int FAST, int TX, int TY>
+__global__ void __launch_bounds__(sweep_threads<TX>(), sweep_ctas<RIE, FAST, TX>())
     sweep_kernel(const __grid_constant__ SweepArgs a)
 {
-    constexpr int NT = TILE_X * TILE_Y;
+    constexpr int NT = sweep_threads<TX>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    auto &s = *reinterpret_cast<SweepSmem64<TILE_X, TY> *>(smem_raw);
+    auto &s = *reinterpret_cast<SweepSmem64<TX, TY> *>(smem_raw);
 
     const GridDesc &g = a.g;
     DevState *st = a.st;
@@ -520,30 +640,35 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, (FAST && (RIE == HLL || RIE ==
     // the cell type), so the launch covers the active tiles only
     const unsigned bid = a.tile0 + blockIdx.x;
     const unsigned tile = a.tiles[bid];
-    const int i0 = g.ng + tile_ix(tile) * TILE_X;
+    const int i0 = g.ng + tile_ix(tile) * TX;
     const int j0 = g.ng + tile_jy(tile) * TY;
     const bool interior = (tile & TILE_INTERIOR) != 0;
     CellStats cs;
-    sweep_tile64<SCH, RIE, LIM, FAST, TILE_X, TY, NT>(s, g, U, V, a.type, i0, j0, dt, cs, a.stage,
-                                                      a.tma ? &a.tmap[cur] : nullptr, &st->status, interior);
-    block_reduce_finalize<NT>(cs, st, a.partial, g, true, false, a.nblocks ? a.nblocks : gridDim.x, bid,
-                              a.stage == 1);
+    sweep_tile64<SCH, RIE, LIM, FAST, TX, TY, NT>(s, g, U, V, a.type, i0, j0, dt, cs, a.stage,
+                                                  a.tma ? &a.tmap[cur] : nullptr, &st->status, interior);
+    const unsigned nblocks = a.nblocks ? a.nblocks : gridDim.x;
+    MassPartials mp;
+    mp.p = a.partial;
+    mp.fine = (TX == FINE_X);
+    mp.n = (TX == FINE_X) ? a.nparents : nblocks;
+    mp.at = (TX == FINE_X) ? a.slot[bid] : bid;
+    block_reduce_finalize<NT, TX, TY>(cs, st, mp, g, true, false, nblocks, a.stage == 1);
 }
 
-template <int SCH, int RIE, int LIM, int FAST, int TY = TILE_Y>
-void launch_sweep(const SweepArgs &a, dim3 grid, dim3 block, cudaStream_t s)
+template <int SCH, int RIE, int LIM, int FAST, int TX, int TY>
+void launch_sweep(const SweepArgs &a, int grid, cudaStream_t s)
 {
-    sweep_kernel<SCH, RIE, LIM, FAST, TY><<<grid, block, sizeof(SweepSmem64<TILE_X, TY>), s>>>(a);
+    sweep_kernel<SCH, RIE, LIM, FAST, TX, TY><<<grid, sweep_threads<TX>(), sizeof(SweepSmem64<TX, TY>), s>>>(a);
 }
 
 // The launcher of one instantiation.  A 32 x FAST_TILE_Y tile's shared memory
 // (59 KB) exceeds the default 48 KB limit: the limit is raised on the current
 // device, once per device, when a case picks the launcher (outside any
 // stream capture).
-template <int SCH, int RIE, int LIM, int FAST, int TY>
+template <int SCH, int RIE, int LIM, int FAST, int TX, int TY>
 SweepLaunch prepared_sweep_launcher()
 {
-    constexpr int smem = (int)sizeof(SweepSmem64<TILE_X, TY>);
+    constexpr int smem = (int)sizeof(SweepSmem64<TX, TY>);
     if (smem > 48 * 1024)
     {
         static std::atomic<unsigned long long> ready{0};
@@ -552,12 +677,39 @@ SweepLaunch prepared_sweep_launcher()
         const unsigned long long bit = 1ull << (dev & 63);
         if (!(ready.load() & bit))
         {
-            cudaFuncSetAttribute(sweep_kernel<SCH, RIE, LIM, FAST, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem);
+            cudaFuncSetAttribute(sweep_kernel<SCH, RIE, LIM, FAST, TX, TY>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             ready.fetch_or(bit);
         }
     }
-    return &launch_sweep<SCH, RIE, LIM, FAST, TY>;
+    return &launch_sweep<SCH, RIE, LIM, FAST, TX, TY>;
+}
+
+template <int SCH, int RIE, int FAST>
+SweepLaunch select_sweep_tile(bool vl, bool fine)
+{
+    constexpr int TY = (FAST && RIE != PVRS) ? FAST_TILE_Y : TILE_Y;
+    if (fine)
+        return vl ? prepared_sweep_launcher<SCH, RIE, VANLEER, FAST, FINE_X, FINE_Y>()
+                  : prepared_sweep_launcher<SCH, RIE, MINMOD, FAST, FINE_X, FINE_Y>();
+    return vl ? prepared_sweep_launcher<SCH, RIE, VANLEER, FAST, TILE_X, TY>()
+              : prepared_sweep_launcher<SCH, RIE, MINMOD, FAST, TILE_X, TY>();
+}
+
+// the sweep of one scheme in strict FP64 (FAST = 0: 32x8 tiles) or fp64_fast
+// (32x16, with PVRS 32x8), or over FINE_X x FINE_Y tiles
+template <int SCH, int FAST>
+SweepLaunch select_sweep(int riemann, int limiter, bool fine)
+{
+    const bool vl = (limiter == VANLEER);
+    switch (riemann)
+    {
+    case PVRS: return select_sweep_tile<SCH, PVRS, FAST>(vl, fine);
+    case SW: return select_sweep_tile<SCH, SW, FAST>(vl, fine);
+    case HLLCT: return select_sweep_tile<SCH, HLLCT, FAST>(vl, fine);
+    case HLLT: return select_sweep_tile<SCH, HLLT, FAST>(vl, fine);
+    default: return select_sweep_tile<SCH, HLL, FAST>(vl, fine);
+    }
 }
 
 } // namespace ibtfo

@@ -103,15 +103,15 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) lax_kernel(const SweepArgs a)
         for (int k = 0; k < 4; k++)
             V[k * P + o] = v[k];
         if (a.stage != 1)
-            cell_stats(v, gam, g.dx, g.dy, cs);
+            cell_stats(v, gam, g.dx, g.dy, cs, cs.mass);
     }
-    block_reduce_finalize<NT>(cs, st, a.partial, g, true, false, a.nblocks ? a.nblocks : gridDim.x, bid,
-                              a.stage == 1);
+    const unsigned nblocks = a.nblocks ? a.nblocks : gridDim.x;
+    block_reduce_finalize<NT>(cs, st, {a.partial, nblocks, false, bid}, g, true, false, nblocks, a.stage == 1);
 }
 
-void launch_lax(const SweepArgs &a, dim3 grid, dim3 block, cudaStream_t s)
+void launch_lax(const SweepArgs &a, int grid, cudaStream_t s)
 {
-    lax_kernel<<<grid, block, sizeof(LaxSmem), s>>>(a);
+    lax_kernel<<<grid, TILE_X * TILE_Y, sizeof(LaxSmem), s>>>(a);
 }
 
 } // namespace

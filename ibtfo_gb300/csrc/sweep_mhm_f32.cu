@@ -4,10 +4,9 @@
 
 namespace ibtfo {
 
-SweepLaunch sweep_launcher_mhm_f32(int riemann, int limiter, int ty)
+SweepLaunch sweep_launcher_mhm_f32(int riemann, int limiter)
 {
-    const bool vl = (limiter == VANLEER);
-    return ty == TILE_Y ? select_f32<MHM, TILE_Y>(riemann, vl) : select_f32<MHM, FAST_TILE_Y>(riemann, vl);
+    return select_f32<MHM>(riemann, limiter == VANLEER);
 }
 
 } // namespace ibtfo

@@ -4,17 +4,9 @@
 
 namespace ibtfo {
 
-SweepLaunch sweep_launcher_muscl(int riemann, int limiter)
+SweepLaunch sweep_launcher_muscl(int riemann, int limiter, bool fine)
 {
-    const bool vl = (limiter == VANLEER);
-    switch (riemann)
-    {
-    case PVRS: return vl ? &launch_sweep<MUSCL, PVRS, VANLEER, 0> : &launch_sweep<MUSCL, PVRS, MINMOD, 0>;
-    case SW: return vl ? &launch_sweep<MUSCL, SW, VANLEER, 0> : &launch_sweep<MUSCL, SW, MINMOD, 0>;
-    case HLLCT: return vl ? &launch_sweep<MUSCL, HLLCT, VANLEER, 0> : &launch_sweep<MUSCL, HLLCT, MINMOD, 0>;
-    case HLLT: return vl ? &launch_sweep<MUSCL, HLLT, VANLEER, 0> : &launch_sweep<MUSCL, HLLT, MINMOD, 0>;
-    default: return vl ? &launch_sweep<MUSCL, HLL, VANLEER, 0> : &launch_sweep<MUSCL, HLL, MINMOD, 0>;
-    }
+    return select_sweep<MUSCL, 0>(riemann, limiter, fine);
 }
 
 } // namespace ibtfo
