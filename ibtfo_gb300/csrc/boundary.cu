@@ -28,22 +28,26 @@ namespace ibtfo {
 struct View
 {
     const double *next, *prev;
-    GridDesc g;
+    const GridDesc &g;
     __device__ __forceinline__ double S(long long o, int k, bool from_next) const
     {
         return state_ld(from_next ? next : prev, k, o, g);
     }
 };
 
-// primitives of S at (i, j), as GFM_Bound.cpp:197-212 computes them
-__device__ __forceinline__ void prim(const View &v, int i, int j, bool from_next, double g, double &rho, double &u,
-                                     double &w, double &p)
+// primitives of S at (i, j), as GFM_Bound.cpp:197-212 computes them.  Every
+// quotient of the pass is taken on the integer pipes (divide_rn, the IEEE
+// value): the pass is short, and its FP64 divisions kept the FP64 unit busy
+// for half of it (channel 2048x1024, FP32 form: 14.8 us a pass).
+__device__ __forceinline__ void prim(const View &v, int i, int j, bool from_next, double &rho, double &u, double &w,
+                                     double &p)
 {
     const long long o = (long long)j * v.g.pitch + i;
     rho = v.S(o, 0, from_next);
-    u = v.S(o, 1, from_next) / rho;
-    w = v.S(o, 2, from_next) / rho;
-    p = (g - 1) * (v.S(o, 3, from_next) - 0.5 * rho * (u * u + w * w));
+    const Divisor by_rho = divisor(rho);
+    u = divide_rn(v.S(o, 1, from_next), by_rho);
+    w = divide_rn(v.S(o, 2, from_next), by_rho);
+    p = v.g.gm1 * (v.S(o, 3, from_next) - 0.5 * rho * (u * u + w * w));
 }
 
 // A ghost record is filled by GHOST_LANES consecutive lanes of one warp
@@ -69,10 +73,10 @@ __device__ __forceinline__ double pick4(int c, double x0, double x1, double x2, 
 // of the quad receives all four averages.  nxt: bit c set when corner c is
 // read from the new state.
 __device__ __forceinline__ void idw_average(const View &v, const Quad &q, int idx, int idy, int nxt, const double *a,
-                                            double g, double w[4])
+                                            double w[4])
 {
     double r, u, vv, p;
-    prim(v, idx + (q.c >= 2), idy + (q.c == 1 || q.c == 2), (nxt >> q.c) & 1, g, r, u, vv, p);
+    prim(v, idx + (q.c >= 2), idy + (q.c == 1 || q.c == 2), (nxt >> q.c) & 1, r, u, vv, p);
     double x[4]; // primitive q.c of corners 0..3
 #pragma unroll
     for (int s = 0; s < 4; s++)
@@ -81,21 +85,22 @@ __device__ __forceinline__ void idw_average(const View &v, const Quad &q, int id
         x[s] = pick4(q.c, rs, us, vs, ps);
     }
     const double sum = a[0] + a[1] + a[2] + a[3];
-    const double mine = (a[0] * x[0] + a[1] * x[1] + a[2] * x[2] + a[3] * x[3]) / sum;
+    const double mine = divide_rn(a[0] * x[0] + a[1] * x[1] + a[2] * x[2] + a[3] * x[3], divisor(sum));
 #pragma unroll
     for (int k = 0; k < 4; k++)
         w[k] = q.get(mine, k);
 }
 
 // conserved component q.c of (rho, u, v, p) stored at o
-__device__ __forceinline__ void store_conserved(double *dst, long long o, const GridDesc &gd, const Quad &q, double g,
+__device__ __forceinline__ void store_conserved(double *dst, long long o, const GridDesc &gd, const Quad &q,
                                                 double rho, double u, double v, double p)
 {
-    state_st(dst, q.c, o, pick4(q.c, rho, rho * u, rho * v, p / (g - 1) + 0.5 * rho * (u * u + v * v)), gd);
+    state_st(dst, q.c, o, pick4(q.c, rho, rho * u, rho * v, divide_rn(p, gd.by_gm1) + 0.5 * rho * (u * u + v * v)),
+             gd);
 }
 
 // reflect the normal velocity and store conserved values, GFM_Bound.cpp:219-228
-__device__ __forceinline__ void store_reflected(double *dst, long long o, const GridDesc &gd, const Quad &q, double g,
+__device__ __forceinline__ void store_reflected(double *dst, long long o, const GridDesc &gd, const Quad &q,
                                                 double nx, double ny, double rho_w, double u_w, double v_w,
                                                 double p_w)
 {
@@ -104,18 +109,17 @@ __device__ __forceinline__ void store_reflected(double *dst, long long o, const 
     u_n = -u_n;
     u_w = u_n * nx + u_t * ny;
     v_w = u_n * ny - u_t * nx;
-    store_conserved(dst, o, gd, q, g, rho_w, u_w, v_w, p_w);
+    store_conserved(dst, o, gd, q, rho_w, u_w, v_w, p_w);
 }
 
 __device__ void fill_ghost(const FillArgs &a, const View &v, double *dst, const GhostRec &h, const Quad &q)
 {
-    const double g = a.g.gamma;
     const long long o = (long long)h.j * a.g.pitch + h.i;
     if (a.bc == BC_IDW)
     {
         double w[4];
-        idw_average(v, q, h.idx, h.idy, h.snext, h.w, g, w);
-        store_reflected(dst, o, a.g, q, g, h.nx, h.ny, w[0], w[1], w[2], w[3]);
+        idw_average(v, q, h.idx, h.idy, h.snext, h.w, w);
+        store_reflected(dst, o, a.g, q, h.nx, h.ny, w[0], w[1], w[2], w[3]);
     }
     else if (a.bc == BC_LINEAR || a.bc == BC_RIEMANNGFM)
     {
@@ -126,16 +130,16 @@ __device__ void fill_ghost(const FillArgs &a, const View &v, double *dst, const 
         {
             const int ci = (h.pick == 1 || h.pick == 2) ? h.idx : h.idx + 1;
             const int cj = (h.pick == 1 || h.pick == 4) ? h.idy : h.idy + 1;
-            prim(v, ci, cj, (h.snext >> (h.pick - 1)) & 1, g, rho, u, w, p);
+            prim(v, ci, cj, (h.snext >> (h.pick - 1)) & 1, rho, u, w, p);
         }
-        store_reflected(dst, o, a.g, q, g, h.nx, h.ny, rho, u, w, p);
+        store_reflected(dst, o, a.g, q, h.nx, h.ny, rho, u, w, p);
     }
     else
     {
         // BCGFM/BCGFM_Bound.cpp:89-175 and HBCGFM_Bound.cpp (pure mirror when |phi| > delta)
         double wi[4], we[4];
-        idw_average(v, q, h.idx, h.idy, h.snext, h.w, g, wi);
-        idw_average(v, q, h.idx2, h.idy2, h.snext >> 4, h.w2, g, we);
+        idw_average(v, q, h.idx, h.idy, h.snext, h.w, wi);
+        idw_average(v, q, h.idx2, h.idy2, h.snext >> 4, h.w2, we);
         const double nx = h.nx, ny = h.ny, delta = h.delta, R_E = h.delta, R_G = h.rg;
         double u_n_i = wi[1] * nx + wi[2] * ny;
         double u_t_i = wi[1] * ny - wi[2] * nx;
@@ -151,14 +155,16 @@ __device__ void fill_ghost(const FillArgs &a, const View &v, double *dst, const 
         }
         else
         {
-            rho_m = (wi[0] * ((delta + R_E) * (delta + R_E) - R_G * R_G) - we[0] * (delta * delta - R_G * R_G)) / (R_E * R_E + 2 * delta * R_E);
-            p_m = (wi[3] * ((delta + R_E) * (delta + R_E) - R_G * R_G) - we[3] * (delta * delta - R_G * R_G)) / (R_E * R_E + 2 * delta * R_E);
-            u_t_m = (u_t_i * ((delta + R_E) * (delta + R_E) - R_G * R_G) - u_t_e * (delta * delta - R_G * R_G)) / (R_E * R_E + 2 * delta * R_E);
-            u_n_m = -(u_n_i * ((delta + R_E) * (delta + R_E) - R_G * R_G) - u_n_e * (delta * delta - R_G * R_G)) / (R_E * R_E + 2 * delta * R_E);
+            const Divisor by_r = divisor(R_E * R_E + 2 * delta * R_E);
+            const double ci = (delta + R_E) * (delta + R_E) - R_G * R_G, ce = delta * delta - R_G * R_G;
+            rho_m = divide_rn(wi[0] * ci - we[0] * ce, by_r);
+            p_m = divide_rn(wi[3] * ci - we[3] * ce, by_r);
+            u_t_m = divide_rn(u_t_i * ci - u_t_e * ce, by_r);
+            u_n_m = -divide_rn(u_n_i * ci - u_n_e * ce, by_r);
         }
         double u_m = u_n_m * nx + u_t_m * ny;
         double v_m = u_n_m * ny - u_t_m * nx;
-        store_conserved(dst, o, a.g, q, g, rho_m, u_m, v_m, p_m);
+        store_conserved(dst, o, a.g, q, rho_m, u_m, v_m, p_m);
     }
 }
 
