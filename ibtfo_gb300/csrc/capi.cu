@@ -818,7 +818,7 @@ static ibtfo_status geometry_from_phi(ibtfo_case *c)
     if (rc == 0)
         rc = active_tiles(g, c->type, c->tile_y, &c->band_list, &c->nband_list, c->stream, &tile_list, true);
     if (rc == 0)
-        rc = active_tiles(g, c->type, c->tile_y, &c->tiles, &c->ntiles, c->stream);
+        rc = active_tiles(g, c->type, c->tile_y, &c->tiles, &c->ntiles, c->stream, nullptr, false, c->ccm != nullptr);
     if (rc == 0)
         rc = make_fine(c);
     if (rc == 0)

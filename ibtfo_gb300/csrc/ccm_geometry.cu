@@ -237,46 +237,47 @@ __global__ void small_list_kernel(GridDesc g, const double *__restrict__ alpha, 
     }
 }
 
-// E_k = w_k (U_t - U_s) from the swept state
+// E_k = w_k (U_t - U_s) from the swept state, one thread per component
 __global__ void mix_exchange_kernel(const MixArgs a)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.nex || !a.st->fill_pending)
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, c = threadIdx.x & 3;
+    if (k >= a.nex)
+        return;
+    const MixExchange e = a.ex[k]; // before the device state: the two loads do not wait on one another
+    if (!a.st->fill_pending)
         return;
     const double *buf = a.st->cur ? a.buf1 : a.buf0;
-    const MixExchange e = a.ex[k];
-    for (int c = 0; c < 4; c++)
-        a.e[4 * k + c] = e.w * (state_ld(buf, c, e.t, a.g) - state_ld(buf, c, e.s, a.g));
+    a.e[4 * k + c] = e.w * (state_ld(buf, c, e.t, a.g) - state_ld(buf, c, e.s, a.g));
 }
 
 // U_p += sum of its exchanges (+E as the small cell, -E as a target) / alpha_p,
-// summed in the fixed order of its link list
+// summed in the fixed order of its link list; one thread per component (one
+// thread for all four was a chain of dependent loads four times as long)
 __global__ void mix_apply_kernel(const MixArgs a)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.npart || !a.st->fill_pending)
+    const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, c = threadIdx.x & 3;
+    if (p >= a.npart)
+        return;
+    const MixParticipant q = a.part[p];
+    if (!a.st->fill_pending)
         return;
     double *buf = a.st->cur ? a.buf1 : a.buf0;
-    const MixParticipant q = a.part[p];
-    for (int c = 0; c < 4; c++)
+    double d = 0.0;
+    for (int l = 0; l < q.count; l++)
     {
-        double d = 0.0;
-        for (int l = 0; l < q.count; l++)
-        {
-            const int x = a.links[q.first + l];
-            const double e = a.e[4 * (x >> 1) + c];
-            d += (x & 1) ? -e : e;
-        }
-        state_st(buf, c, q.o, state_ld(buf, c, q.o, a.g) + d * q.inv_alpha, a.g);
+        const int x = a.links[q.first + l];
+        const double e = a.e[4 * (x >> 1) + c];
+        d += (x & 1) ? -e : e;
     }
+    state_st(buf, c, q.o, state_ld(buf, c, q.o, a.g) + d * q.inv_alpha, a.g);
 }
 
 void launch_mix(const MixArgs &a, cudaStream_t s)
 {
     if (a.nex == 0)
         return;
-    mix_exchange_kernel<<<nblk(a.nex, 128), 128, 0, s>>>(a);
-    mix_apply_kernel<<<nblk(a.npart, 128), 128, 0, s>>>(a);
+    mix_exchange_kernel<<<nblk(4LL * a.nex, 128), 128, 0, s>>>(a);
+    mix_apply_kernel<<<nblk(4LL * a.npart, 128), 128, 0, s>>>(a);
     count_launch(2);
 }
 

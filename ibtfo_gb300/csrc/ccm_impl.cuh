@@ -2,8 +2,8 @@
 // reference, which has no cut-cell method: this is a Cartesian cut-cell
 // finite-volume update written from the literature.
 //
-// One CTA per active 32x8 tile, as in sweep_impl.cuh, with the cell types of
-// the tile and its halo staged beside the state:
+// One CTA per active tile, as in sweep_impl.cuh, with the cell types of the
+// tile and its halo staged beside the state where the body is near:
 //   * faces: every X and Y face of the tile; a face whose four-cell stencil
 //     touches a cut or solid cell takes the first-order pair (the two cell
 //     averages), the others the scheme's reconstruction (and MHM predictor);
@@ -35,7 +35,9 @@ struct CcmSmem
     T sF[4][TY + 1][TX + 1];
     T sG[4][TY + 1][TX];
     T sC[4];
-    uint8_t sT[TY + 4][TX + 4];
+    uint8_t sT[TY + 4][TX + 4];      // not staged in an interior tile
+    unsigned short cut[TX * TY];     // the tile's cut cells
+    int ncut[TX * TY / 32];          // cut cells of each 32 cells (a warp's pass)
 };
 
 __device__ __forceinline__ bool low_order_cell(uint8_t t) { return t == CELL_SOLID || t == CELL_CUT; }
@@ -53,7 +55,7 @@ constexpr int ccm_tile_rows()
 }
 
 template <int SCH, int RIE, int LIM, int PREC>
-__global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_kernel(const CcmArgs ca)
+__global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_kernel(const __grid_constant__ CcmArgs ca)
 {
     using T = typename std::conditional<PREC == 2, float, double>::type;
     constexpr int TX = TILE_X, TY = ccm_tile_rows<PREC>(), NT = TILE_X * TILE_Y, WX = TX + 4, WY = TY + 4;
@@ -78,6 +80,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
     const unsigned tile = a.tiles[blockIdx.x];
     const int i0 = g.ng + tile_ix(tile) * TX;
     const int j0 = g.ng + tile_jy(tile) * TY;
+    const bool interior = (tile & TILE_INTERIOR) != 0;
     const int tid = threadIdx.x;
     if (tid == 0)
     {
@@ -95,26 +98,50 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
         s.sC[2] = (T)0.5 * s.sC[0];
         s.sC[3] = (T)0.5 * s.sC[1];
     }
-    // stage the tile, its halo and their cell types: one index computation per cell
-    for (int q = tid; q < WX * WY; q += NT)
+    // stage the tile and its halo: an interior tile by one bulk tensor copy,
+    // without cell types (none is solid or cut within two cells, so every face
+    // is reconstructed and every cell full), others with theirs, one index
+    // computation per cell
+    bool staged = false;
+    __shared__ uint64_t bar;
+    if (interior && a.tma)
     {
-        const int ly = q / WX, lx = q - ly * WX;
-        const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
-        T v[4] = {(T)0, (T)0, (T)0, (T)0};
-        uint8_t t = (uint8_t)CELL_SOLID;
-        if (gi < g.M && gj < g.N)
+        if (tid == 0)
+            mbar_init(&bar, 1);
+        __syncthreads();
+        if (tid == 0)
         {
-            const long long o = (long long)gj * pitch + gi;
+            mbar_expect_tx(&bar, (unsigned)sizeof(s.sU));
+            tma_load_3d(&s.sU[0][0][0], &a.tmap[cur], i0 - 2, j0 - 2, 0, &bar);
+        }
+        staged = __syncthreads_and(mbar_wait(&bar, 0));
+        // as in sweep_tile64: a missed wait fails the step, the tile is staged
+        // element-wise, and the copy is waited for again before the CTA leaves
+        if (!staged && tid == 0)
+            atomicOr(&st->status, STATUS_STALL);
+    }
+    if (!staged)
+        for (int q = tid; q < WX * WY; q += NT)
+        {
+            const int ly = q / WX, lx = q - ly * WX;
+            const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
+            T v[4] = {(T)0, (T)0, (T)0, (T)0};
+            uint8_t t = (uint8_t)CELL_SOLID;
+            if (gi < g.M && gj < g.N)
+            {
+                const long long o = (long long)gj * pitch + gi;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    v[k] = U[k * P + o];
+                if (!interior)
+                    t = a.type[o];
+            }
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                v[k] = U[k * P + o];
-            t = a.type[o];
+                s.sU[k][ly][lx] = v[k];
+            if (!interior)
+                s.sT[ly][lx] = t;
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            s.sU[k][ly][lx] = v[k];
-        s.sT[ly][lx] = t;
-    }
     __syncthreads();
 
     const GasConst<T> K = [&] {
@@ -146,8 +173,9 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
                 c2[k] = s.sU[k][r + 1][fc + 2];
                 c3[k] = s.sU[k][r + 1][fc + 3];
             }
-            const bool lo = low_order_cell(s.sT[r + 1][fc]) || low_order_cell(s.sT[r + 1][fc + 1]) ||
-                            low_order_cell(s.sT[r + 1][fc + 2]) || low_order_cell(s.sT[r + 1][fc + 3]);
+            const bool lo = !interior &&
+                            (low_order_cell(s.sT[r + 1][fc]) || low_order_cell(s.sT[r + 1][fc + 1]) ||
+                             low_order_cell(s.sT[r + 1][fc + 2]) || low_order_cell(s.sT[r + 1][fc + 3]));
             if constexpr (PREC == 2)
                 ccm_face<1, SCH, RIE, LIM>(c0, c1, c2, c3, K, hx2, lo, f);
             else
@@ -168,8 +196,8 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
                 c2[k] = s.sU[k][r + 2][c + 2];
                 c3[k] = s.sU[k][r + 3][c + 2];
             }
-            const bool lo = low_order_cell(s.sT[r][c + 2]) || low_order_cell(s.sT[r + 1][c + 2]) ||
-                            low_order_cell(s.sT[r + 2][c + 2]) || low_order_cell(s.sT[r + 3][c + 2]);
+            const bool lo = !interior && (low_order_cell(s.sT[r][c + 2]) || low_order_cell(s.sT[r + 1][c + 2]) ||
+                                          low_order_cell(s.sT[r + 2][c + 2]) || low_order_cell(s.sT[r + 3][c + 2]));
             if constexpr (PREC == 2)
                 ccm_face<2, SCH, RIE, LIM>(c0, c1, c2, c3, K, hy2, lo, f);
             else
@@ -183,14 +211,22 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
 
     using Stats = typename std::conditional<PREC == 2, CellStats32, CellStats>::type;
     Stats cs;
+    static_assert(TX == 32 && (TX * TY) % NT == 0, "a warp's pass is a row of the tile");
 #pragma unroll 1
     for (int q = tid; q < TX * TY; q += NT)
     {
         const int c = q % TX, r = q / TX;
         const int i = i0 + c, j = j0 + r;
-        const uint8_t t = s.sT[r + 2][c + 2];
+        const bool in = i < g.ng + g.n_x && j < g.ng + g.n_y;
+        const uint8_t t = interior ? (uint8_t)CELL_FLUID : s.sT[r + 2][c + 2];
         const long long o = (long long)j * pitch + i;
-        if (i < g.ng + g.n_x && j < g.ng + g.n_y && t == CELL_FLUID)
+        if (!interior)
+        {
+            const unsigned m = __ballot_sync(0xffffffffu, in && t == CELL_CUT);
+            if ((tid & 31) == 0)
+                s.ncut[r] = __popc(m);
+        }
+        if (in && t == CELL_FLUID)
         {
             const T lx = s.sC[0], ly = s.sC[1];
             if constexpr (PREC == 2)
@@ -247,30 +283,58 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
                 cell_stats_fast(v, cl, K, g.dxdy, cs, cs.mass);
             }
         }
-        else if (i < g.ng + g.n_x && j < g.ng + g.n_y && t == CELL_CUT)
+    }
+    // The tile's cut cells, listed row by row and then taken by consecutive
+    // threads: their FP64 arithmetic (about 100 instructions on a unit that
+    // takes 16 clocks for each, whatever the number of lanes) would otherwise
+    // run for one or two lanes of every warp whose row the outline crosses.
+    // 4096x2048, 24 bodies, FP32 form: the FP64 unit was busy for 59% of the sweep.
+    if (!interior)
+    {
+        __syncthreads();
+        for (int q = tid; q < TX * TY; q += NT)
         {
+            const int c = q % TX, r = q / TX;
+            const bool cut = i0 + c < g.ng + g.n_x && j0 + r < g.ng + g.n_y && s.sT[r + 2][c + 2] == CELL_CUT;
+            const unsigned m = __ballot_sync(0xffffffffu, cut);
+            int at = 0;
+            for (int k = 0; k < r; k++)
+                at += s.ncut[k];
+            if (cut)
+                s.cut[at + __popc(m & ((1u << c) - 1u))] = (unsigned short)q;
+        }
+        int ncut = 0;
+        for (int k = 0; k < TY; k++)
+            ncut += s.ncut[k];
+        __syncthreads();
+        const double lxd = dt * g.idx, lyd = dt * g.idy, K64 = g.ggm1; // gamma (gamma - 1)
+        for (int n = tid; n < ncut; n += NT)
+        {
+            const int c = s.cut[n] % TX, r = s.cut[n] / TX;
+            const long long o = (long long)(j0 + r) * pitch + (i0 + c);
             // FP64: the cell's full state (hi + lo in the FP32 form), apertures,
             // volume fraction and the wall
-            const double al = ca.alpha[o];
+            const double al = ca.alpha[o], ial = rcp_t(al);
             const double aw = ca.ax[o - 1], ae = ca.ax[o], as = ca.ay[o - pitch], an = ca.ay[o];
             const double nLx = (aw - ae) * g.dy, nLy = (as - an) * g.dx;
-            const double L = sqrt(nLx * nLx + nLy * nLy);
+            const double L2 = nLx * nLx + nLy * nLy, L = L2 > 0.0 ? sqrt_t(L2) : 0.0;
             double W[4] = {0.0, 0.0, 0.0, 0.0};
             if (L > 0.0)
             {
+                const double iL = rcp_t(L);
                 T Uc[4], Wt[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     Uc[k] = s.sU[k][r + 2][c + 2];
                 if constexpr (PREC == 2)
-                    ccm_wall_flux<RIE>(Uc, (T)(nLx / L), (T)(nLy / L), K, Wt);
+                    ccm_wall_flux<RIE>(Uc, (T)(nLx * iL), (T)(nLy * iL), K, Wt);
                 else
-                    ccm_wall_flux64<RIE>(Uc, nLx / L, nLy / L, K, Wt);
+                    ccm_wall_flux64<RIE>(Uc, nLx * iL, nLy * iL, K, Wt);
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     W[k] = (double)Wt[k];
             }
-            const double lxd = dt / g.dx, lyd = dt / g.dy, lw = dt / (g.dx * g.dy) * L;
+            const double lw = (lxd * g.idy) * L;
             double v[4];
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -278,36 +342,30 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
                 const double u0 = state_ld(Ud, k, o, g);
                 const double fx = face_term(ae, (double)s.sF[k][r + 1][c + 1]) - face_term(aw, (double)s.sF[k][r + 1][c]);
                 const double gy = face_term(an, (double)s.sG[k][r + 1][c]) - face_term(as, (double)s.sG[k][r][c]);
-                v[k] = (al * u0 - lxd * fx - lyd * gy - lw * W[k]) / al;
+                v[k] = (al * u0 - lxd * fx - lyd * gy - lw * W[k]) * ial;
             }
+            Cell64 cl = cell64(v);
             // the floor only where no mixing follows: a small cell's swept state
             // is provisional (divided by a small alpha) until it is mixed
             if constexpr (safeguarded(RIE))
                 if (al >= 0.5)
-                {
-                    Cell64 cl = cell64(v);
                     pressure_floor64(v, cl);
-                }
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 state_st(Vd, k, o, v[k], g);
             // statistics: mass alpha rho; CFL only from cells that are not mixed
             const double m = al * v[0];
             const bool cfl = al >= 0.5;
-            const double ir = 1.0 / v[0];
-            const double uu = v[1] * ir, ww = v[2] * ir;
-            const double p = (g.gamma - 1.0) * (v[3] - 0.5 * v[0] * (uu * uu + ww * ww));
-            const double snd = sqrt(g.gamma * p * ir);
-            const int bad = (isnan(v[0]) || isnan(v[1]) || isnan(v[2]) || isnan(v[3])) ? 1 : 0;
+            const int bad = any_nan4(v);
             if constexpr (PREC == 2)
             {
                 const float mh = (float)m;
                 two_float_acc(cs.mhi, cs.mlo, mh, (float)(m - (double)mh));
                 if (cfl)
                 {
-                    cs.amax = fmaxf(cs.amax, (float)snd);
-                    cs.umax = fmaxf(cs.umax, (float)fabs(uu));
-                    cs.vmax = fmaxf(cs.vmax, (float)fabs(ww));
+                    cs.amax = fmaxf(cs.amax, (float)sqrt_t(K64 * (cl.ir * cl.ei)));
+                    cs.umax = fmaxf(cs.umax, (float)magnitude(cl.u));
+                    cs.vmax = fmaxf(cs.vmax, (float)magnitude(cl.v));
                 }
                 cs.nans += bad;
             }
@@ -316,14 +374,17 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 1) ccm_sweep_k
                 cs.mass += m * g.dxdy;
                 if (cfl)
                 {
-                    cs.amax = fmax(cs.amax, snd);
-                    cs.umax = fmax(cs.umax, fabs(uu));
-                    cs.vmax = fmax(cs.vmax, fabs(ww));
+                    cs.a2max = max_nonneg(cs.a2max, K64 * (cl.ir * cl.ei));
+                    cs.umax = max_nonneg(cs.umax, magnitude(cl.u));
+                    cs.vmax = max_nonneg(cs.vmax, magnitude(cl.v));
                 }
                 cs.nans += bad;
             }
         }
     }
+    // a copy that missed the first wait is waited for once more (bounded)
+    if (interior && a.tma && tid == 0 && !staged)
+        mbar_wait(&bar, 0);
     if constexpr (PREC == 2)
         block_reduce_finalize32<NT>(cs, st, a.partial, g, gridDim.x, blockIdx.x);
     else

@@ -267,10 +267,11 @@ static inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) 
 
 // per tx x ty sweep tile: the number of interior fluid (or cut) cells it
 // holds, plus TILE_COUNT_INTERIOR when every cell of the tile and of its
-// one-cell ring is an interior fluid cell
+// one-cell ring is an interior fluid cell (`ccm`, a cut-cell case: when the
+// tile lies inside the domain and no cell within two of it is solid or cut)
 constexpr int TILE_COUNT_INTERIOR = 1 << 30;
 __global__ void tile_counts_kernel(GridDesc g, const uint8_t *__restrict__ type, int tx, int ty, int ntx, int nty,
-                                   int *counts)
+                                   int ccm, int *counts)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntx * nty)
@@ -281,26 +282,30 @@ __global__ void tile_counts_kernel(GridDesc g, const uint8_t *__restrict__ type,
     for (int j = j0; j < j0 + ty && j < g.ng + g.n_y; j++)
         for (int i = i0; i < i0 + tx && i < g.ng + g.n_x; i++)
             n += updated_cell(type[(long long)j * g.pitch + i]) ? 1 : 0;
-    bool interior = i0 - 1 >= g.ng && j0 - 1 >= g.ng && i0 + tx < g.ng + g.n_x && j0 + ty < g.ng + g.n_y;
-    for (int j = j0 - 1; j <= j0 + ty && interior; j++)
-        for (int i = i0 - 1; i <= i0 + tx; i++)
-            if (type[(long long)j * g.pitch + i] != CELL_FLUID)
+    const int r = ccm ? 0 : 1, h = ccm ? 2 : 1;
+    bool interior = i0 - r >= g.ng && j0 - r >= g.ng && i0 + tx + r <= g.ng + g.n_x && j0 + ty + r <= g.ng + g.n_y;
+    for (int j = j0 - h; j < j0 + ty + h && interior; j++)
+        for (int i = i0 - h; i < i0 + tx + h; i++)
+        {
+            const uint8_t t = type[(long long)j * g.pitch + i];
+            if (ccm ? (t == CELL_SOLID || t == CELL_CUT) : t != CELL_FLUID)
             {
                 interior = false;
                 break;
             }
+        }
     counts[t] = n | (interior ? TILE_COUNT_INTERIOR : 0);
 }
 
 int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, std::vector<unsigned> &list,
-                     cudaStream_t s, bool row_order)
+                     cudaStream_t s, bool row_order, bool ccm)
 {
     const int ntx = (g.n_x + tx - 1) / tx, nty = (g.n_y + ty - 1) / ty;
     const int n = ntx * nty;
     int *d_counts = nullptr;
     if (cudaMallocAsync(&d_counts, sizeof(int) * n, s) != cudaSuccess)
         return 2;
-    tile_counts_kernel<<<nblk(n, 256), 256, 0, s>>>(g, d_type, tx, ty, ntx, nty, d_counts);
+    tile_counts_kernel<<<nblk(n, 256), 256, 0, s>>>(g, d_type, tx, ty, ntx, nty, ccm ? 1 : 0, d_counts);
     count_launch();
     std::vector<int> counts(n);
     cudaError_t e = cudaMemcpyAsync(counts.data(), d_counts, sizeof(int) * n, cudaMemcpyDeviceToHost, s);
@@ -339,10 +344,10 @@ int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, s
 }
 
 int active_tiles(const GridDesc &g, const uint8_t *d_type, int ty, unsigned **d_tiles, int *ntiles, cudaStream_t s,
-                 std::vector<unsigned> *host_list, bool row_order)
+                 std::vector<unsigned> *host_list, bool row_order, bool ccm)
 {
     std::vector<unsigned> list;
-    int rc = active_tile_list(g, d_type, TILE_X, ty, list, s, row_order);
+    int rc = active_tile_list(g, d_type, TILE_X, ty, list, s, row_order, ccm);
     if (rc)
         return rc;
     if (host_list)

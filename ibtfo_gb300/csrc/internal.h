@@ -229,7 +229,9 @@ constexpr int FINE_X = 16, FINE_Y = 8, FINE_THREADS = 160;
 // A tile-list entry: the tile's column index in bits 0-15, its row index in
 // bits 16-30, and TILE_INTERIOR when every cell of the tile and of the
 // one-cell ring around it is an interior fluid cell (the sweep then solves
-// every face without looking at cell types).
+// every face without looking at cell types).  In a cut-cell case: when no cell
+// of the tile or within two of it is solid or cut, and the tile lies inside
+// the domain.
 constexpr unsigned TILE_INTERIOR = 0x80000000u;
 __host__ __device__ __forceinline__ int tile_ix(unsigned t) { return (int)(t & 0xFFFFu); }
 __host__ __device__ __forceinline__ int tile_jy(unsigned t) { return (int)((t >> 16) & 0x7FFFu); }
@@ -352,13 +354,13 @@ void vtk_writer_destroy(VtkWriter *w, cudaStream_t s);
 // geometry set-up (geometry.cu)
 // the tiles of TILE_X x ty cells holding fluid cells, on the device and (host_list) on the host
 int active_tiles(const GridDesc &g, const uint8_t *d_type, int ty, unsigned **d_tiles, int *ntiles, cudaStream_t s,
-                 std::vector<unsigned> *host_list = nullptr, bool row_order = false);
+                 std::vector<unsigned> *host_list = nullptr, bool row_order = false, bool ccm = false);
 // host list of the tx x ty tiles holding at least one fluid cell (bx | by << 16,
 // with TILE_INTERIOR where it applies): 32x16 tiles longest first unless
 // row_order, others in row order;
 // 0, or 2 (allocation) / 5 (CUDA error)
 int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, std::vector<unsigned> &list,
-                     cudaStream_t s, bool row_order = false);
+                     cudaStream_t s, bool row_order = false, bool ccm = false);
 int setup_geometry(const GridDesc &g, int bc, const double *d_phi, double *d_nx, double *d_ny, uint8_t *d_type,
                    GhostRec **d_ghosts, int *nghost, cudaStream_t s);
 

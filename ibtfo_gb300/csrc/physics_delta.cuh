@@ -59,9 +59,9 @@ __device__ __forceinline__ Prim<float> prim_of_base(const float U[4], const Delt
     return s;
 }
 
-// physical() from the primitive variables: positive density and an internal
+// physical() from the pressure: positive density and an internal
 // energy p / (gamma - 1) above 1e-6 of E (NaN fails)
-__device__ __forceinline__ bool physical_prim(float r, float p, float E, const GasConst<float> &K)
+__device__ __forceinline__ bool physical_pressure(float r, float p, float E, const GasConst<float> &K)
 {
     return r > 0.0f && p * K.igm1 > 1e-6f * fabsf(E);
 }
@@ -164,8 +164,8 @@ __device__ __forceinline__ void face_delta(const float h0[4], const float l0[4],
         }
         L = prim_fast<float, NRM>(UL, K);
         R = prim_fast<float, NRM>(UR, K);
-        if (physical_prim(UcL[0], bL.p, UcL[3], K) && physical_prim(UcR[0], bR.p, UcR[3], K) &&
-            !(physical_prim(L.r, L.p, UL[3], K) && physical_prim(R.r, R.p, UR[3], K)))
+        if (physical_pressure(UcL[0], bL.p, UcL[3], K) && physical_pressure(UcR[0], bR.p, UcR[3], K) &&
+            !(physical_pressure(L.r, L.p, UL[3], K) && physical_pressure(R.r, R.p, UR[3], K)))
         {
             // positivity fallback: the first-order pair (the two cell averages)
 #pragma unroll

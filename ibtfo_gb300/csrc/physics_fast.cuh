@@ -386,7 +386,7 @@ __device__ __forceinline__ bool physical(const T U[4])
 template <typename T>
 __device__ __forceinline__ void positivity_fallback(const T c1[4], const T c2[4], T UL[4], T UR[4])
 {
-    if (!physical(c1) || !physical(c2) || (physical(UL) && physical(UR)))
+    if ((physical(UL) && physical(UR)) || !physical(c1) || !physical(c2))
         return;
 #pragma unroll
     for (int k = 0; k < 4; k++)
@@ -413,6 +413,25 @@ __device__ __forceinline__ bool pressure_floor_energy(const T U[4], T &E)
     return true;
 }
 
+// The flux of a face between cells c1 and c2 from its pair; false: the Y face
+// keeps its slot's X-face flux (HLL only).  SAFE: with the positivity fallback.
+template <typename T, int NRM, int RIE, bool SAFE>
+__device__ __forceinline__ bool face_solve(const T c1[4], const T c2[4], T UL[4], T UR[4], const GasConst<T> &K,
+                                           T F[4])
+{
+    if (SAFE)
+        positivity_fallback(c1, c2, UL, UR);
+    if constexpr (RIE == SW)
+        sw_fast<T, NRM>(UL, UR, K, F);
+    else if constexpr (RIE == HLLCT)
+        hllc_toro<T, NRM>(UL, UR, K, F);
+    else if constexpr (RIE == HLLT)
+        hll_plain<T, NRM>(UL, UR, K, F);
+    else
+        return hll_fast<T, NRM>(UL, UR, K, F);
+    return true;
+}
+
 template <typename T, int SCH, int RIE, int LIM>
 __device__ __forceinline__ void x_face_fast(const T c0[4], const T c1[4], const T c2[4], const T c3[4],
                                             const GasConst<T> &K, T h2, T F[4])
@@ -421,17 +440,7 @@ __device__ __forceinline__ void x_face_fast(const T c0[4], const T c1[4], const 
     face_states_fast<T, SCH, LIM>(c0, c1, c2, c3, UL, UR);
     if (SCH == MHM)
         mhm_predict_fast<T, 1>(UL, UR, K, h2);
-    if constexpr (safeguarded(RIE))
-        if (SCH != GODUNOV)
-            positivity_fallback(c1, c2, UL, UR);
-    if constexpr (RIE == SW)
-        sw_fast<T, 1>(UL, UR, K, F);
-    else if constexpr (RIE == HLLCT)
-        hllc_toro<T, 1>(UL, UR, K, F);
-    else if constexpr (RIE == HLLT)
-        hll_plain<T, 1>(UL, UR, K, F);
-    else
-        hll_fast<T, 1>(UL, UR, K, F);
+    face_solve<T, 1, RIE, safeguarded(RIE) && SCH != GODUNOV>(c1, c2, UL, UR, K, F);
 }
 
 template <typename T, int SCH, int RIE, int LIM>
@@ -442,26 +451,7 @@ __device__ __forceinline__ int y_face_fast(const T c0[4], const T c1[4], const T
     face_states_fast<T, SCH, LIM>(c0, c1, c2, c3, UD, UU);
     if (SCH == MHM)
         mhm_predict_fast<T, 2>(UD, UU, K, h2);
-    if constexpr (safeguarded(RIE))
-        if (SCH != GODUNOV)
-            positivity_fallback(c1, c2, UD, UU);
-    if constexpr (RIE == SW)
-    {
-        sw_fast<T, 2>(UD, UU, K, G);
-        return 0;
-    }
-    else if constexpr (RIE == HLLCT)
-    {
-        hllc_toro<T, 2>(UD, UU, K, G);
-        return 0;
-    }
-    else if constexpr (RIE == HLLT)
-    {
-        hll_plain<T, 2>(UD, UU, K, G);
-        return 0;
-    }
-    else
-        return hll_fast<T, 2>(UD, UU, K, G) ? 0 : 0xF;
+    return face_solve<T, 2, RIE, safeguarded(RIE) && SCH != GODUNOV>(c1, c2, UD, UU, K, G) ? 0 : 0xF;
 }
 
 // ---------------------------------------------------------------- cut cells
@@ -471,18 +461,6 @@ __device__ __forceinline__ int y_face_fast(const T c0[4], const T c1[4], const T
 // slot reuse), Steger-Warming, or the contact-restoring HLLC_Toro; the
 // reference's HLL (the HLL and HLLC keys) has no cut-cell form.
 
-template <typename T, int NRM, int RIE>
-__device__ __forceinline__ void ccm_solve(const T UL[4], const T UR[4], const GasConst<T> &K, T F[4])
-{
-    static_assert(RIE == SW || RIE == HLLCT || RIE == HLLT, "no cut-cell form of this solver");
-    if constexpr (RIE == SW)
-        sw_fast<T, NRM>(UL, UR, K, F);
-    else if constexpr (RIE == HLLCT)
-        hllc_toro<T, NRM>(UL, UR, K, F);
-    else
-        hll_plain<T, NRM>(UL, UR, K, F);
-}
-
 // One face of a cut-cell case, normal NRM (1: X, 2: Y), from the four cells
 // across it.  first_order: a stencil cell is cut or solid, so the face takes
 // the two cell averages (no slopes, no predictor); a reconstructed pair that
@@ -491,8 +469,8 @@ template <int NRM, int SCH, int RIE, int LIM>
 __device__ __forceinline__ void ccm_face(const float c0[4], const float c1[4], const float c2[4], const float c3[4],
                                          const GasConst<float> &K, float h2, bool first_order, float F[4])
 {
-    using T = float;
-    T UL[4], UR[4];
+    static_assert(RIE == SW || RIE == HLLCT || RIE == HLLT, "no cut-cell form of this solver");
+    float UL[4], UR[4];
     if (first_order || SCH == GODUNOV)
     {
 #pragma unroll
@@ -504,12 +482,12 @@ __device__ __forceinline__ void ccm_face(const float c0[4], const float c1[4], c
     }
     else
     {
-        face_states_fast<T, SCH, LIM>(c0, c1, c2, c3, UL, UR);
+        face_states_fast<float, SCH, LIM>(c0, c1, c2, c3, UL, UR);
         if (SCH == MHM)
-            mhm_predict_fast<T, NRM>(UL, UR, K, h2);
-        positivity_fallback(c1, c2, UL, UR); // every cut-cell solver: no face with p <= 0
+            mhm_predict_fast<float, NRM>(UL, UR, K, h2);
     }
-    ccm_solve<T, NRM, RIE>(UL, UR, K, F);
+    // every cut-cell solver: no face with p <= 0 (a first-order pair is the cell averages already)
+    face_solve<float, NRM, RIE, SCH != GODUNOV>(c1, c2, UL, UR, K, F);
 }
 
 // Flux through a wall of outward unit normal (nx, ny) out of a cell of state
@@ -520,16 +498,13 @@ __device__ __forceinline__ void ccm_face(const float c0[4], const float c1[4], c
 template <int RIE>
 __device__ __forceinline__ void ccm_wall_flux(const float U[4], float nx, float ny, const GasConst<float> &K, float W[4])
 {
-    using T = float;
-    const T mn = U[1] * nx + U[2] * ny, mt = -U[1] * ny + U[2] * nx;
-    const T UL[4] = {U[0], mn, mt, U[3]};
-    const T UR[4] = {U[0], -mn, mt, U[3]};
-    T F[4];
-    ccm_solve<T, 1, RIE>(UL, UR, K, F);
-    W[0] = (T)0;
+    const float mn = U[1] * nx + U[2] * ny, mt = -U[1] * ny + U[2] * nx;
+    float UL[4] = {U[0], mn, mt, U[3]}, UR[4] = {U[0], -mn, mt, U[3]}, F[4];
+    face_solve<float, 1, RIE, false>(UL, UR, UL, UR, K, F);
+    W[0] = 0.0f;
     W[1] = F[1] * nx;
     W[2] = F[1] * ny;
-    W[3] = (T)0;
+    W[3] = 0.0f;
 }
 
 } // namespace ibtfo
