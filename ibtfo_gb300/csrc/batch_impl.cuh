@@ -14,12 +14,46 @@
 namespace ibtfo {
 
 template <int SCH, int RIE, int LIM, int PREC, int TX, int TY>
-__global__ void __launch_bounds__(BATCH_THREADS, (PREC == 2 && RIE == HLLT) ? 3 : 1)
+__global__ void __launch_bounds__(f32_threads<SCH, RIE, PREC>(), (PREC == 2 && RIE == HLLT) ? 3 : 1)
     batch_sweep_kernel(const BatchHeader *__restrict__ h, int stage)
 {
-    constexpr int NT = BATCH_THREADS;
+    constexpr int NT = f32_threads<SCH, RIE, PREC>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int ntiles = h->ntiles;
+    // the FP32 difference form stages its next tile while it commits the last
+    __shared__ uint64_t bar;
+    TileStager ts{&bar, 0u, false, false};
+    if constexpr (PREC == 2 && RIE == HLLT)
+    {
+        if (threadIdx.x == 0)
+            mbar_init(&bar, 1);
+        __syncthreads();
+    }
+    // the copy of the first tile from `t` on whose case still runs
+    const auto next_box = [&](int t) {
+        StageBox b{};
+        for (; t < ntiles; t += gridDim.x)
+        {
+            const BatchTile e = h->tiles[t];
+            const SweepArgs &a = h->cases[e.z].s;
+            if (!(a.st->now_t < a.t_end && a.st->iter < a.max_iter))
+                continue;
+            if (!a.tma || TX != TILE_X || TY != FAST_TILE_Y)
+                break;
+            const int cur = a.st->cur;
+            b.map = &a.tmap[cur];
+            tensormap_acquire(b.map);
+            if (stage == 2)
+            {
+                b.vmap = &a.tmap[cur ^ 1];
+                tensormap_acquire(b.vmap);
+            }
+            b.x = a.g.ng + tile_ix(e.x) * TX - 2;
+            b.y = a.g.ng + tile_jy(e.x) * TY - 2;
+            break;
+        }
+        return b;
+    };
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
     {
         const BatchTile e = h->tiles[t];
@@ -45,8 +79,12 @@ __global__ void __launch_bounds__(BATCH_THREADS, (PREC == 2 && RIE == HLLT) ? 3 
             if (a.tma)
             {
                 tm = &a.tmap[cur];
-                if (threadIdx.x == 0)
+                if (threadIdx.x == 0 && !ts.issued)
+                {
                     tensormap_acquire(tm);
+                    if (stage == 2)
+                        tensormap_acquire(&a.tmap[cur ^ 1]);
+                }
             }
         int *status = tm ? &st->status : nullptr;
         if constexpr (PREC == 2)
@@ -56,7 +94,10 @@ __global__ void __launch_bounds__(BATCH_THREADS, (PREC == 2 && RIE == HLLT) ? 3 
             CellStats32 cs;
             if constexpr (RIE == HLLT)
                 sweep_tile32_delta<SCH, RIE, LIM, TX, TY, NT>(*reinterpret_cast<SweepSmem32D<TX, TY> *>(smem_raw), g,
-                                                              U, V, a.type, i0, j0, dt, cs, stage, tm, status,
+                                                              U, V, a.type, i0, j0, dt, cs, stage,
+                                                              StageBox{tm, stage == 2 ? &a.tmap[cur ^ 1] : nullptr,
+                                                                       i0 - 2, j0 - 2},
+                                                              ts, [&] { return next_box(t + gridDim.x); }, status,
                                                               interior);
             else
                 sweep_tile32<SCH, RIE, LIM, TX, TY, NT>(*reinterpret_cast<SweepSmem32<TX, TY> *>(smem_raw), g, U, V,
@@ -86,7 +127,7 @@ struct BatchVariant
     }
     static void launch(const BatchHeader *h, int grid, cudaStream_t s, int stage)
     {
-        batch_sweep_kernel<SCH, RIE, LIM, PREC, TX, TY><<<grid, BATCH_THREADS, smem(), s>>>(h, stage);
+        batch_sweep_kernel<SCH, RIE, LIM, PREC, TX, TY><<<grid, f32_threads<SCH, RIE, PREC>(), smem(), s>>>(h, stage);
     }
     static int prepare()
     {
@@ -94,7 +135,7 @@ struct BatchVariant
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem()) != cudaSuccess)
             return 0;
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, BATCH_THREADS, smem()) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, f32_threads<SCH, RIE, PREC>(), smem()) != cudaSuccess)
             return 0;
         return n;
     }

@@ -148,7 +148,7 @@ struct ibtfo_case
 {
     ibtfo_config cfg;
     GridDesc g;
-    int device = 0;
+    int device = 0, sms = 0;
     cudaStream_t own = nullptr, stream = nullptr;
     double *buf[2] = {nullptr, nullptr};
     double *ic = nullptr;      // Regular: initial state (U_NEW's never-written cells)
@@ -622,6 +622,7 @@ ibtfo_status ibtfo_create(const ibtfo_config *cfg, ibtfo_case **out)
     ibtfo_case *c = new ibtfo_case();
     c->cfg = k;
     cudaGetDevice(&c->device);
+    cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
     GridDesc &g = c->g;
     g.n_x = k.n_x;
     g.n_y = k.n_y;
@@ -965,6 +966,7 @@ static SweepArgs sweep_args(ibtfo_case *c, int guard)
     a.t_end = c->cfg.psy_time;
     a.max_iter = c->cfg.max_iter;
     a.guard = guard;
+    a.sms = c->sms;
     return a;
 }
 

@@ -127,7 +127,9 @@ struct SweepArgs
     int guard;               // apply the reference loop condition before stepping
     int stage;               // 0: one step; Time = RK2: 1 the first stage, 2 the second stage and average
     int tile0;               // a step split over several launches: first tile of this launch
-    int nblocks;             // ... and the tiles of the whole step (0: one launch, its grid)
+    int nblocks;             // ... and the tiles of the whole step (0: one launch, its tiles)
+    int ntiles;              // tiles of this launch (sweeps of persistent CTAs; set by the launcher)
+    int sms;                 // SMs of the device
     const unsigned *slot;    // FINE_X x FINE_Y tiles: where each one's mass sum goes
     unsigned nparents;       // ... and the 32x16 tiles they belong to
     int tma;                 // stage tiles with the tensor maps below (else element-wise loads)

@@ -15,6 +15,7 @@
 // the same bytes as the FP64 path, with the arithmetic on the FP32 pipes.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "internal.h"
@@ -291,28 +292,75 @@ struct SweepSmem32D
     float sU[8][TY + 4][TX + 4]; // planes 0-3 hi, 4-7 lo (the buffer's plane order)
     float sFP[4][TY + 1][TX + 1];
     float sFQ[4][TY + 1][TX + 1];
-    float sGP[4][TY + 1][TX];
-    float sGQ[4][TY + 1][TX];
+    alignas(8) float sGP[4][TY + 1][TX]; // pairs of columns, stored together
+    alignas(8) float sGQ[4][TY + 1][TX];
     float sC[4];
-    unsigned char sKeep[TY + 1][TX]; // no slot reuse under HLL_Toro: cleared, kept for the face list
-    TileFaces<TX, TY> tf;
+    int next; // the CTA has a next tile to stage by copies
+    TilePairs<TX, TY> tf;
 };
+// Threads of an FP32 or batched CTA: 256, or in the FP32 difference form 160,
+// three CTAs per SM, 128 registers (192 threads leave 96: 4% slower on the
+// vortex and in batches, where they spill; 128 threads, or 256 and two CTAs,
+// 4% and 20% slower).  A 32x16 tile's 536 pairs of faces are 3.4 passes.
+constexpr int F32_DELTA_CTAS = 3;
+template <int SCH, int RIE, int PREC>
+constexpr int f32_threads()
+{
+    if (RIE == HLLT && PREC == 2)
+        return 160;
+    return TILE_X * TILE_Y;
+}
 
 // the FP32 tile's shared memory for a Riemann key
 template <int RIE, int TX, int TY>
 using Smem32 = typename std::conditional<RIE == HLLT, SweepSmem32D<TX, TY>, SweepSmem32<TX, TY>>::type;
 
+// Staging of a persistent CTA's tiles by bulk tensor copies: one barrier, a
+// phase for each tile.  While a tile's faces are solved one thread finds the
+// CTA's next tile, and as soon as the update has read the staged planes it
+// issues that tile's copies, so that they run beside this tile's reduction
+// and commit (atomics, a fence and a ticket) and the next one's face list.
+struct TileStager
+{
+    uint64_t *bar;
+    unsigned parity; // of the phase in use or to come
+    bool issued;     // the coming tile's copies are on their way
+    bool dead;       // a copy never arrived: later tiles are staged element-wise
+};
+
+struct StageBox
+{
+    const CUtensorMap *map;  // null: no copy
+    const CUtensorMap *vmap; // RK2's second stage: the output buffer's, brought into L2
+    int x, y;
+};
+
+template <typename Planes>
+__device__ __forceinline__ void stage_box(Planes &sU, const StageBox &b, uint64_t *bar)
+{
+    mbar_expect_tx(bar, (unsigned)sizeof(sU));
+    tma_load_3d(&sU[0][0][0], b.map, b.x, b.y, 0, bar);
+    tma_load_3d(&sU[4][0][0], b.map, b.x, b.y, 4, bar);
+    // the second stage averages with the state the output buffer holds
+    if (b.vmap)
+    {
+        tma_prefetch_3d(b.vmap, b.x, b.y, 0);
+        tma_prefetch_3d(b.vmap, b.x, b.y, 4);
+    }
+}
+
 // sweep_tile32 for HLL_Toro in difference form: the same tile, face list,
 // update, floor, RK2 stages and statistics; the faces store (P, Q) and the
-// update takes P_east - Q_west and P_north - Q_south.  With `tmap` the hi
+// update takes P_east - Q_west and P_north - Q_south.  With `box.map` the hi
 // and lo planes of the box come by two bulk tensor copies (planes 0-3 and
-// 4-7 of the case's 8-plane tensor map).
-template <int SCH, int RIE, int LIM, int TX, int TY, int NT>
+// 4-7 of the case's 8-plane tensor map); `next` gives the box of the CTA's
+// next tile (called by one thread).
+template <int SCH, int RIE, int LIM, int TX, int TY, int NT, typename Next>
 __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, const GridDesc &g,
                                                    const float *__restrict__ U, float *__restrict__ V,
                                                    const uint8_t *__restrict__ type, int i0, int j0, double dt,
-                                                   CellStats32 &cs, int stage = 0, const CUtensorMap *tmap = nullptr,
-                                                   int *status = nullptr, bool interior = false)
+                                                   CellStats32 &cs, int stage, const StageBox &box, TileStager &ts,
+                                                   const Next &next, int *status, bool interior)
 {
     constexpr int WX = TX + 4, WY = TY + 4;
     const long long P = g.plane;
@@ -326,27 +374,17 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
         s.sC[2] = 0.5f * s.sC[0];
         s.sC[3] = 0.5f * s.sC[1];
     }
+    const bool copy = box.map && !ts.dead;
     bool staged = false;
-    __shared__ uint64_t bar;
-    if (tmap)
+    if (copy && !ts.issued && tid == 0)
+        stage_box(s.sU, box, ts.bar);
+    tile_pairs_build<TX, TY, NT>(s.tf, g, type, i0, j0, interior);
+    if (copy)
     {
-        if (tid == 0)
-            mbar_init(&bar, 1);
-        __syncthreads();
-        if (tid == 0)
-        {
-            mbar_expect_tx(&bar, (unsigned)sizeof(s.sU));
-            tma_load_3d(&s.sU[0][0][0], tmap, i0 - 2, j0 - 2, 0, &bar);
-            tma_load_3d(&s.sU[4][0][0], tmap, i0 - 2, j0 - 2, 4, &bar);
-        }
-    }
-    tile_faces_build<TX, TY, NT>(s.tf, s.sKeep, g, type, i0, j0, interior);
-    if (tmap)
-    {
-        staged = __syncthreads_and(mbar_wait(&bar, 0));
+        staged = __syncthreads_and(mbar_wait(ts.bar, ts.parity));
         // as in sweep_tile32: a missed wait fails the step, the tile is staged
-        // element-wise, and the copy is waited for again before the CTA leaves
-        if (!staged && tid == 0 && status)
+        // element-wise, and the copy is waited for again below
+        if (!staged && tid == 0)
             atomicOr(status, STATUS_STALL);
     }
     if (!staged)
@@ -368,61 +406,79 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
         }
     __syncthreads();
 
-    const GasConst<float> K(g.gf, g.gm1f, g.c1f, g.c2f, g.igm1f, g.ig2f);
     const float hx2 = s.sC[2], hy2 = s.sC[3];
-    constexpr int NXF = TileFaces<TX, TY>::NXF;
-    const int nfaces = s.tf.n;
-    for (int t = tid; t < nfaces; t += NT)
+    const GasConst2 K2(g);
+    const int npairs = s.tf.n;
+    for (int t = tid; t < npairs; t += NT)
     {
-        const int q = tile_face(s.tf, t);
-        float h[4][4], l[4][4], fp[4], fq[4];
-        if (q < NXF)
+        const int q = s.tf.all ? t : (int)s.tf.list[t];
+        F2 fp[4], fq[4];
+        if (q < TilePairs<TX, TY>::NXP)
         {
             int r, fc;
-            x_face_of<TX, TY>(q, r, fc);
-#pragma unroll
-            for (int n = 0; n < 4; n++)
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                {
-                    h[n][k] = s.sU[k][r + 1][fc + n];
-                    l[n][k] = s.sU[4 + k][r + 1][fc + n];
-                }
-            face_delta<SCH, LIM, 1>(h[0], l[0], h[1], l[1], h[2], l[2], h[3], l[3], K, hx2, fp, fq);
+            x_pair_of<TX, TY>(q, r, fc);
+            const auto ld = [&](int n, int k) { return f2(s.sU[k][r + 1][fc + n], s.sU[k][r + 2][fc + n]); };
+            face_delta<SCH, LIM, 1>(ld, K2, hx2, fp, fq);
 #pragma unroll
             for (int k = 0; k < 4; k++)
             {
-                s.sFP[k][r][fc] = fp[k];
-                s.sFQ[k][r][fc] = fq[k];
+                s.sFP[k][r][fc] = lo(fp[k]);
+                s.sFP[k][r + 1][fc] = hi(fp[k]);
+                s.sFQ[k][r][fc] = lo(fq[k]);
+                s.sFQ[k][r + 1][fc] = hi(fq[k]);
             }
         }
         else
         {
             int r, c;
-            y_face_of<TX, TY>(q, r, c);
-#pragma unroll
-            for (int n = 0; n < 4; n++)
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                {
-                    h[n][k] = s.sU[k][r + n][c + 2];
-                    l[n][k] = s.sU[4 + k][r + n][c + 2];
-                }
-            face_delta<SCH, LIM, 2>(h[0], l[0], h[1], l[1], h[2], l[2], h[3], l[3], K, hy2, fp, fq);
+            y_pair_of<TX, TY>(q, r, c);
+            const auto ld = [&](int n, int k) { return *reinterpret_cast<const F2 *>(&s.sU[k][r + n][c + 2]); };
+            face_delta<SCH, LIM, 2>(ld, K2, hy2, fp, fq);
 #pragma unroll
             for (int k = 0; k < 4; k++)
             {
-                s.sGP[k][r][c] = fp[k];
-                s.sGQ[k][r][c] = fq[k];
+                *reinterpret_cast<F2 *>(&s.sGP[k][r][c]) = fp[k];
+                *reinterpret_cast<F2 *>(&s.sGQ[k][r][c]) = fq[k];
             }
         }
     }
+    // the first thread of the last warp, which has the fewest pairs
+    StageBox nb{};
+    if (tid == NT - 32)
+    {
+        nb = next();
+        s.next = nb.map ? 1 : 0;
+    }
+    // second stage: the output buffer's state of a thread's first cell, asked
+    // for before the wait for the other warps' faces, and in the loop below of
+    // the next cell before this one is updated (198 -> 191 us a step on
+    // 1800x1100; with the MHM predictor the registers are full and it costs 1%)
+    constexpr bool AHEAD = SCH != MHM;
+    float old[8];
+    const auto load_old = [&](int cell) {
+        const int c = cell % TX, r = cell / TX;
+        if (stage == 2 && cell < TX * TY && (s.tf.all || s.tf.fluid[r + 1][c + 1]))
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                old[k] = V[k * P + (long long)(j0 + r) * pitch + (i0 + c)];
+    };
+    if (AHEAD)
+        load_old(tid);
     __syncthreads();
 
+    const GasConst<float> K(g.gf, g.gm1f, g.c1f, g.c2f, g.igm1f, g.ig2f);
     for (int cell = tid; cell < TX * TY; cell += NT)
     {
         const int c = cell % TX, r = cell / TX;
-        if (tile_cell_fluid(s.tf, r, c))
+        if (!AHEAD)
+            load_old(cell);
+        float was[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            was[k] = old[k];
+        if (AHEAD)
+            load_old(cell + NT);
+        if (s.tf.all || s.tf.fluid[r + 1][c + 1])
         {
             const long long o = (long long)(j0 + r) * pitch + (i0 + c);
             const float lx = s.sC[0], ly = s.sC[1];
@@ -447,7 +503,7 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
             {
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    two_float_average(hi[k], lo[k], V[k * P + o], V[(4 + k) * P + o]);
+                    two_float_average(hi[k], lo[k], was[k], was[4 + k]);
             }
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -467,10 +523,16 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
             cs.nans += (isnan(hi[0]) || isnan(hi[1]) || isnan(hi[2]) || isnan(hi[3])) ? 1 : 0;
         }
     }
-    // a copy that missed the first wait is waited for once more (bounded);
-    // the barrier is then released for the next tile of a persistent CTA
-    if (tmap && tid == 0 && (staged || mbar_wait(&bar, 0)))
-        mbar_inval(&bar);
+    // a copy that missed the first wait is waited for once more (bounded), so
+    // that it lands while this tile owns the planes
+    if (copy && !staged && !__syncthreads_and(mbar_wait(ts.bar, ts.parity)))
+        ts.dead = true;
+    else if (copy)
+        ts.parity ^= 1;
+    __syncthreads(); // the planes have been read
+    ts.issued = s.next && !ts.dead;
+    if (ts.issued && tid == NT - 32)
+        stage_box(s.sU, nb, ts.bar);
 }
 
 // Block reduction in FP32 (compensated for the mass); thread 0 converts the
@@ -532,14 +594,14 @@ __device__ __forceinline__ void block_reduce_finalize32(CellStats32 cs, DevState
     block_commit_finalize<NT>(amax, umax, vmax, mass, n, st, {partial, nblocks, false, bid}, g, true, false, nblocks);
 }
 
-// one case: one 256-thread CTA per active tile of 32x16 cells (5 CTAs per SM;
-// the difference form of HLL_Toro: 3 CTAs per SM, its tile holding 62 KB of
-// shared memory)
+// one case: one CTA per active tile of 32x16 cells (256 threads, 5 CTAs per SM;
+// the difference form of HLL_Toro: 160 or 192, 3 CTAs per SM, its tile
+// holding 61 KB of shared memory)
 template <int SCH, int RIE, int LIM>
-__global__ void __launch_bounds__(TILE_X *TILE_Y, RIE == HLLT ? 3 : 5)
+__global__ void __launch_bounds__(f32_threads<SCH, RIE, 2>(), RIE == HLLT ? F32_DELTA_CTAS : 5)
     sweep_f32_kernel(const __grid_constant__ SweepArgs a)
 {
-    constexpr int NT = TILE_X * TILE_Y, TY = FAST_TILE_Y;
+    constexpr int NT = f32_threads<SCH, RIE, 2>(), TY = FAST_TILE_Y;
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
     const GridDesc &g = a.g;
@@ -552,27 +614,60 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, RIE == HLLT ? 3 : 5)
     const int cur = st->cur;
     const float *U = reinterpret_cast<const float *>(cur ? a.buf1 : a.buf0);
     float *V = reinterpret_cast<float *>(cur ? a.buf0 : a.buf1);
-    const unsigned bid = a.tile0 + blockIdx.x;
-    const unsigned tile = a.tiles[bid];
-    const int i0 = g.ng + tile_ix(tile) * TILE_X;
-    const int j0 = g.ng + tile_jy(tile) * TY;
-    const bool interior = (tile & TILE_INTERIOR) != 0;
-    CellStats32 cs;
     if constexpr (RIE == HLLT)
-        sweep_tile32_delta<SCH, RIE, LIM, TILE_X, TY, NT>(*reinterpret_cast<SweepSmem32D<TILE_X, TY> *>(smem_raw), g,
-                                                          U, V, a.type, i0, j0, dt, cs, a.stage,
-                                                          a.tma ? &a.tmap[cur] : nullptr, &st->status, interior);
+    {
+        // persistent: the grid is the resident CTAs, each takes every
+        // gridDim.x-th tile of the launch
+        __shared__ uint64_t bar;
+        if (threadIdx.x == 0)
+            mbar_init(&bar, 1);
+        __syncthreads();
+        TileStager ts{&bar, 0u, false, false};
+        auto &s = *reinterpret_cast<SweepSmem32D<TILE_X, TY> *>(smem_raw);
+        const auto box_of = [&](unsigned t) {
+            StageBox b{};
+            if (t >= (unsigned)a.ntiles || !a.tma)
+                return b;
+            const unsigned tile = a.tiles[a.tile0 + t];
+            b.map = &a.tmap[cur];
+            b.vmap = a.stage == 2 ? &a.tmap[cur ^ 1] : nullptr;
+            b.x = g.ng + tile_ix(tile) * TILE_X - 2;
+            b.y = g.ng + tile_jy(tile) * TY - 2;
+            return b;
+        };
+        for (unsigned t = blockIdx.x; t < (unsigned)a.ntiles; t += gridDim.x)
+        {
+            const unsigned bid = a.tile0 + t, tile = a.tiles[bid];
+            const int i0 = g.ng + tile_ix(tile) * TILE_X, j0 = g.ng + tile_jy(tile) * TY;
+            CellStats32 cs;
+            sweep_tile32_delta<SCH, RIE, LIM, TILE_X, TY, NT>(
+                s, g, U, V, a.type, i0, j0, dt, cs, a.stage, box_of(t), ts, [&] { return box_of(t + gridDim.x); },
+                &st->status, (tile & TILE_INTERIOR) != 0);
+            block_reduce_finalize32<NT>(cs, st, a.partial, g, a.nblocks ? a.nblocks : a.ntiles, bid, a.stage == 1);
+        }
+    }
     else
+    {
+        const unsigned bid = a.tile0 + blockIdx.x;
+        const unsigned tile = a.tiles[bid];
+        const int i0 = g.ng + tile_ix(tile) * TILE_X;
+        const int j0 = g.ng + tile_jy(tile) * TY;
+        CellStats32 cs;
         sweep_tile32<SCH, RIE, LIM, TILE_X, TY, NT>(*reinterpret_cast<SweepSmem32<TILE_X, TY> *>(smem_raw), g, U, V,
                                                     a.type, i0, j0, dt, cs, a.stage, a.tma ? &a.tmap[cur] : nullptr,
-                                                    &st->status, interior);
-    block_reduce_finalize32<NT>(cs, st, a.partial, g, a.nblocks ? a.nblocks : gridDim.x, bid, a.stage == 1);
+                                                    &st->status, (tile & TILE_INTERIOR) != 0);
+        block_reduce_finalize32<NT>(cs, st, a.partial, g, a.nblocks ? a.nblocks : gridDim.x, bid, a.stage == 1);
+    }
 }
 
 template <int SCH, int RIE, int LIM>
-void launch_sweep_f32(const SweepArgs &a, int grid, cudaStream_t s)
+void launch_sweep_f32(const SweepArgs &a0, int grid, cudaStream_t s)
 {
-    sweep_f32_kernel<SCH, RIE, LIM><<<grid, TILE_X * TILE_Y, sizeof(Smem32<RIE, TILE_X, FAST_TILE_Y>), s>>>(a);
+    SweepArgs a = a0;
+    a.ntiles = grid;
+    if (RIE == HLLT)
+        grid = std::min(grid, F32_DELTA_CTAS * a.sms);
+    sweep_f32_kernel<SCH, RIE, LIM><<<grid, f32_threads<SCH, RIE, 2>(), sizeof(Smem32<RIE, TILE_X, FAST_TILE_Y>), s>>>(a);
 }
 
 // The launcher of one instantiation; a tile whose shared memory exceeds the

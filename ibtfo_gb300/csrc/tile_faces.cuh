@@ -158,4 +158,102 @@ __device__ __forceinline__ bool x_face_listed(const TileFaces<TX, TY> &f, int r,
     return r > 0 && (f.all || f.fluid[r][fc] || f.fluid[r][fc + 1]);
 }
 
+// ---------------------------------------------------------------- pairs of faces
+//
+// The FP32 difference form solves faces two at a time: X faces of rows r and
+// r + 1 (the same column), Y faces of columns c and c + 1 (the same row), so
+// that a warp reads whole rows of the staged tile either way.  A pair is listed
+// when one of its faces is read by a fluid cell; the other's value then goes
+// unread.
+template <int TX, int TY>
+struct TilePairs
+{
+    static constexpr int NXP = (TX + 1) * TY / 2; // X faces of the tile's rows
+    static constexpr int NYP = TX / 2 * (TY + 1); // Y faces below, inside and above the tile
+    unsigned char fluid[TY + 2][TX + 2];          // as in TileFaces
+    unsigned short list[NXP + NYP];
+    int n, all;
+};
+
+// X pair q < NXP: sF rows r and r + 1 (r odd, 1..TY-1), column fc
+template <int TX, int TY>
+__device__ __forceinline__ void x_pair_of(int q, int &r, int &fc)
+{
+    if (q < TX * TY / 2)
+        r = 2 * (q / TX) + 1, fc = q % TX;
+    else
+        r = 2 * (q - TX * TY / 2) + 1, fc = TX;
+}
+
+// Y pair q >= NXP: sG row r (0..TY), columns c and c + 1 (c even)
+template <int TX, int TY>
+__device__ __forceinline__ void y_pair_of(int q, int &r, int &c)
+{
+    const int qq = q - TilePairs<TX, TY>::NXP;
+    r = qq / (TX / 2);
+    c = 2 * (qq - r * (TX / 2));
+}
+
+// flags and list as tile_faces_build; all NT threads call it, ends with a barrier
+template <int TX, int TY, int NT>
+__device__ __forceinline__ void tile_pairs_build(TilePairs<TX, TY> &f, const GridDesc &g,
+                                                 const uint8_t *__restrict__ type, int i0, int j0, bool interior)
+{
+    constexpr int W = TX + 2, H = TY + 2;
+    constexpr int NC = TilePairs<TX, TY>::NXP + TilePairs<TX, TY>::NYP;
+    const int tid = threadIdx.x;
+    int mine = 1;
+    if (!interior)
+        for (int q = tid; q < W * H; q += NT)
+        {
+            const int ly = q / W, lx = q - ly * W;
+            const int i = i0 - 1 + lx, j = j0 - 1 + ly;
+            const bool in = i >= g.ng && i < g.ng + g.n_x && j >= g.ng && j < g.ng + g.n_y;
+            const int fl = in && type[(long long)j * g.pitch + i] == 0;
+            f.fluid[ly][lx] = (unsigned char)fl;
+            mine &= fl;
+        }
+    if (tid == 0)
+        f.n = 0;
+    const int all = __syncthreads_and(mine);
+    if (all)
+    {
+        if (tid == 0)
+        {
+            f.n = NC;
+            f.all = 1;
+        }
+        __syncthreads();
+        return;
+    }
+    const int lane = tid & 31;
+    for (int base = 0; base < NC; base += NT)
+    {
+        const int q = base + tid;
+        bool need = false;
+        if (q < TilePairs<TX, TY>::NXP)
+        {
+            int r, fc;
+            x_pair_of<TX, TY>(q, r, fc);
+            need = f.fluid[r][fc] | f.fluid[r][fc + 1] | f.fluid[r + 1][fc] | f.fluid[r + 1][fc + 1];
+        }
+        else if (q < NC)
+        {
+            int r, c;
+            y_pair_of<TX, TY>(q, r, c);
+            need = f.fluid[r][c + 1] | f.fluid[r + 1][c + 1] | f.fluid[r][c + 2] | f.fluid[r + 1][c + 2];
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, need);
+        int off = 0;
+        if (lane == 0 && m)
+            off = atomicAdd(&f.n, __popc(m));
+        off = __shfl_sync(0xffffffffu, off, 0);
+        if (need)
+            f.list[off + __popc(m & ((1u << lane) - 1u))] = (unsigned short)q;
+    }
+    if (tid == 0)
+        f.all = 0;
+    __syncthreads();
+}
+
 } // namespace ibtfo

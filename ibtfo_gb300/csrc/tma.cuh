@@ -39,6 +39,15 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
                  : "memory");
 }
 
+// asks for one 3-D box of the tensor to be brought into L2
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(z)
+                 : "memory");
+}
+
 // true once the barrier's phase `parity` has completed
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity)
 {
