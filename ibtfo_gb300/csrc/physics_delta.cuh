@@ -22,10 +22,10 @@
 // Two faces are solved at once in packed FP32 arithmetic (one instruction for
 // two operations, each half rounding as the single one does): a third fewer
 // instructions (vortex 2048^2: 158.7 M -> 108.4 M warp instructions a sweep).
-// The bits are those of the single form.  The gain in time is smaller (the
-// registers of two faces leave 15 warps per SM, not 24; issue 69% -> 52%): with
-// the staging of sweep_tile32_delta, cylinder 1800x1100 MUSCL + RK2 214 -> 191
-// us a step, vortex 2048^2 MHM + RK2 461 -> 447 us, 4096^2 1.70 -> 1.63 ms.
+// The bits are those of the single form.  The gain in time is smaller, since
+// the registers of two faces leave 15 warps per SM, not 24.  With the staging
+// of sweep_tile32_delta, per step: cylinder 1800x1100 MUSCL + RK2 214-216 ->
+// 192-197 us, vortex MHM + RK2 2048^2 460 -> 449 us, 4096^2 1.70 -> 1.65 ms.
 // The algorithm is HLL_Toro's (MUSCL / MHM / Godunov reconstruction with the
 // limiter, the positivity fallback and the same HLL flux); only the order of
 // evaluation differs.

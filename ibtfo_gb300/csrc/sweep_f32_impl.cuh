@@ -451,8 +451,9 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
     }
     // second stage: the output buffer's state of a thread's first cell, asked
     // for before the wait for the other warps' faces, and in the loop below of
-    // the next cell before this one is updated (198 -> 191 us a step on
-    // 1800x1100; with the MHM predictor the registers are full and it costs 1%)
+    // the next cell before this one is updated.  With the MHM predictor the
+    // registers are full: there the state is read where it is averaged (vortex
+    // 2048^2 449 us a step, 455 with the state loaded into registers first)
     constexpr bool AHEAD = SCH != MHM;
     float old[8];
     const auto load_old = [&](int cell) {
@@ -470,14 +471,14 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
     for (int cell = tid; cell < TX * TY; cell += NT)
     {
         const int c = cell % TX, r = cell / TX;
-        if (!AHEAD)
-            load_old(cell);
         float was[8];
+        if constexpr (AHEAD)
+        {
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            was[k] = old[k];
-        if (AHEAD)
+            for (int k = 0; k < 8; k++)
+                was[k] = old[k];
             load_old(cell + NT);
+        }
         if (s.tf.all || s.tf.fluid[r + 1][c + 1])
         {
             const long long o = (long long)(j0 + r) * pitch + (i0 + c);
@@ -503,7 +504,10 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
             {
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    two_float_average(hi[k], lo[k], was[k], was[4 + k]);
+                    if constexpr (AHEAD)
+                        two_float_average(hi[k], lo[k], was[k], was[4 + k]);
+                    else
+                        two_float_average(hi[k], lo[k], V[k * P + o], V[(4 + k) * P + o]);
             }
 #pragma unroll
             for (int k = 0; k < 4; k++)
