@@ -64,6 +64,7 @@ __device__ __forceinline__ double pow_half(double x)
 //   for doubles |a| > |b| implies |a|/|b| >= 1 + ulp(b)/|b| > 1 + 2^-53,
 //   which rounds above 1, and |a| <= |b| gives a quotient <= 1; magnitudes of
 //   non-NaN doubles order like their bit patterns.
+static __device__ __noinline__ bool product_positive(double a, double b) { return (a * b) > 0; }
 __device__ __forceinline__ double lim_minmod(double a, double b)
 {
     const long long ma = magnitude_bits(a), mb = magnitude_bits(b);
@@ -73,7 +74,7 @@ __device__ __forceinline__ double lim_minmod(double a, double b)
     {
         const int ea = (int)(ma >> 52), eb = (int)(mb >> 52);
         if (!(ea != 0 && eb != 0 && ea + eb >= 972))
-            pos = (a * b) > 0;
+            pos = product_positive(a, b);
     }
     return pos ? ((ma > mb) ? b : a) : 0.0;
 }

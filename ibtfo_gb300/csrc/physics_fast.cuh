@@ -49,18 +49,23 @@ struct GasConst<double>
 // 1/x of a double on the integer pipes (int64math.cuh; no FP64 instruction,
 // four before).  Zero, subnormal and non-finite x, and results near the ends
 // of the exponent range: the hardware estimate of the double's high word and
-// two Newton steps.
-__device__ __forceinline__ double rcp_t(double x)
+// two Newton steps, in a call: a short rare path is if-converted, and its
+// predicated FP64 instructions then take the unit's time in every face (with
+// those of lim_minmod and above_fraction: Sod 400x100 strict 17.4 -> 17.0 ms
+// to its end, 2048x1024 fp64_fast within the noise).
+static __device__ __noinline__ double rcp_hardware(double x)
 {
-    const uint64_t b = double_bits(x);
-    if (rcp_range(b))
-        return rcp_int(b);
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     double e = fma(-x, y, 1.0);
     y = fma(y, e, y);
     e = fma(-x, y, 1.0);
     return fma(y, e, y);
+}
+__device__ __forceinline__ double rcp_t(double x)
+{
+    const uint64_t b = double_bits(x);
+    return rcp_range(b) ? rcp_int(b) : rcp_hardware(x);
 }
 // FP32 form: hardware reciprocal seed + one Newton step (within ~1 ulp; no
 // correctly-rounded slow path), and the hardware square root approximation

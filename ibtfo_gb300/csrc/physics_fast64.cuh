@@ -216,13 +216,14 @@ __device__ __forceinline__ void mhm_predict64(double UL[4], double UR[4], const 
 // where x / |E| is well above it: a high word is a number's exponent and the
 // leading bits of its significand, so that a difference above -(DROP << 20)
 // means x / |E| > 2^-(DROP + 0.1); closer values are compared in FP64
+static __device__ __noinline__ bool above_fraction_fp64(double x, double E, double f) { return x > f * fabs(E); }
 template <int DROP>
 __device__ __forceinline__ bool above_fraction(double x, double E, double f)
 {
     const int hx = __double2hiint(x), hE = __double2hiint(E) & 0x7fffffff;
     if (hx >= 0x00100000 && hx < 0x7ff00000 && hE < 0x7ff00000 && hx - hE >= -(DROP << 20))
         return true;
-    return x > f * fabs(E);
+    return above_fraction_fp64(x, E, f);
 }
 // positive density and an internal energy above 1e-6 E (physical())
 __device__ __forceinline__ bool physical64(const Prim64 &s)
@@ -248,12 +249,17 @@ __device__ __forceinline__ Cell64 cell64(const double U[4])
 
 // the pressure floor (pressure_floor_energy) of an updated cell: raises U[3]
 // and c.ei where the internal energy is below 1e-5 E
+static __device__ __noinline__ double floored_energy(double rho, double ei, double E)
+{
+    const double f = 1e-5 * fabs(E);
+    return (rho > 0.0 && !(ei >= f)) ? f : ei;
+}
 __device__ __forceinline__ void pressure_floor64(double U[4], Cell64 &c)
 {
-    if (above_fraction<15>(c.ei, U[3], 1e-5) || !(U[0] > 0.0))
+    if (above_fraction<15>(c.ei, U[3], 1e-5))
         return;
-    const double f = 1e-5 * fabs(U[3]);
-    if (c.ei >= f)
+    const double f = floored_energy(U[0], c.ei, U[3]);
+    if (__double_as_longlong(f) == __double_as_longlong(c.ei))
         return;
     U[3] = (U[3] - c.ei) + f;
     c.ei = f;
