@@ -641,15 +641,12 @@ ibtfo_status ibtfo_create(const ibtfo_config *cfg, ibtfo_case **out)
     g.f32 = (k.precision == IBTFO_PRECISION_FP32_COMPENSATED) ? 1 : 0;
     set_derived_constants(g);
     c->nblocks = ((k.n_x + TILE_X - 1) / TILE_X) * ((k.n_y + TILE_Y - 1) / TILE_Y);
-    // rows per tile: the fp64_fast and FP32 sweeps and the FP32 cut-cell sweep
-    // run 32 x FAST_TILE_Y tiles, except with PVRS; Lax, the strict form and
-    // the FP64 cut-cell sweeps 32x8 (ccm_tile_rows in csrc/ccm_impl.cuh)
+    // rows per tile: the FP64 and FP32 sweeps and the FP32 cut-cell sweep run
+    // 32 x FAST_TILE_Y tiles, except with PVRS; Lax and the FP64 cut-cell
+    // sweeps 32x8 (ccm_tile_rows in csrc/ccm_impl.cuh)
     const bool ccm = k.boundary == IBTFO_BOUNDARY_CCM;
     const bool f32 = k.precision == IBTFO_PRECISION_FP32_COMPENSATED;
-    c->tile_y = ((k.precision == IBTFO_PRECISION_FP64_FAST && !ccm) || f32) && k.scheme != IBTFO_SCHEME_LAX &&
-                        k.riemann != IBTFO_RIEMANN_PVRS
-                    ? FAST_TILE_Y
-                    : TILE_Y;
+    c->tile_y = (!ccm || f32) && k.scheme != IBTFO_SCHEME_LAX && k.riemann != IBTFO_RIEMANN_PVRS ? FAST_TILE_Y : TILE_Y;
     if (ccm)
         c->ccm = ccm_launcher(k.scheme, k.riemann, k.limiter, k.precision);
     else
@@ -724,21 +721,22 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
     return geometry_from_phi(c);
 }
 
-// Up to how many active 32x16 tiles the fp64_fast sweeps take 16x8 tiles.  A
+// Up to how many active 32x16 tiles the FP64 sweeps take 16x8 tiles.  A
 // 32x16 CTA lasts 45 us, most of it latency, and few of them leave SMs idle;
-// four 16x8 CTAs in its place spread over the SMs but solve 5% more faces and
-// reduce four times.  Measured (GB300, 152 SMs; us per step, 32x16 / 16x8
-// tiles): 48x24 cells 44 / 24, 256x128 (64 tiles) 46 / 30, channel 600x300
+// four 16x8 CTAs in its place spread over the SMs but solve 5% more faces, in
+// 40 warp passes where it takes 35 (136 X and 144 Y faces do not fill their
+// warps), and reduce four times.  Measured (GB300, 152 SMs; us per step, 32x16
+// / 16x8 tiles): fp64_fast 48x24 cells 44 / 24, 256x128 (64 tiles) 46 / 30, channel 600x300
 // (100) 50 / 43, 400x200 (169) 60 / 54, channel 777x389 (190) 58 / 58, 512x256
-// (256) 70 / 69, channel 1000x500 (300) 76 / 86, 1200x600 (1444) 287 / 311.
+// (256) 70 / 69, channel 1000x500 (300) 76 / 86, 1200x600 (1444) 287 / 311;
+// strict HLL 48x24 59 / 31, 400x200 87 / 77, channel 777x389 81 / 79, channel
+// 1000x500 106 / 118, 1200x600 442 / 479, channel 2048x1024 (1114) 326 / 369.
 constexpr int FINE_PARENTS = 256;
 
 // The 16x8 tiles of a case's device steps (ibtfo_advance, ibtfo_step; the
-// row bands of the host-array step and batches keep the case's tiles): for
-// fp64_fast on grids of few tiles, and for the strict sweeps and the PVRS
-// solvers on every grid (32x8 / 16x8: strict HLL 48x24 41 / 31, 400x200 84 / 76,
-// 1200x600 511 / 482, channel 2048x1024 386 / 376 us per step; PVRS 1200x600
-// 2238 / 1889).  0, 2 (allocation) or 5 (CUDA error)
+// row bands of the host-array step and batches keep the case's tiles): on
+// grids of few tiles, and with the PVRS solvers, whose tiles are 32x8, on every
+// grid (1200x600, 32x8 / 16x8: 2238 / 1889 us per step).  0, 2 (allocation) or 5 (CUDA error)
 static int make_fine(ibtfo_case *c)
 {
     for (void *p : {(void *)c->fine_tiles, (void *)c->fine_slot, (void *)c->fine_partial})
@@ -755,8 +753,7 @@ static int make_fine(ibtfo_case *c)
     const GridDesc &g = c->g;
     std::vector<unsigned> parents, fine;
     int rc = active_tile_list(g, c->type, TILE_X, FAST_TILE_Y, parents, c->stream);
-    const bool fast = c->cfg.precision == IBTFO_PRECISION_FP64_FAST && c->cfg.riemann != IBTFO_RIEMANN_PVRS;
-    if (rc || (fast && parents.size() > FINE_PARENTS))
+    if (rc || (c->cfg.riemann != IBTFO_RIEMANN_PVRS && parents.size() > FINE_PARENTS))
         return rc;
     rc = active_tile_list(g, c->type, FINE_X, FINE_Y, fine, c->stream);
     if (rc)

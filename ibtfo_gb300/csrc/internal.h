@@ -219,9 +219,9 @@ typedef void (*SweepLaunch)(const SweepArgs &, int grid, cudaStream_t s);
 // sweep tile (interior cells per CTA)
 constexpr int TILE_X = 32;
 constexpr int TILE_Y = 8;
-// Rows of the fp64_fast sweep's tiles (not with the PVRS solvers, whose 158
+// Rows of the FP64 sweeps' tiles (not with the PVRS solvers, whose 158
 // registers leave room for one 32x8 tile per SM at most): a 32x16 tile solves
-// 2.16 faces per cell where a 32x8 tile solves 2.28, and stages 1.41 cells
+// 2.09 faces per cell where a 32x8 tile solves 2.28, and stages 1.41 cells
 // per cell, not 1.69.  Every sweep CTA has TILE_X x TILE_Y threads.
 constexpr int FAST_TILE_Y = 16;
 // The FP64 sweeps' small tiles (capi.cu, make_fine): a 16x8 tile's 280 faces

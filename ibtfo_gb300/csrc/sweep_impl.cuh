@@ -610,12 +610,15 @@ constexpr int sweep_ctas()
         return 1;
     if (TX == FINE_X)
         return 5;
-    return (FAST && (RIE == HLL || RIE == SW)) ? 3 : 1;
+    return 3;
 }
 
-// one case: one CTA per active tile of TX x TY cells.  fp64_fast with HLL or
-// Steger-Warming: 32x16 tiles in 85 registers (3 CTAs per SM, 59 KB of
-// shared memory each), which measured 4% faster than 512 threads per tile.
+// one case: one CTA per active tile of TX x TY cells.  32x16 tiles in 80
+// registers (3 CTAs per SM, 59 KB of shared memory each): with fp64_fast HLL
+// 4% faster than 512 threads per tile; HLL_Toro, which had two CTAs of 106
+// registers, spills 16 bytes and gains 3% (vortex 1024^2 MHM + RK2 9.47 ->
+// 9.15 ms for eight steps, a sixth of it from calls in place of if-converted
+// rare paths); the strict form: capi.cu, FINE_PARENTS.
 template <int SCH, int RIE, int LIM, int FAST, int TX, int TY>
 __global__ void __launch_bounds__(sweep_threads<TX>(), sweep_ctas<RIE, FAST, TX>())
     sweep_kernel(const __grid_constant__ SweepArgs a)
@@ -688,7 +691,7 @@ SweepLaunch prepared_sweep_launcher()
 template <int SCH, int RIE, int FAST>
 SweepLaunch select_sweep_tile(bool vl, bool fine)
 {
-    constexpr int TY = (FAST && RIE != PVRS) ? FAST_TILE_Y : TILE_Y;
+    constexpr int TY = (RIE != PVRS) ? FAST_TILE_Y : TILE_Y;
     if (fine)
         return vl ? prepared_sweep_launcher<SCH, RIE, VANLEER, FAST, FINE_X, FINE_Y>()
                   : prepared_sweep_launcher<SCH, RIE, MINMOD, FAST, FINE_X, FINE_Y>();
