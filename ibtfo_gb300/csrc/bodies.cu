@@ -122,10 +122,10 @@ __global__ void x_split_init_kernel(GridDesc g, const uint8_t *__restrict__ type
     double4 u = (x < x_split) ? L : R;
     if (type[o] == 1)
         u = make_double4(-1.0, 0.0, 0.0, -1.0);
-    state_st(buf, 0, o, u.x, g);
-    state_st(buf, 1, o, u.y, g);
-    state_st(buf, 2, o, u.z, g);
-    state_st(buf, 3, o, u.w, g);
+    state_st_bulk(buf, 0, o, u.x, g);
+    state_st_bulk(buf, 1, o, u.y, g);
+    state_st_bulk(buf, 2, o, u.z, g);
+    state_st_bulk(buf, 3, o, u.w, g);
 }
 
 // initial values at the corner-column sources of the Regular domain edges

@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) reduce_kernel(const ReduceArgs
         {
             double v[4];
             for (int k = 0; k < 4; k++)
-                v[k] = state_ld(a.u, k, o, g);
+                v[k] = state_ld_bulk(a.u, k, o, g);
             cell_stats(v, g.gamma, g.dx, g.dy, cs, cs.mass);
         }
         else if (a.type[o] == CELL_CUT && a.alpha)
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) reduce_kernel(const ReduceArgs
             // (smaller cells are mixed with their neighbours)
             double v[4];
             for (int k = 0; k < 4; k++)
-                v[k] = state_ld(a.u, k, o, g);
+                v[k] = state_ld_bulk(a.u, k, o, g);
             CellStats c1;
             cell_stats(v, g.gamma, g.dx, g.dy, c1, c1.mass);
             cs.mass += a.alpha[o] * c1.mass;
@@ -478,39 +478,80 @@ void launch_reduce(const ReduceArgs &a, int, cudaStream_t s)
 
 // ---------------------------------------------------------------- layouts
 
-__global__ void aos_to_soa_kernel(const double *__restrict__ aos, double *__restrict__ soa, GridDesc g)
+// one cell of a host-layout array: two 16-byte accesses where the array allows
+// (page-locked host memory written over the host link moves in whole sectors)
+__device__ __forceinline__ void load_aos_cell(const double *aos, long long c, double v[4])
 {
-    long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (long long)g.M * g.N)
-        return;
-    int j = (int)(c / g.M), i = (int)(c - (long long)j * g.M);
-    long long o = (long long)j * g.pitch + i;
-    for (int k = 0; k < 4; k++)
-        state_st(soa, k, o, aos[c * 4 + k], g);
+    const double *p = aos + c * 4;
+    if ((reinterpret_cast<uintptr_t>(aos) & 15) == 0)
+    {
+        const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+        v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+    }
+    else
+        for (int k = 0; k < 4; k++)
+            v[k] = p[k];
+}
+__device__ __forceinline__ void store_aos_cell(double *aos, long long c, const double v[4])
+{
+    double *p = aos + c * 4;
+    if ((reinterpret_cast<uintptr_t>(aos) & 15) == 0)
+    {
+        reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
+    }
+    else
+        for (int k = 0; k < 4; k++)
+            p[k] = v[k];
 }
 
-__global__ void soa_to_aos_kernel(const double *__restrict__ soa, double *__restrict__ aos, GridDesc g)
+// Whole arrays.  The conversions' FP64 time bound them: with the pairs of the
+// FP32 form made and read on the integer pipes (pair32.cuh), 16-byte accesses
+// and a row of blocks per array row (no 64-bit division per cell) 2048^2 cells
+// go in in 36 us, not 123 (7.4 TB/s of the traffic, part of it still in L2),
+// and out in 79, not 93; 4096^2 through ibtfo_set_state 4.36 -> 4.00 ms, of
+// which the host link takes 2.6.
+__global__ void __launch_bounds__(256) aos_to_soa_kernel(const double *__restrict__ aos, double *__restrict__ soa,
+                                                         GridDesc g)
 {
-    long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (long long)g.M * g.N)
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= g.M)
         return;
-    int j = (int)(c / g.M), i = (int)(c - (long long)j * g.M);
-    long long o = (long long)j * g.pitch + i;
-    for (int k = 0; k < 4; k++)
-        aos[c * 4 + k] = state_ld(soa, k, o, g);
+    for (int j = blockIdx.y; j < g.N; j += gridDim.y)
+    {
+        double v[4];
+        load_aos_cell(aos, (long long)j * g.M + i, v);
+        for (int k = 0; k < 4; k++)
+            state_st_bulk(soa, k, (long long)j * g.pitch + i, v[k], g);
+    }
 }
+
+__global__ void __launch_bounds__(256) soa_to_aos_kernel(const double *__restrict__ soa, double *__restrict__ aos,
+                                                         GridDesc g)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= g.M)
+        return;
+    for (int j = blockIdx.y; j < g.N; j += gridDim.y)
+    {
+        double v[4];
+        for (int k = 0; k < 4; k++)
+            v[k] = state_ld_bulk(soa, k, (long long)j * g.pitch + i, g);
+        store_aos_cell(aos, (long long)j * g.M + i, v);
+    }
+}
+
+static dim3 row_blocks(const GridDesc &g) { return dim3((g.M + 255) / 256, g.N < 65535 ? g.N : 65535); }
 
 void launch_aos_to_soa(const double *aos, double *soa, const GridDesc &g, cudaStream_t s)
 {
-    long long n = (long long)g.M * g.N;
-    aos_to_soa_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(aos, soa, g);
+    aos_to_soa_kernel<<<row_blocks(g), 256, 0, s>>>(aos, soa, g);
     count_launch();
 }
 
 void launch_soa_to_aos(const double *soa, double *aos, const GridDesc &g, cudaStream_t s)
 {
-    long long n = (long long)g.M * g.N;
-    soa_to_aos_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(soa, aos, g);
+    soa_to_aos_kernel<<<row_blocks(g), 256, 0, s>>>(soa, aos, g);
     count_launch();
 }
 
@@ -575,21 +616,6 @@ __global__ void cur_rows_to_aos_kernel(const double *b0, const double *b1, const
     long long o = (long long)j * g.pitch + i;
     for (int k = 0; k < 4; k++)
         aos[c * 4 + k] = state_ld(soa, k, o, g);
-}
-
-// one cell of a host-layout array: two 16-byte stores where the array allows
-// (page-locked host memory written over the host link moves in whole sectors)
-__device__ __forceinline__ void store_aos_cell(double *aos, long long c, const double v[4])
-{
-    double *p = aos + c * 4;
-    if ((reinterpret_cast<uintptr_t>(aos) & 15) == 0)
-    {
-        reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
-        reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
-    }
-    else
-        for (int k = 0; k < 4; k++)
-            p[k] = v[k];
 }
 
 __global__ void snapshot_rows_to_aos_kernel(const double *b0, const double *b1, const DevState *__restrict__ st,

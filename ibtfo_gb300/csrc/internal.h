@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "int64math.cuh"
+#include "pair32.cuh"
 
 namespace ibtfo {
 
@@ -109,6 +110,32 @@ __device__ __forceinline__ void state_st(double *b, int k, long long o, double v
         const float hi = (float)v;
         f[k * g.plane + o] = hi;
         f[(4 + k) * g.plane + o] = (float)(v - (double)hi);
+        return;
+    }
+    b[k * g.plane + o] = v;
+}
+// The same for kernels over whole arrays, which the conversions' FP64 time
+// would bound (pair32.cuh).  Not for the boundary pass: its few cells wait on
+// a chain of operations, which the integer form lengthens (eight served
+// requests 62.9 -> 64.2 ms).
+__device__ __forceinline__ double state_ld_bulk(const double *b, int k, long long o, const GridDesc &g)
+{
+    if (g.f32)
+    {
+        const float *f = reinterpret_cast<const float *>(b);
+        return widen(f[k * g.plane + o]) + widen(f[(4 + k) * g.plane + o]);
+    }
+    return b[k * g.plane + o];
+}
+__device__ __forceinline__ void state_st_bulk(double *b, int k, long long o, double v, const GridDesc &g)
+{
+    if (g.f32)
+    {
+        float *f = reinterpret_cast<float *>(b);
+        float hi, lo;
+        split_pair(v, hi, lo);
+        f[k * g.plane + o] = hi;
+        f[(4 + k) * g.plane + o] = lo;
         return;
     }
     b[k * g.plane + o] = v;

@@ -240,6 +240,42 @@ __device__ __forceinline__ double tile_mass_16x8(double v)
            ((part[1][0] + part[1][1]) + (part[1][2] + part[1][3]));
 }
 
+// The sum of 256 threads' values: per warp, lanes 16 apart, then 8, 4, 2, 1;
+// then the warps in order (thread 0 receives it).  The partial sums are
+// gathered after each level, so that a level takes as many FP64 warp
+// instructions as it has sums (16 for the block; 47 with every lane of every
+// warp adding at every level).
+__device__ __forceinline__ double block_sum_256(double v)
+{
+    __shared__ double part[256];
+    const int t = threadIdx.x;
+    part[t] = v;
+    __syncthreads();
+    if (t < 128)
+        v = part[(t >> 4) * 32 + (t & 15)] + part[(t >> 4) * 32 + (t & 15) + 16];
+    __syncthreads();
+    if (t < 128)
+        part[t] = v;
+    __syncthreads();
+    if (t < 64)
+        v = part[(t >> 3) * 16 + (t & 7)] + part[(t >> 3) * 16 + (t & 7) + 8];
+    __syncthreads();
+    if (t < 64)
+        part[t] = v;
+    __syncthreads();
+    if (t < 32)
+    {
+        v = part[(t >> 2) * 8 + (t & 3)] + part[(t >> 2) * 8 + (t & 3) + 4];
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        double m = v; // lane 4 w: the sum of warp w
+        for (int w = 1; w < 8; w++)
+            m += __shfl_sync(0xffffffffu, v, 4 * w);
+        v = m;
+    }
+    return v;
+}
+
 // Block-wide FP64 reduction of the per-thread statistics, then
 // block_commit_finalize.  CELLS: the warps that hold updated cells come first
 // (a block with more threads than cells).
@@ -267,6 +303,9 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
         m = tile_mass_16x8(cs.mass);
     if constexpr (!TREE && TX * TY > NT)
         cs.mass += cs.mass_upper;
+    constexpr bool GATHER = !TREE && NT == 256 && NW == 8;
+    if constexpr (GATHER)
+        m = block_sum_256(cs.mass);
     if (wid < NW)
     {
 #pragma unroll
@@ -276,7 +315,7 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
             cs.a2max = max_nonneg(cs.a2max, __shfl_xor_sync(0xffffffffu, cs.a2max, o));
             cs.umax = max_nonneg(cs.umax, __shfl_xor_sync(0xffffffffu, cs.umax, o));
             cs.vmax = max_nonneg(cs.vmax, __shfl_xor_sync(0xffffffffu, cs.vmax, o));
-            if (!TREE)
+            if (!TREE && !GATHER)
                 cs.mass += __shfl_xor_sync(0xffffffffu, cs.mass, o);
             cs.nans += __shfl_xor_sync(0xffffffffu, cs.nans, o);
         }
@@ -298,7 +337,7 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
         double a2 = red[4][0];
         a = red[0][0], u = red[1][0], v = red[2][0];
         n = rnan[0];
-        if (!TREE)
+        if (!TREE && !GATHER)
             m = red[3][0];
         for (int w = 1; w < NW; w++)
         {
@@ -306,7 +345,7 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
             a2 = max_nonneg(a2, red[4][w]);
             u = max_nonneg(u, red[1][w]);
             v = max_nonneg(v, red[2][w]);
-            if (!TREE)
+            if (!TREE && !GATHER)
                 m += red[3][w];
             n += rnan[w];
         }
