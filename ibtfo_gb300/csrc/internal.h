@@ -252,7 +252,7 @@ constexpr int TILE_Y = 8;
 // per cell, not 1.69.  Every sweep CTA has TILE_X x TILE_Y threads.
 constexpr int FAST_TILE_Y = 16;
 // The FP64 sweeps' small tiles (capi.cu, make_fine): a 16x8 tile's 280 faces
-// are two passes of 160 threads, five CTAs per SM in 80 registers
+// are two passes of 160 threads, five CTAs per SM in 72 registers
 constexpr int FINE_X = 16, FINE_Y = 8, FINE_THREADS = 160;
 
 // A tile-list entry: the tile's column index in bits 0-15, its row index in

@@ -21,9 +21,10 @@
 //   are formed from the FP32 face states.
 // Two faces are solved at once in packed FP32 arithmetic (one instruction for
 // two operations, each half rounding as the single one does): a third fewer
-// instructions (vortex 2048^2: 158.7 M -> 108.4 M warp instructions a sweep).
+// instructions (vortex 2048^2, first stage: 158.7 M -> 110.5 M warp instructions).
 // The bits are those of the single form.  The gain in time is smaller, since
-// the registers of two faces leave 15 warps per SM, not 24.  With the staging
+// the registers of two faces leave 15 warps per SM, not 24 (issue slots used 69%
+// -> 51%).  With the staging
 // of sweep_tile32_delta, per step: cylinder 1800x1100 MUSCL + RK2 214-216 ->
 // 192-197 us, vortex MHM + RK2 2048^2 460 -> 449 us, 4096^2 1.70 -> 1.65 ms.
 // The algorithm is HLL_Toro's (MUSCL / MHM / Godunov reconstruction with the

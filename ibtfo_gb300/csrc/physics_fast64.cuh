@@ -1,9 +1,10 @@
 // The fp64_fast faces: the algorithms of physics_fast.cuh in the fewest FP64
 // instructions.
 //
-// What bounds the FP64 sweeps is the FP64 pipe (two thread instructions per
-// SM and clock, one sixty-fourth of the FP32 rate), so an FP64 instruction
-// costs as much as 64 integer or FP32 ones.  Three things follow:
+// What bounds the FP64 sweeps is the FP64 unit, one per SM, which takes 16
+// clocks for a warp instruction: an FP64 instruction costs as much as 64
+// integer or FP32 ones, and a partly filled warp as much as a full one.
+// Three things follow:
 //   * reciprocals and square roots are taken on the integer and FP32 pipes
 //     (int64math.cuh), which the faces leave idle;
 //   * comparisons and the positivity tests read bit patterns;
@@ -14,11 +15,12 @@
 //     where u_K - S_K is the root c_K just taken (20 instructions instead of
 //     32), and Steger-Warming's sums over the three waves are regrouped
 //     around T = 2 (gamma - 1) l1 + l3 + l4 (41 per state instead of 77).
-// Instructions per MUSCL + minmod face, reconstruction included: HLL 80
-// (121 before), Steger-Warming 102 (200 before), HLL_Toro 83 (about 165
-// before: the positivity test repeated four reciprocals).
-// Measured on GB300, ms per step: see the dispatch in capi.cu and the sweep
-// kernels of sweep_impl.cuh.
+// Channel 2048x1024, MUSCL + HLL, one sweep: 161.4 M -> 87.3 M FP64 thread
+// instructions, 372 -> 212 us, the unit busy for 82% of the active cycles.
+// Also tried: the products too on the integer pipes, exactly (four 32-bit
+// multiplies and the rounding, about 40 instructions each): the same bits, but
+// the code outgrows the instruction cache (fp64_fast 7.8 -> 8.6 ms for 32
+// steps, strict 5.5 -> 6.5 for 12).
 #pragma once
 
 #include "physics_fast.cuh"
