@@ -133,21 +133,24 @@ __device__ __forceinline__ void sweep_tile32(SweepSmem32<TX, TY> &s, const GridD
     }
     // stage the tile and its halo: one index computation per cell, four planes
     if (!staged)
-        for (int q = tid; q < WX * WY; q += NT)
     {
-        const int ly = q / WX, lx = q - ly * WX;
-        const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
-        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (gi < g.M && gj < g.N)
+        for (int q = tid; q < WX * WY; q += NT)
         {
-            const float *src = U + (long long)gj * pitch + gi;
+            const int ly = q / WX, lx = q - ly * WX;
+            const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (gi < g.M && gj < g.N)
+            {
+                const float *src = U + (long long)gj * pitch + gi;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    v[k] = src[k * P];
+            }
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                v[k] = src[k * P];
+                s.sU[k][ly][lx] = v[k];
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            s.sU[k][ly][lx] = v[k];
+        stores_before_copies(); // a batch's next tile
     }
     __syncthreads();
 
@@ -388,6 +391,7 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
             atomicOr(status, STATUS_STALL);
     }
     if (!staged)
+    {
         for (int q = tid; q < WX * WY; q += NT)
         {
             const int ly = q / WX, lx = q - ly * WX;
@@ -404,6 +408,8 @@ __device__ __forceinline__ void sweep_tile32_delta(SweepSmem32D<TX, TY> &s, cons
             for (int k = 0; k < 8; k++)
                 s.sU[k][ly][lx] = v[k];
         }
+        stores_before_copies(); // the next tile's box may come by copies
+    }
     __syncthreads();
 
     const float hx2 = s.sC[2], hy2 = s.sC[3];

@@ -463,21 +463,24 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
     // stage the tile and its halo (always inside the padded array: ng >= 2),
     // one index computation per cell for the four planes
     if (!staged)
-        for (int q = tid; q < WX * WY; q += NT)
     {
-        const int ly = q / WX, lx = q - ly * WX;
-        const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
-        double v[4] = {0.0, 0.0, 0.0, 0.0};
-        if (gi < g.M && gj < g.N)
+        for (int q = tid; q < WX * WY; q += NT)
         {
-            const double *src = U + (long long)gj * pitch + gi;
+            const int ly = q / WX, lx = q - ly * WX;
+            const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            if (gi < g.M && gj < g.N)
+            {
+                const double *src = U + (long long)gj * pitch + gi;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    v[k] = src[k * P];
+            }
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                v[k] = src[k * P];
+                s.sU[k][ly][lx] = v[k];
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            s.sU[k][ly][lx] = v[k];
+        stores_before_copies(); // a batch's next tile
     }
     __syncthreads();
 

@@ -39,6 +39,16 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
                  : "memory");
 }
 
+// Orders this thread's shared-memory stores before bulk copies that later land
+// on the same bytes: a barrier alone does not order ordinary stores against the
+// asynchronous proxy's.  A thread that staged part of a tile element-wise calls
+// it before the next barrier; in a persistent CTA the next tile's box may
+// come by a bulk copy (a batch holds cases with tensor maps and cases without).
+__device__ __forceinline__ void stores_before_copies()
+{
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // asks for one 3-D box of the tensor to be brought into L2
 __device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z)
 {
