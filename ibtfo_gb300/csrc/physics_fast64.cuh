@@ -11,7 +11,7 @@
 //   * the HLL flux takes both sides' fluxes apart, so that each velocity is
 //     multiplied once (hll_combine64: 25 instructions, 27 before), and
 //     Steger-Warming's sums over the three waves are regrouped around
-//     T = 2 (gamma - 1) l1 + l3 + l4 (41 per state instead of 77).
+//     T = 2 (gamma - 1) l1 + l3 + l4 (43 per state instead of 77).
 // Channel 2048x1024, MUSCL + HLL, one sweep: 161.4 M -> 87.3 M FP64 thread
 // instructions, 372 -> 212 us, the unit busy for 82% of the active cycles.
 // Also tried: the products too on the integer pipes, exactly (four 32-bit
@@ -179,26 +179,31 @@ __device__ __forceinline__ void hllc_toro64(const Prim64 &L, const Prim64 &R, co
 // One side of the Steger-Warming splitting (StegerWarming/Riemann_solver.cpp:
 // 173-234 X, :262-325 Y), added to F.  With L_k = lambda_k +- sqrt(lambda_k^2
 // + delta^2) (twice the reference's), T = 2 (gamma - 1) L1 + L3 + L4,
-// X = a (L4 - L3), w = rho / (4 gamma) and h - |u|^2 / 2 = a^2 / (gamma - 1):
-//   F = w (T, u_n T + X, u_t T, |u|^2 / 2 T + a^2 / (gamma - 1) (L3 + L4) + u_n X)
+// X = a (L4 - L3), w = rho / (4 gamma), k = rho |u|^2 and the internal energy
+// ei = rho a^2 / (gamma (gamma - 1)):
+//   F = (w T, u_n w T + w X, u_t w T, k/2 T/(4 gamma) + ei/4 (L3 + L4) + u_n w X)
+// Each of T, a and ei is rounded as often as in the plain form or less: ei is
+// taken from E and not from E / rho, and the two small wave speeds are added
+// first in T (a sum around L3 + L4 had 9% more error in the mass flux of one
+// side; tests/test_fast64_faces_cpu.py).
 template <int NRM, int SIGN>
 __device__ __forceinline__ void sw_split64(const double U[4], const GasConst<double> &K, double F[4])
 {
     const double ir = rcp_t(U[0]);
     const double un = U[NRM] * ir, ut = U[3 - NRM] * ir;
-    const double q2 = fma(un, un, ut * ut);          // |u|^2
-    const double e = fma(-0.5, q2, U[3] * ir);       // internal energy per unit mass
-    const double a2 = K.ggm1 * e, a = sqrt_t(a2);
+    const double k = fma(U[NRM], un, U[3 - NRM] * ut);
+    const double ei = fma(-0.5, k, U[3]);
+    const double a = sqrt_t((K.g * ir) * (K.gm1 * ei));
     const double d2 = 1e-12; // delta = 1e-6 (:193)
     auto lam = [&](double x) {
         const double r = sqrt_t(fma(x, x, d2));
         return SIGN > 0 ? x + r : x - r;
     };
     const double l1 = lam(un), l3 = lam(un - a), l4 = lam(un + a);
-    const double s = l3 + l4, T = fma(K.gm1x2, l1, s), X = a * (l4 - l3);
-    const double w = K.ig4 * U[0];
-    const double wT = w * T, wX = w * X;
-    const double g2 = fma(0.5 * q2, wT, fma(un, wX, w * (s * (K.g * e))));
+    // SIGN > 0: l3 is the small one below Mach 1; SIGN < 0: l4
+    const double T = SIGN > 0 ? fma(K.gm1x2, l1, l3) + l4 : fma(K.gm1x2, l1, l4) + l3, X = a * (l4 - l3);
+    const double t = K.ig4 * T, wT = U[0] * t, wX = (K.ig4 * U[0]) * X;
+    const double g2 = fma(0.5 * k, t, fma(un, wX, (0.25 * ei) * (l3 + l4)));
     F[0] = (SIGN > 0) ? wT : F[0] + wT;
     F[NRM] = (SIGN > 0) ? fma(un, wT, wX) : F[NRM] + fma(un, wT, wX);
     F[3 - NRM] = (SIGN > 0) ? ut * wT : fma(ut, wT, F[3 - NRM]);
