@@ -311,34 +311,35 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 3) ccm_sweep_k
         for (int k = 0; k < TY; k++)
             ncut += s.ncut[k];
         __syncthreads();
-        const double lxd = dt * g.idx, lyd = dt * g.idy, K64 = g.ggm1; // gamma (gamma - 1)
+        const double lxd = divide_rn(dt, g.by_dx), lyd = divide_rn(dt, g.by_dy);
+        const double lwd = divide_rn(dt, divisor(g.dx * g.dy)), K64 = g.ggm1; // gamma (gamma - 1)
         for (int n = tid; n < ncut; n += NT)
         {
             const int c = s.cut[n] % TX, r = s.cut[n] / TX;
             const long long o = (long long)(j0 + r) * pitch + (i0 + c);
             // FP64: the cell's full state (hi + lo in the FP32 form), apertures,
             // volume fraction and the wall
-            const double al = ca.alpha[o], ial = rcp_t(al);
+            const double al = ca.alpha[o];
+            const Divisor by_al = divisor(al);
             const double aw = ca.ax[o - 1], ae = ca.ax[o], as = ca.ay[o - pitch], an = ca.ay[o];
             const double nLx = (aw - ae) * g.dy, nLy = (as - an) * g.dx;
-            const double L2 = nLx * nLx + nLy * nLy, L = L2 > 0.0 ? sqrt_t(L2) : 0.0;
+            const CutWall wall = cut_wall(nLx, nLy);
             double W[4] = {0.0, 0.0, 0.0, 0.0};
-            if (L > 0.0)
+            if (wall.L > 0.0)
             {
-                const double iL = rcp_t(L);
                 T Uc[4], Wt[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     Uc[k] = s.sU[k][r + 2][c + 2];
                 if constexpr (PREC == 2)
-                    ccm_wall_flux<RIE>(Uc, (T)(nLx * iL), (T)(nLy * iL), K, Wt);
+                    ccm_wall_flux<RIE>(Uc, (T)wall.nx, (T)wall.ny, K, Wt);
                 else
-                    ccm_wall_flux64<RIE>(Uc, nLx * iL, nLy * iL, K, Wt);
+                    ccm_wall_flux64<RIE>(Uc, wall.nx, wall.ny, K, Wt);
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     W[k] = (double)Wt[k];
             }
-            const double lw = (lxd * g.idy) * L;
+            const double lw = lwd * wall.L;
             double v[4];
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 3) ccm_sweep_k
                 const double u0 = state_ld(Ud, k, o, g);
                 const double fx = face_term(ae, (double)s.sF[k][r + 1][c + 1]) - face_term(aw, (double)s.sF[k][r + 1][c]);
                 const double gy = face_term(an, (double)s.sG[k][r + 1][c]) - face_term(as, (double)s.sG[k][r][c]);
-                v[k] = (al * u0 - lxd * fx - lyd * gy - lw * W[k]) * ial;
+                v[k] = cut_update(by_al, u0, lxd, fx, lyd, gy, lw, W[k]);
             }
             Cell64 cl = cell64(v);
             // the floor only where no mixing follows: a small cell's swept state

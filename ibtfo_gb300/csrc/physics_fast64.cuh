@@ -401,4 +401,30 @@ __device__ __forceinline__ void ccm_wall_flux64(const double U[4], double nx, do
     W[3] = 0.0;
 }
 
+// A cut cell's wall: its length and outward unit normal, from the aperture
+// differences times the cell sides (nLx, nLy)
+struct CutWall
+{
+    double L, nx, ny;
+};
+__device__ __forceinline__ CutWall cut_wall(double nLx, double nLy)
+{
+    CutWall w{sqrt_rn(nLx * nLx + nLy * nLy), 0.0, 0.0};
+    if (w.L > 0.0)
+    {
+        const Divisor by_L = divisor(w.L);
+        w.nx = divide_rn(nLx, by_L);
+        w.ny = divide_rn(nLy, by_L);
+    }
+    return w;
+}
+
+// one component of a cut cell: (alpha U - dt/dx fx - dt/dy gy - dt/(dx dy) L W) / alpha,
+// the quotients IEEE's (a product with a rounded reciprocal adds up to an ulp)
+__device__ __forceinline__ double cut_update(const Divisor &by_alpha, double U, double lx, double fx, double ly,
+                                             double gy, double lw, double W)
+{
+    return divide_rn(by_alpha.b * U - lx * fx - ly * gy - lw * W, by_alpha);
+}
+
 } // namespace ibtfo
