@@ -109,12 +109,15 @@ __device__ __forceinline__ bool hll64(const double UL[4], const double UR[4], co
     return true;
 }
 
-// w > 2 p for w >= 0 (false where either is NaN): doubles of one sign order
-// like their bits, and doubling a normal number adds one to its exponent
+// w > 2 p for a w that is zero, normal or +Inf (not NaN): doubles of one sign
+// order like their bits, and halving a normal number takes one from its exponent
+// (w >= 0, so that the difference cannot overflow).  True for every negative
+// p, -0 and NaNs with the sign bit among them; false for p = +Inf and the
+// other NaNs.  Either way a NaN p makes the wave speed NaN.  w = +Inf counts as
+// 2^1024: not above twice a p of 2^1023 or more.
 __device__ __forceinline__ bool exceeds_twice(double w, double p)
 {
-    const long long bw = __double_as_longlong(w), bp = __double_as_longlong(p);
-    return bw > bp + 0x0010000000000000LL;
+    return __double_as_longlong(w) - 0x0010000000000000LL > __double_as_longlong(p);
 }
 
 // HLL with Toro's wave-speed estimates (hll_plain: p* >= 0, q_K = 1 for p* <= p_K)

@@ -49,7 +49,7 @@ IBTFO_DEVICE float2 split_hardware(double v) { const float h = (float)v; return 
 """
 
 
-def build(folder, program):
+def build(folder, program, *flags):
     """PRELUDE + program, compiled into `folder`."""
     cxx, nvcc = shutil.which("g++"), shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
@@ -57,7 +57,7 @@ def build(folder, program):
         pytest.skip("no host compiler or CUDA headers")
     src, exe = folder / "t.cpp", folder / "t"
     src.write_text(PRELUDE + program)
-    subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-w", "-I", cuda, "-I",
+    subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-w", *flags, "-I", cuda, "-I",
                     os.path.join(ROOT, "include"), "-I", os.path.join(ROOT, "ibtfo_gb300", "csrc"), str(src), "-o",
                     str(exe)], check=True)
     return str(exe)
