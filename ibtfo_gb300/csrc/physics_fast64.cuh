@@ -111,10 +111,10 @@ __device__ __forceinline__ bool hll64(const double UL[4], const double UR[4], co
 
 // w > 2 p for a w that is zero, normal or +Inf (not NaN): doubles of one sign
 // order like their bits, and halving a normal number takes one from its exponent
-// (w >= 0, so that the difference cannot overflow).  True for every negative
-// p, -0 and NaNs with the sign bit among them; false for p = +Inf and the
-// other NaNs.  Either way a NaN p makes the wave speed NaN.  w = +Inf counts as
-// 2^1024: not above twice a p of 2^1023 or more.
+// (w >= 0, so that the difference cannot overflow).  True for every finite
+// negative p and -0; false for p = +Inf and for NaNs without the sign bit (-Inf and
+// the other NaNs: either; the sound speed is NaN then, and the wave speed with
+// it).  w = +Inf counts as 2^1024: not above twice a p of 2^1023 or more.
 __device__ __forceinline__ bool exceeds_twice(double w, double p)
 {
     return __double_as_longlong(w) - 0x0010000000000000LL > __double_as_longlong(p);

@@ -18,7 +18,7 @@ int main()
     for (double w : {0.0, 2.2250738585072014e-308, 1.0, 1.79e308, inf})
     {
         bad += exceeds_twice(w, inf) + exceeds_twice(w, nan) + exceeds_twice(w, nan_max);
-        for (double p : {-0.0, -5e-324, -1.0, -inf, -nan, -nan_max}) bad += !exceeds_twice(w, p);
+        for (double p : {-0.0, -5e-324, -1.0, -1.79e308}) bad += !exceeds_twice(w, p);
     }
     bad += exceeds_twice(0.0, 0.0) + !exceeds_twice(inf, 8e307) + exceeds_twice(inf, 1e308) + !exceeds_twice(1.0, 0.0);
     for (int i = 0; i < 1000000; i++)
