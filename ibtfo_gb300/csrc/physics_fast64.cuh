@@ -280,7 +280,8 @@ __device__ __forceinline__ void pressure_floor64(double U[4], Cell64 &c)
     if (__double_as_longlong(f) == __double_as_longlong(c.ei))
         return;
     U[3] = (U[3] - c.ei) + f;
-    c.ei = f;
+    // a cell left NaN (a momentum that is, or E = -Inf) stays out of the CFL maximum
+    c.ei = magnitude_bits(U[3]) <= 0x7ff0000000000000LL ? f : U[3];
 }
 
 // The primitive variables of a face's pair; a pair that is not physical
