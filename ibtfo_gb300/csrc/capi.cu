@@ -164,16 +164,17 @@ struct ibtfo_case
     CUtensorMap tmap[2];        // boxes of TILE_X x tile_y cells and their halo
     unsigned *tiles = nullptr;  // active sweep tiles (TILE_X x tile_y)
     int ntiles = 0;
-    // the device steps of a small grid sweep FINE_X x FINE_Y tiles (make_fine); 0: not in use
+    // the device steps of a small grid sweep FINE_X x FINE_Y tiles (make_tiles); 0: not in use
     int nfine = 0, fine_tma = 0;
     unsigned nparents = 0;      // 32x16 tiles the fine tiles' mass sums are grouped by
     SweepLaunch fine_sweep = nullptr;
     CUtensorMap fine_tmap[2];
     unsigned *fine_tiles = nullptr, *fine_slot = nullptr;
-    double *fine_partial = nullptr;
+    double *fine_partial = nullptr; // nparents x 4
     // the same tiles in row order: the row bands of the host-array step
     unsigned *band_list = nullptr;
     int nband_list = 0;
+    void *tile_mem = nullptr; // the lists above and fine_partial: one allocation
     // cut cells (BC_CCM): volume fractions, apertures, small-cell mixing lists
     double *alpha = nullptr, *ax = nullptr, *ay = nullptr;
     MixExchange *mix_ex = nullptr;
@@ -574,8 +575,7 @@ ibtfo_status ibtfo_destroy(ibtfo_case *c)
     // device-wide synchronisation (other cases keep running)
     cudaStream_t fs = c->own ? c->own : c->stream;
     void *bufs[] = {c->buf[0], c->buf[1], c->ic, c->staging, c->phi, c->nx, c->ny, c->type, c->ghosts,
-                    c->st, c->partial, c->ring_ic, c->tiles, c->band_list, c->fine_tiles, c->fine_slot,
-                    c->fine_partial, c->alpha, c->ax, c->ay, c->mix_ex, c->mix_part,
+                    c->st, c->partial, c->ring_ic, c->tile_mem, c->alpha, c->ax, c->ay, c->mix_ex, c->mix_part,
                     c->mix_links, c->mix_e};
     for (void *p : bufs)
         if (p)
@@ -733,56 +733,98 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
 // 1000x500 106 / 118, 1200x600 442 / 479, channel 2048x1024 (1114) 326 / 369.
 constexpr int FINE_PARENTS = 256;
 
-// The 16x8 tiles of a case's device steps (ibtfo_advance, ibtfo_step; the
-// row bands of the host-array step and batches keep the case's tiles): on
-// grids of few tiles, and with the PVRS solvers, whose tiles are 32x8, on every
-// grid (1200x600, 32x8 / 16x8: 2238 / 1889 us per step).  0, 2 (allocation) or 5 (CUDA error)
-static int make_fine(ibtfo_case *c)
+// The tile lists of a case: its tiles (c->tiles), the same in row order for
+// the host-array step's bands (c->band_list, copied to `bands`), and the 16x8
+// tiles of the device steps (ibtfo_advance, ibtfo_step; the bands and batches
+// keep the case's tiles) on grids of few tiles, and with the PVRS solvers, whose
+// tiles are 32x8, on every grid (1200x600, 32x8 / 16x8: 2238 / 1889 us per step).
+// Set-up is part of every served request: the counts of all tilings come in one
+// read-back (two on a grid of many tiles of which few are active), the lists go
+// in one copy into one allocation.  0, 2 (allocation) or 5 (CUDA error)
+static int make_tiles(ibtfo_case *c, std::vector<unsigned> &bands)
 {
-    for (void *p : {(void *)c->fine_tiles, (void *)c->fine_slot, (void *)c->fine_partial})
-        if (p)
-            cudaFreeAsync(p, c->stream);
-    c->fine_tiles = c->fine_slot = nullptr;
+    if (c->tile_mem)
+        cudaFreeAsync(c->tile_mem, c->stream);
+    c->tile_mem = nullptr;
+    c->tiles = c->band_list = c->fine_tiles = c->fine_slot = nullptr;
     c->fine_partial = nullptr;
     c->nfine = 0;
-    if (c->ccm)
-        return 0;
-    c->fine_sweep = sweep_launcher(c->cfg.scheme, c->cfg.riemann, c->cfg.limiter, c->cfg.precision, true);
-    if (!c->fine_sweep)
-        return 0;
     const GridDesc &g = c->g;
-    std::vector<unsigned> parents, fine;
-    int rc = active_tile_list(g, c->type, TILE_X, FAST_TILE_Y, parents, c->stream);
-    if (rc || (c->cfg.riemann != IBTFO_RIEMANN_PVRS && parents.size() > FINE_PARENTS))
-        return rc;
-    rc = active_tile_list(g, c->type, FINE_X, FINE_Y, fine, c->stream);
+    c->fine_sweep = c->ccm ? nullptr
+                           : sweep_launcher(c->cfg.scheme, c->cfg.riemann, c->cfg.limiter, c->cfg.precision, true);
+    const Tiling own{TILE_X, c->tile_y, false}, parent{TILE_X, FAST_TILE_Y, false}, small{FINE_X, FINE_Y, false};
+    const bool pvrs = c->cfg.riemann == IBTFO_RIEMANN_PVRS;
+    std::vector<int> counts[3];
+    bool have_small = false;
+    int rc;
+    if (c->ccm)
+        rc = tile_counts(g, c->type, {own, Tiling{TILE_X, c->tile_y, true}}, counts, c->stream);
+    else if (!c->fine_sweep)
+        rc = tile_counts(g, c->type, {own}, counts, c->stream);
+    else if (pvrs)
+        rc = tile_counts(g, c->type, {own, small, parent}, counts, c->stream);
+    else if ((have_small = (long long)own.columns(g) * own.rows(g) <= 4 * FINE_PARENTS))
+        rc = tile_counts(g, c->type, {own, small}, counts, c->stream);
+    else
+        rc = tile_counts(g, c->type, {own}, counts, c->stream);
     if (rc)
         return rc;
-    // a fine tile's mass sum: places per 32x16 tile, in the order of the
-    // list, so that the total adds up as over the 32x16 tiles (mass_partial)
-    const int ntx = (g.n_x + TILE_X - 1) / TILE_X, nty = (g.n_y + FAST_TILE_Y - 1) / FAST_TILE_Y;
-    std::vector<unsigned> place((size_t)ntx * nty, 0u), slot(fine.size());
-    for (size_t q = 0; q < parents.size(); q++)
-        place[(size_t)tile_jy(parents[q]) * ntx + tile_ix(parents[q])] = (unsigned)q;
-    constexpr int PX = TILE_X / FINE_X, PY = FAST_TILE_Y / FINE_Y;
-    for (size_t q = 0; q < fine.size(); q++)
+    bands = tile_list(g, own, counts[0], true);
+    const std::vector<unsigned> tiles = c->ccm ? tile_list(g, Tiling{TILE_X, c->tile_y, true}, counts[1], false)
+                                               : tile_list(g, own, counts[0], false);
+    std::vector<unsigned> parents, fine, slot;
+    if (c->fine_sweep)
+        parents = pvrs ? tile_list(g, parent, counts[2], false) : tiles;
+    if (c->fine_sweep && (pvrs || parents.size() <= FINE_PARENTS))
     {
-        const int ix = tile_ix(fine[q]), jy = tile_jy(fine[q]);
-        slot[q] = place[(size_t)(jy / PY) * ntx + ix / PX] * (PX * PY) + (unsigned)((jy % PY) * PX + ix % PX);
+        if (!pvrs && !have_small)
+        {
+            rc = tile_counts(g, c->type, {small}, &counts[1], c->stream);
+            if (rc)
+                return rc;
+        }
+        fine = tile_list(g, small, counts[1], true);
+        // a fine tile's mass sum: places per 32x16 tile, in the order of the
+        // list, so that the total adds up as over the 32x16 tiles (mass_partial)
+        const int ntx = parent.columns(g);
+        std::vector<unsigned> place((size_t)ntx * parent.rows(g), 0u);
+        for (size_t q = 0; q < parents.size(); q++)
+            place[(size_t)tile_jy(parents[q]) * ntx + tile_ix(parents[q])] = (unsigned)q;
+        constexpr int PX = TILE_X / FINE_X, PY = FAST_TILE_Y / FINE_Y;
+        for (unsigned t : fine)
+        {
+            const int ix = tile_ix(t), jy = tile_jy(t);
+            slot.push_back(place[(size_t)(jy / PY) * ntx + ix / PX] * (PX * PY) +
+                           (unsigned)((jy % PY) * PX + ix % PX));
+        }
     }
-    const size_t n = fine.size() * sizeof(unsigned), np = parents.size() * PX * PY * sizeof(double);
-    if (cudaMallocAsync(&c->fine_tiles, n, c->stream) != cudaSuccess ||
-        cudaMallocAsync(&c->fine_slot, n, c->stream) != cudaSuccess ||
-        cudaMallocAsync(&c->fine_partial, np, c->stream) != cudaSuccess)
+    // the mass sums (zero: tiles without fluid cells have none), then the lists
+    const size_t sums = fine.empty() ? 0 : parents.size() * 4 * sizeof(double);
+    std::vector<unsigned> lists;
+    const std::vector<unsigned> *parts[] = {&tiles, &bands, &fine, &slot};
+    for (const std::vector<unsigned> *l : parts)
+        lists.insert(lists.end(), l->begin(), l->end());
+    const size_t n = lists.size() * sizeof(unsigned);
+    if (cudaMallocAsync(&c->tile_mem, sums + n, c->stream) != cudaSuccess)
         return 2;
-    if (cudaMemcpyAsync(c->fine_tiles, fine.data(), n, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-        cudaMemcpyAsync(c->fine_slot, slot.data(), n, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-        cudaMemsetAsync(c->fine_partial, 0, np, c->stream) != cudaSuccess ||
+    unsigned *u = (unsigned *)((char *)c->tile_mem + sums);
+    if ((sums && cudaMemsetAsync(c->tile_mem, 0, sums, c->stream) != cudaSuccess) ||
+        cudaMemcpyAsync(u, lists.data(), n, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
         return 5;
-    c->fine_tma = make_state_tmaps(c, FINE_X, FINE_Y, c->fine_tmap);
-    c->nparents = (unsigned)parents.size();
-    c->nfine = (int)fine.size();
+    c->tiles = u;
+    c->band_list = u + tiles.size();
+    c->ntiles = (int)tiles.size();
+    c->nband_list = (int)bands.size();
+    if (!fine.empty())
+    {
+        c->fine_tiles = c->band_list + bands.size();
+        c->fine_slot = c->fine_tiles + fine.size();
+        c->fine_partial = (double *)c->tile_mem;
+        c->fine_tma = make_state_tmaps(c, FINE_X, FINE_Y, c->fine_tmap);
+        c->nparents = (unsigned)parents.size();
+        c->nfine = (int)fine.size();
+    }
     return 0;
 }
 
@@ -812,23 +854,19 @@ static ibtfo_status geometry_from_phi(ibtfo_case *c)
     }
     else
         rc = setup_geometry(g, c->cfg.boundary, c->phi, c->nx, c->ny, c->type, &c->ghosts, &c->nghost, c->stream);
-    std::vector<unsigned> tile_list;
+    std::vector<unsigned> bands;
     if (rc == 0)
-        rc = active_tiles(g, c->type, c->tile_y, &c->band_list, &c->nband_list, c->stream, &tile_list, true);
-    if (rc == 0)
-        rc = active_tiles(g, c->type, c->tile_y, &c->tiles, &c->ntiles, c->stream, nullptr, false, c->ccm != nullptr);
-    if (rc == 0)
-        rc = make_fine(c);
+        rc = make_tiles(c, bands);
     if (rc == 0)
     {
-        make_bands(c, tile_list);
+        make_bands(c, bands);
         std::vector<GhostRec> gl(c->nghost);
         if (c->nghost && (cudaMemcpyAsync(gl.data(), c->ghosts, sizeof(GhostRec) * c->nghost, cudaMemcpyDeviceToHost,
                                           c->stream) != cudaSuccess ||
                           cudaStreamSynchronize(c->stream) != cudaSuccess))
             rc = 5;
         make_ghost_bands(c, gl);
-        make_in_boxes(c, tile_list);
+        make_in_boxes(c, bands);
         c->mirror_in = nullptr;
     }
     if (rc == 2)

@@ -297,26 +297,46 @@ __global__ void tile_counts_kernel(GridDesc g, const uint8_t *__restrict__ type,
     counts[t] = n | (interior ? TILE_COUNT_INTERIOR : 0);
 }
 
-int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, std::vector<unsigned> &list,
-                     cudaStream_t s, bool row_order, bool ccm)
+int tile_counts(const GridDesc &g, const uint8_t *d_type, std::initializer_list<Tiling> tilings,
+                std::vector<int> *counts, cudaStream_t s)
 {
-    const int ntx = (g.n_x + tx - 1) / tx, nty = (g.n_y + ty - 1) / ty;
-    const int n = ntx * nty;
+    std::vector<size_t> first;
+    size_t total = 0;
+    for (const Tiling &t : tilings)
+    {
+        first.push_back(total);
+        total += (size_t)t.columns(g) * t.rows(g);
+    }
     int *d_counts = nullptr;
-    if (cudaMallocAsync(&d_counts, sizeof(int) * n, s) != cudaSuccess)
+    if (cudaMallocAsync(&d_counts, sizeof(int) * total, s) != cudaSuccess)
         return 2;
-    tile_counts_kernel<<<nblk(n, 256), 256, 0, s>>>(g, d_type, tx, ty, ntx, nty, ccm ? 1 : 0, d_counts);
-    count_launch();
-    std::vector<int> counts(n);
-    cudaError_t e = cudaMemcpyAsync(counts.data(), d_counts, sizeof(int) * n, cudaMemcpyDeviceToHost, s);
+    size_t k = 0;
+    for (const Tiling &t : tilings)
+    {
+        const int ntx = t.columns(g), nty = t.rows(g);
+        tile_counts_kernel<<<nblk((long long)ntx * nty, 256), 256, 0, s>>>(g, d_type, t.tx, t.ty, ntx, nty,
+                                                                            t.ccm ? 1 : 0, d_counts + first[k++]);
+        count_launch();
+    }
+    std::vector<int> all(total);
+    cudaError_t e = cudaMemcpyAsync(all.data(), d_counts, sizeof(int) * total, cudaMemcpyDeviceToHost, s);
     cudaFreeAsync(d_counts, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e != cudaSuccess)
         return 5;
-    list.clear();
+    for (size_t q = 0; q < first.size(); q++)
+        counts[q].assign(all.begin() + first[q], all.begin() + (q + 1 < first.size() ? first[q + 1] : total));
+    return 0;
+}
+
+std::vector<unsigned> tile_list(const GridDesc &g, const Tiling &tiling, const std::vector<int> &counts,
+                                bool row_order)
+{
+    const int ntx = tiling.columns(g);
+    std::vector<unsigned> list;
     std::vector<int> work;
-    for (int t = 0; t < n; t++)
+    for (int t = 0; t < (int)counts.size(); t++)
         if (counts[t])
         {
             const bool interior = (counts[t] & TILE_COUNT_INTERIOR) != 0;
@@ -325,7 +345,7 @@ int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, s
         }
     if (list.empty())
         list.push_back(0u); // a tile without fluid still runs the loop accounting
-    else if (!row_order && tx == TILE_X && ty == FAST_TILE_Y)
+    else if (!row_order && tiling.tx == TILE_X && tiling.ty == FAST_TILE_Y)
     {
         // the 32x16 sweeps solve only the faces their fluid cells read, so a
         // tile's time follows its fluid count: longest first, so that the last
@@ -340,29 +360,18 @@ int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, s
             sorted[k] = list[idx[k]];
         list.swap(sorted);
     }
-    return 0;
+    return list;
 }
 
-int active_tiles(const GridDesc &g, const uint8_t *d_type, int ty, unsigned **d_tiles, int *ntiles, cudaStream_t s,
-                 std::vector<unsigned> *host_list, bool row_order, bool ccm)
+int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, std::vector<unsigned> &list,
+                     cudaStream_t s)
 {
-    std::vector<unsigned> list;
-    int rc = active_tile_list(g, d_type, TILE_X, ty, list, s, row_order, ccm);
-    if (rc)
-        return rc;
-    if (host_list)
-        *host_list = list;
-    if (*d_tiles)
-        cudaFreeAsync(*d_tiles, s);
-    *d_tiles = nullptr;
-    if (cudaMallocAsync(d_tiles, sizeof(unsigned) * list.size(), s) != cudaSuccess)
-        return 2;
-    if (cudaMemcpyAsync(*d_tiles, list.data(), sizeof(unsigned) * list.size(), cudaMemcpyHostToDevice, s) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return 5;
-    *ntiles = (int)list.size();
-    return 0;
+    const Tiling t{tx, ty, false};
+    std::vector<int> counts;
+    const int rc = tile_counts(g, d_type, {t}, &counts, s);
+    if (rc == 0)
+        list = tile_list(g, t, counts, false);
+    return rc;
 }
 
 int setup_geometry(const GridDesc &g, int bc, const double *d_phi, double *d_nx, double *d_ny, uint8_t *d_type,

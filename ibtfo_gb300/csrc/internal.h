@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cuda.h> // CUtensorMap (the tensor maps are encoded through the runtime's driver entry point)
 #include <cuda_runtime.h>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -251,7 +252,7 @@ constexpr int TILE_Y = 8;
 // 2.09 faces per cell where a 32x8 tile solves 2.28, and stages 1.41 cells
 // per cell, not 1.69.  Every sweep CTA has TILE_X x TILE_Y threads.
 constexpr int FAST_TILE_Y = 16;
-// The FP64 sweeps' small tiles (capi.cu, make_fine): a 16x8 tile's 280 faces
+// The FP64 sweeps' small tiles (capi.cu, make_tiles): a 16x8 tile's 280 faces
 // are two passes of 160 threads, five CTAs per SM in 72 registers
 constexpr int FINE_X = 16, FINE_Y = 8, FINE_THREADS = 160;
 
@@ -381,15 +382,26 @@ int vtk_writer_wait(VtkWriter *w, std::string *why);
 void vtk_writer_destroy(VtkWriter *w, cudaStream_t s);
 
 // geometry set-up (geometry.cu)
-// the tiles of TILE_X x ty cells holding fluid cells, on the device and (host_list) on the host
-int active_tiles(const GridDesc &g, const uint8_t *d_type, int ty, unsigned **d_tiles, int *ntiles, cudaStream_t s,
-                 std::vector<unsigned> *host_list = nullptr, bool row_order = false, bool ccm = false);
-// host list of the tx x ty tiles holding at least one fluid cell (bx | by << 16,
-// with TILE_INTERIOR where it applies): 32x16 tiles longest first unless
-// row_order, others in row order;
-// 0, or 2 (allocation) / 5 (CUDA error)
+// tiles of tx x ty cells over the interior; ccm: TILE_INTERIOR as in a cut-cell case
+struct Tiling
+{
+    int tx, ty;
+    bool ccm;
+    int columns(const GridDesc &g) const { return (g.n_x + tx - 1) / tx; }
+    int rows(const GridDesc &g) const { return (g.n_y + ty - 1) / ty; }
+};
+// what tile_list needs to know of each tiling's tiles, in counts[0], counts[1],
+// ...: one read-back and one synchronisation for all; 0, or 2 (allocation) / 5 (CUDA error)
+int tile_counts(const GridDesc &g, const uint8_t *d_type, std::initializer_list<Tiling> tilings,
+                std::vector<int> *counts, cudaStream_t s);
+// the tiles holding at least one fluid cell (column | row << 16, with
+// TILE_INTERIOR where it applies): 32x16 tiles longest first unless
+// row_order, others in row order
+std::vector<unsigned> tile_list(const GridDesc &g, const Tiling &tiling, const std::vector<int> &counts,
+                                bool row_order);
+// both for one tiling
 int active_tile_list(const GridDesc &g, const uint8_t *d_type, int tx, int ty, std::vector<unsigned> &list,
-                     cudaStream_t s, bool row_order = false, bool ccm = false);
+                     cudaStream_t s);
 int setup_geometry(const GridDesc &g, int bc, const double *d_phi, double *d_nx, double *d_ny, uint8_t *d_type,
                    GhostRec **d_ghosts, int *nghost, cudaStream_t s);
 
