@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(f32_threads<SCH, RIE, PREC>(), (PREC == 2 && R
             CellStats cs;
             sweep_tile64<SCH, RIE, LIM, 1, TX, TY, NT>(s, g, U, V, a.type, i0, j0, dt, cs, stage, tm, status,
                                                        interior);
-            block_reduce_finalize<NT, TX, TY>(cs, st, {a.partial, (unsigned)bc.ntiles, false, e.y}, g, true, false,
+            block_reduce_finalize<NT, TX, TY>(cs, st, {a.partial, (unsigned)bc.ntiles, 1, e.y}, g, true, false,
                                               (unsigned)bc.ntiles, stage == 1);
         }
     }

@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) reduce_kernel(const ReduceArgs
         }
     }
     const unsigned nblocks = gridDim.x * gridDim.y;
-    block_reduce_finalize<TILE_X * TILE_Y>(cs, a.st, {a.partial, nblocks, false, blockIdx.y * gridDim.x + blockIdx.x},
+    block_reduce_finalize<TILE_X * TILE_Y>(cs, a.st, {a.partial, nblocks, 1, blockIdx.y * gridDim.x + blockIdx.x},
                                            g, false, a.set_start, nblocks);
 }
 

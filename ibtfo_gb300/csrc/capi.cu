@@ -166,14 +166,15 @@ struct ibtfo_case
     int ntiles = 0;
     // the device steps of a small grid sweep FINE_X x FINE_Y tiles (make_tiles); 0: not in use
     int nfine = 0, fine_tma = 0;
-    unsigned nparents = 0;      // 32x16 tiles the fine tiles' mass sums are grouped by
+    unsigned nparents = 0;      // 32x16 tiles that group the mass sums of the FP64 sweeps
     SweepLaunch fine_sweep = nullptr;
     CUtensorMap fine_tmap[2];
     unsigned *fine_tiles = nullptr, *fine_slot = nullptr;
     double *fine_partial = nullptr; // nparents x 4
     // the same tiles in row order: the row bands of the host-array step
-    unsigned *band_list = nullptr;
+    unsigned *band_list = nullptr, *band_slot = nullptr;
     int nband_list = 0;
+    double *band_partial = nullptr; // PVRS: nparents x 2; otherwise c->partial
     void *tile_mem = nullptr; // the lists above and fine_partial: one allocation
     // cut cells (BC_CCM): volume fractions, apertures, small-cell mixing lists
     double *alpha = nullptr, *ax = nullptr, *ay = nullptr;
@@ -734,7 +735,8 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
 constexpr int FINE_PARENTS = 256;
 
 // The tile lists of a case: its tiles (c->tiles), the same in row order for
-// the host-array step's bands (c->band_list, copied to `bands`), and the 16x8
+// the host-array step's bands (c->band_list, copied to `bands`; with the FP64
+// sweeps the places of their mass sums in the device steps' order), and the 16x8
 // tiles of the device steps (ibtfo_advance, ibtfo_step; the bands and batches
 // keep the case's tiles) on grids of few tiles, and with the PVRS solvers, whose
 // tiles are 32x8, on every grid (1200x600, 32x8 / 16x8: 2238 / 1889 us per step).
@@ -746,8 +748,8 @@ static int make_tiles(ibtfo_case *c, std::vector<unsigned> &bands)
     if (c->tile_mem)
         cudaFreeAsync(c->tile_mem, c->stream);
     c->tile_mem = nullptr;
-    c->tiles = c->band_list = c->fine_tiles = c->fine_slot = nullptr;
-    c->fine_partial = nullptr;
+    c->tiles = c->band_list = c->band_slot = c->fine_tiles = c->fine_slot = nullptr;
+    c->fine_partial = c->band_partial = nullptr;
     c->nfine = 0;
     const GridDesc &g = c->g;
     c->fine_sweep = c->ccm ? nullptr
@@ -772,9 +774,24 @@ static int make_tiles(ibtfo_case *c, std::vector<unsigned> &bands)
     bands = tile_list(g, own, counts[0], true);
     const std::vector<unsigned> tiles = c->ccm ? tile_list(g, Tiling{TILE_X, c->tile_y, true}, counts[1], false)
                                                : tile_list(g, own, counts[0], false);
-    std::vector<unsigned> parents, fine, slot;
+    std::vector<unsigned> parents, fine, slot, band_slot, place;
+    const int ntx = parent.columns(g);
+    // tile (ix, jy) of a tiling with px x py tiles in a 32x16 one: the place of its
+    // mass sum, by 32x16 tile in the order of the list, so that the total adds
+    // up in one tree (mass_partial)
+    const auto place_of = [&](unsigned t, int px, int py) {
+        const int ix = tile_ix(t), jy = tile_jy(t);
+        return place[(size_t)(jy / py) * ntx + ix / px] * (px * py) + (unsigned)((jy % py) * px + ix % px);
+    };
     if (c->fine_sweep)
+    {
         parents = pvrs ? tile_list(g, parent, counts[2], false) : tiles;
+        place.assign((size_t)ntx * parent.rows(g), 0u);
+        for (size_t q = 0; q < parents.size(); q++)
+            place[(size_t)tile_jy(parents[q]) * ntx + tile_ix(parents[q])] = (unsigned)q;
+        for (unsigned t : bands)
+            band_slot.push_back(place_of(t, 1, FAST_TILE_Y / c->tile_y));
+    }
     if (c->fine_sweep && (pvrs || parents.size() <= FINE_PARENTS))
     {
         if (!pvrs && !have_small)
@@ -784,24 +801,14 @@ static int make_tiles(ibtfo_case *c, std::vector<unsigned> &bands)
                 return rc;
         }
         fine = tile_list(g, small, counts[1], true);
-        // a fine tile's mass sum: places per 32x16 tile, in the order of the
-        // list, so that the total adds up as over the 32x16 tiles (mass_partial)
-        const int ntx = parent.columns(g);
-        std::vector<unsigned> place((size_t)ntx * parent.rows(g), 0u);
-        for (size_t q = 0; q < parents.size(); q++)
-            place[(size_t)tile_jy(parents[q]) * ntx + tile_ix(parents[q])] = (unsigned)q;
-        constexpr int PX = TILE_X / FINE_X, PY = FAST_TILE_Y / FINE_Y;
         for (unsigned t : fine)
-        {
-            const int ix = tile_ix(t), jy = tile_jy(t);
-            slot.push_back(place[(size_t)(jy / PY) * ntx + ix / PX] * (PX * PY) +
-                           (unsigned)((jy % PY) * PX + ix % PX));
-        }
+            slot.push_back(place_of(t, TILE_X / FINE_X, FAST_TILE_Y / FINE_Y));
     }
     // the mass sums (zero: tiles without fluid cells have none), then the lists
-    const size_t sums = fine.empty() ? 0 : parents.size() * 4 * sizeof(double);
+    const size_t nfine_sums = fine.empty() ? 0 : parents.size() * 4, nband_sums = pvrs ? parents.size() * 2 : 0;
+    const size_t sums = (nfine_sums + nband_sums) * sizeof(double);
     std::vector<unsigned> lists;
-    const std::vector<unsigned> *parts[] = {&tiles, &bands, &fine, &slot};
+    const std::vector<unsigned> *parts[] = {&tiles, &bands, &band_slot, &fine, &slot};
     for (const std::vector<unsigned> *l : parts)
         lists.insert(lists.end(), l->begin(), l->end());
     const size_t n = lists.size() * sizeof(unsigned);
@@ -816,13 +823,16 @@ static int make_tiles(ibtfo_case *c, std::vector<unsigned> &bands)
     c->band_list = u + tiles.size();
     c->ntiles = (int)tiles.size();
     c->nband_list = (int)bands.size();
+    c->nparents = (unsigned)parents.size();
+    if (!band_slot.empty())
+        c->band_slot = c->band_list + bands.size();
+    c->band_partial = nband_sums ? (double *)c->tile_mem + nfine_sums : c->partial;
     if (!fine.empty())
     {
-        c->fine_tiles = c->band_list + bands.size();
+        c->fine_tiles = c->band_slot + band_slot.size();
         c->fine_slot = c->fine_tiles + fine.size();
         c->fine_partial = (double *)c->tile_mem;
         c->fine_tma = make_state_tmaps(c, FINE_X, FINE_Y, c->fine_tmap);
-        c->nparents = (unsigned)parents.size();
         c->nfine = (int)fine.size();
     }
     return 0;
@@ -1345,10 +1355,10 @@ ibtfo_status ibtfo_case_bytes(const ibtfo_config *k, long long *resident, long l
         r += 4 * 8 * plane;                               // Regular: initial state
     if (k->boundary == IBTFO_BOUNDARY_CCM)
         r += 3 * 8 * plane;                               // cut cells: alpha and the two apertures
-    r += plane + (long long)sizeof(DevState) + 8 * nblocks + 4 * nblocks + 2 * 2 * k->num_ghost_cell * 4 * 8;
-    // the fine tiles' lists and mass sums (FP64 precisions): a tile of 16x8 cells holds 16 bytes
+    r += plane + (long long)sizeof(DevState) + 8 * nblocks + 12 * nblocks + 2 * 2 * k->num_ghost_cell * 4 * 8;
+    // the fine tiles' lists and mass sums (FP64 precisions): a tile of 16x8 cells holds 16 bytes, with PVRS 20
     if (k->precision != IBTFO_PRECISION_FP32_COMPENSATED && k->boundary != IBTFO_BOUNDARY_CCM)
-        r += 16LL * ((k->n_x + 31) / 32 * 2) * ((k->n_y + 15) / 16 * 2);
+        r += 20LL * ((k->n_x + 31) / 32 * 2) * ((k->n_y + 15) / 16 * 2);
     // ghost records: at most every interior cell next to the outline, bounded
     // here by two layers around the domain perimeter per unit of perimeter
     if (k->boundary != IBTFO_BOUNDARY_REGULAR)
@@ -1856,6 +1866,9 @@ static ibtfo_status step_host_banded(ibtfo_case *c, const double *u_in, double *
     SweepArgs a = sweep_args(c, 0);
     a.tiles = c->band_list;
     a.nblocks = c->nband_list;
+    a.slot = c->band_slot;
+    a.nparents = c->nparents;
+    a.partial = c->band_partial;
     FillArgs f = fill_args(c);
     const bool gfm = c->cfg.boundary != IBTFO_BOUNDARY_REGULAR;
     auto finish = [&](int k) -> ibtfo_status {

@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y, PREC == 2 ? 4 : 3) ccm_sweep_k
     if constexpr (PREC == 2)
         block_reduce_finalize32<NT>(cs, st, a.partial, g, gridDim.x, blockIdx.x);
     else
-        block_reduce_finalize<NT>(cs, st, {a.partial, gridDim.x, false, blockIdx.x}, g, true, false, gridDim.x);
+        block_reduce_finalize<NT>(cs, st, {a.partial, gridDim.x, 1, blockIdx.x}, g, true, false, gridDim.x);
 }
 
 template <int SCH, int RIE, int LIM, int PREC>

@@ -158,8 +158,8 @@ struct SweepArgs
     int nblocks;             // ... and the tiles of the whole step (0: one launch, its tiles)
     int ntiles;              // tiles of this launch (sweeps of persistent CTAs; set by the launcher)
     int sms;                 // SMs of the device
-    const unsigned *slot;    // FINE_X x FINE_Y tiles: where each one's mass sum goes
-    unsigned nparents;       // ... and the 32x16 tiles they belong to
+    const unsigned *slot;    // where each tile's mass sum goes (null: in the order of the list)
+    unsigned nparents;       // ... and the 32x16 tiles the sums are grouped by
     int tma;                 // stage tiles with the tensor maps below (else element-wise loads)
     CUtensorMap tmap[2];     // buf0 / buf1 as (column, row, plane) tensors, box = tile + halo, 4 planes
 };

@@ -556,7 +556,7 @@ __device__ __forceinline__ void block_reduce_finalize32(CellStats32 cs, DevState
     if (first_stage)
     {
         __syncthreads(); // every thread of the block has stored its cells
-        block_commit_finalize<NT>(0, 0, 0, 0, 0, st, {partial, nblocks, false, bid}, g, false, false, nblocks, true);
+        block_commit_finalize<NT>(0, 0, 0, 0, 0, st, {partial, nblocks, 1, bid}, g, false, false, nblocks, true);
         return;
     }
     __shared__ float red[5][NT / 32];
@@ -601,7 +601,7 @@ __device__ __forceinline__ void block_reduce_finalize32(CellStats32 cs, DevState
         vmax = (double)fv;
         mass = ((double)h + (double)l) * g.dxdy;
     }
-    block_commit_finalize<NT>(amax, umax, vmax, mass, n, st, {partial, nblocks, false, bid}, g, true, false, nblocks);
+    block_commit_finalize<NT>(amax, umax, vmax, mass, n, st, {partial, nblocks, 1, bid}, g, true, false, nblocks);
 }
 
 // one case: one CTA per active tile of 32x16 cells (256 threads, 5 CTAs per SM;

@@ -34,22 +34,24 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *addr, doub
     atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
-// the partial mass sums a step's last block adds up: `n` of them, or with
-// `fine` those of the FINE_X x FINE_Y tiles of each 32x16 tile (lower row
-// first), which are added in the tree of tile_mass_32x16
+// the partial mass sums a step's last block adds up: `n` of them, or those of
+// `n` 32x16 tiles in `parts` parts each, which are added in the tree of
+// tile_mass_32x16: four FINE_X x FINE_Y tiles (lower row first), or two 32x8 ones
 struct MassPartials
 {
     double *p;
-    unsigned n;    // 32x16 tiles (fine), or partials
-    bool fine;
+    unsigned n;
+    int parts;
     unsigned at;   // where the block's own sum goes
 };
 
 __device__ __forceinline__ double mass_partial(const MassPartials &m, unsigned b)
 {
     const volatile double *p = m.p;
-    if (!m.fine)
+    if (m.parts == 1)
         return p[b];
+    if (m.parts == 2)
+        return p[2 * (size_t)b] + p[2 * (size_t)b + 1];
     static_assert(TILE_X == 2 * FINE_X && FAST_TILE_Y == 2 * FINE_Y, "four fine tiles in a 32x16 tile");
     const volatile double *q = p + 4 * (size_t)b;
     return (q[0] + q[1]) + (q[2] + q[3]);
@@ -186,8 +188,9 @@ __device__ __forceinline__ double max_nonneg(double m, double x)
 // The mass of a 32x16 tile, added as a tree over its 8x8 blocks: in a block
 // the columns in pairs, fours and eights, then the rows likewise; then the
 // four blocks of each half, then the halves.  A sum of the same cells swept
-// as 16x8 tiles (mass_partial) has the same bits.  Warp w holds rows w (mass)
-// and w + 8 (mass_upper), lane c column c; thread 0 receives the sum.
+// as 16x8 or 32x8 tiles (mass_partial) has the same bits.  Warp w holds rows w
+// (mass) and w + 8 (mass_upper; zero in a 32x8 tile), lane c column c; thread 0
+// receives the sum.
 __device__ __forceinline__ double tile_mass_32x16(double lower, double upper)
 {
     __shared__ double col[2][4][8], half[2];
@@ -279,7 +282,8 @@ __device__ __forceinline__ double block_sum_256(double v)
 // Block-wide FP64 reduction of the per-thread statistics, then
 // block_commit_finalize.  CELLS: the warps that hold updated cells come first
 // (a block with more threads than cells).
-template <int NT, int TX = 0, int TY = 0>
+// HALF: a 32x8 tile added as a half of a 32x16 one.
+template <int NT, int TX = 0, int TY = 0, bool HALF = false>
 __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st, const MassPartials &mp,
                                                       const GridDesc &g, bool step_accounting, bool set_start,
                                                       unsigned nblocks, bool first_stage = false)
@@ -290,7 +294,8 @@ __device__ __forceinline__ void block_reduce_finalize(CellStats cs, DevState *st
         block_commit_finalize<NT>(0, 0, 0, 0, 0, st, mp, g, false, false, nblocks, true);
         return;
     }
-    constexpr bool TREE = (TX == 32 && TY == 16 && NT == 256) || (TX == FINE_X && TY == FINE_Y);
+    static_assert(!HALF || (TX == 32 && TY == 8 && NT == 256), "rows by warps");
+    constexpr bool TREE = (TX == 32 && TY == 16 && NT == 256) || (TX == FINE_X && TY == FINE_Y) || HALF;
     constexpr int CELLS = TX * TY ? TX * TY : NT;
     constexpr int NW = (CELLS < NT ? CELLS : NT) / 32; // warps with cells
     __shared__ double red[5][NW];
@@ -692,12 +697,12 @@ __global__ void __launch_bounds__(sweep_threads<TX>(), sweep_ctas<RIE, FAST, TX>
     sweep_tile64<SCH, RIE, LIM, FAST, TX, TY, NT>(s, g, U, V, a.type, i0, j0, dt, cs, a.stage,
                                                   a.tma ? &a.tmap[cur] : nullptr, &st->status, interior);
     const unsigned nblocks = a.nblocks ? a.nblocks : gridDim.x;
-    MassPartials mp;
-    mp.p = a.partial;
-    mp.fine = (TX == FINE_X);
-    mp.n = (TX == FINE_X) ? a.nparents : nblocks;
-    mp.at = (TX == FINE_X) ? a.slot[bid] : bid;
-    block_reduce_finalize<NT, TX, TY>(cs, st, mp, g, true, false, nblocks, a.stage == 1);
+    // a tile's sum has its place by 32x16 tile in the order of the case's list,
+    // whatever tiles are swept in whatever order (the row bands of the
+    // host-array step: a.slot), so that the mass has the same bits
+    constexpr int PARTS = (TX == FINE_X) ? 4 : (RIE == PVRS) ? 2 : 1;
+    const MassPartials mp{a.partial, a.slot ? a.nparents : nblocks, a.slot ? PARTS : 1, a.slot ? a.slot[bid] : bid};
+    block_reduce_finalize<NT, TX, TY, PARTS == 2>(cs, st, mp, g, true, false, nblocks, a.stage == 1);
 }
 
 template <int SCH, int RIE, int LIM, int FAST, int TX, int TY>

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(TILE_X *TILE_Y) lax_kernel(const SweepArgs a)
             cell_stats(v, gam, g.dx, g.dy, cs, cs.mass);
     }
     const unsigned nblocks = a.nblocks ? a.nblocks : gridDim.x;
-    block_reduce_finalize<NT>(cs, st, {a.partial, nblocks, false, bid}, g, true, false, nblocks, a.stage == 1);
+    block_reduce_finalize<NT>(cs, st, {a.partial, nblocks, 1, bid}, g, true, false, nblocks, a.stage == 1);
 }
 
 void launch_lax(const SweepArgs &a, int grid, cudaStream_t s)
