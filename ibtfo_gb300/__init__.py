@@ -271,15 +271,16 @@ def fp64_pipe_rate(iters: int = 4096) -> tuple[float, float]:
 
 
 FAST_MATH = {"rcp_f64": 0, "sqrt_f64": 1, "rcp_f32": 2, "sqrt_f32": 3, "div_f64": 4, "libsqrt_f64": 5,
-             "div_f32": 6, "libsqrt_f32": 7}
+             "div_f32": 6, "libsqrt_f32": 7, "divide_rn_f64": 8, "sqrt_rn_f64": 9, "pair_hi": 10, "pair_lo": 11, "widen": 12}
 
 
 def fast_math_eval(fn: str, x) -> np.ndarray:
-    """The fast precisions' reciprocal / square root (or CUDA's IEEE ones)
-    evaluated on the GPU at the values x (float64 in and out)."""
+    """One of the sweeps' arithmetic functions (or CUDA's IEEE ones) evaluated
+    on the GPU at the values x (float64 in and out); "divide_rn_f64" takes
+    the dividends and the divisors, stacked."""
     x = np.ascontiguousarray(x, dtype=np.float64).reshape(-1)
-    y = np.empty_like(x)
-    _check(lib().ibtfo_fast_math_eval(FAST_MATH[fn], _dp(x), _dp(y), int(x.size)))
+    y = np.empty(x.size // 2 if fn == "divide_rn_f64" else x.size)
+    _check(lib().ibtfo_fast_math_eval(FAST_MATH[fn], _dp(x), _dp(y), int(y.size)))
     return y
 
 

@@ -1,6 +1,6 @@
 // Diagnostics with no reference counterpart: the FP64 pipe rate of the
-// current GPU, and an evaluator of the fp64_fast / FP32 form's reciprocal and
-// square root for error-bound tests.
+// current GPU, and an evaluator of the sweeps' reciprocals, quotients, square
+// roots and float pairs for tests.
 //
 // FP64 pipe rate.  The plain FP64 sweep is bound by the FP64 pipe rather than
 // by HBM, so its roofline denominator is the pipe's instruction rate.  The
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kThreads) fp64_fma_chains_kernel(double *sink,
         sink[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
 
-// y[i] = f(x[i]) for the function selected by `fn` (IBTFO_MATH_*)
+// y[i] = f(x[i]) for the function selected by `fn` (IBTFO_MATH_*); a quotient's divisors follow the dividends
 __global__ void fast_math_kernel(int fn, const double *__restrict__ x, double *__restrict__ y, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -64,6 +64,17 @@ __global__ void fast_math_kernel(int fn, const double *__restrict__ x, double *_
     case IBTFO_MATH_DIV_F64: r = 1.0 / v; break;
     case IBTFO_MATH_LIBSQRT_F64: r = sqrt(v); break;
     case IBTFO_MATH_DIV_F32: r = (double)(1.0f / (float)v); break;
+    case IBTFO_MATH_DIVIDE_RN_F64: r = ibtfo::divide_rn(v, ibtfo::divisor(x[(size_t)n + i])); break;
+    case IBTFO_MATH_SQRT_RN_F64: r = ibtfo::sqrt_rn(v); break;
+    case IBTFO_MATH_PAIR_HI:
+    case IBTFO_MATH_PAIR_LO:
+    {
+        float hi, lo;
+        ibtfo::split_pair(v, hi, lo);
+        r = (double)(fn == IBTFO_MATH_PAIR_HI ? hi : lo);
+        break;
+    }
+    case IBTFO_MATH_WIDEN: r = ibtfo::widen((float)v); break;
     default: r = sqrtf((float)v); break;
     }
     y[i] = r;
@@ -141,18 +152,18 @@ extern "C" ibtfo_status ibtfo_fp64_pipe_rate(int iters, double *inst_per_s, doub
 extern "C" ibtfo_status ibtfo_fast_math_eval(int fn, const double *x, double *y, int n)
 {
     using namespace ibtfo;
-    if (!x || !y || n < 1 || fn < 0 || fn > IBTFO_MATH_LIBSQRT_F32)
+    if (!x || !y || n < 1 || fn < 0 || fn > IBTFO_MATH_WIDEN)
     {
         set_last_error("ibtfo_fast_math_eval: need x, y, n >= 1 and a known function");
         return IBTFO_EINVAL;
     }
-    const size_t bytes = (size_t)n * sizeof(double);
+    const size_t bytes = (size_t)n * sizeof(double), in = (fn == IBTFO_MATH_DIVIDE_RN_F64 ? 2 : 1) * bytes;
     DevBuf dx, dy;
-    cudaError_t e = cudaMalloc(&dx.p, bytes);
+    cudaError_t e = cudaMalloc(&dx.p, in);
     if (e == cudaSuccess)
         e = cudaMalloc(&dy.p, bytes);
     if (e == cudaSuccess)
-        e = cudaMemcpy(dx.p, x, bytes, cudaMemcpyHostToDevice);
+        e = cudaMemcpy(dx.p, x, in, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
     {
         fast_math_kernel<<<(n + 255) / 256, 256>>>(fn, static_cast<const double *>(dx.p), static_cast<double *>(dy.p),

@@ -498,10 +498,12 @@ ibtfo_status ibtfo_host_free(void *p);
  * by this rate, not by HBM bandwidth. */
 ibtfo_status ibtfo_fp64_pipe_rate(int iters, double *inst_per_s, double *seconds);
 /* y[i] = f(x[i]) on the GPU for n host values (copies in and out), for
- * error-bound tests of the arithmetic the fast precisions use: their
- * reciprocal and square root (Newton-Raphson refinements of the hardware
- * estimates; the FP32 ones take x and return the result as float) and,
- * for comparison, CUDA's IEEE division and square root. */
+ * tests of the arithmetic the sweeps use: the fast precisions' reciprocal and
+ * square root (the double ones on the integer pipes; the FP32 ones take x and
+ * return the result as float), the IEEE quotient and square root on the integer
+ * pipes, the FP32 form's pairs, and, for comparison, CUDA's IEEE division and
+ * square root.  IBTFO_MATH_DIVIDE_RN_F64 has two operands: x holds n
+ * dividends, then n divisors. */
 enum {
     IBTFO_MATH_RCP_F64 = 0,     /* fp64_fast 1/x */
     IBTFO_MATH_SQRT_F64 = 1,    /* fp64_fast sqrt(x) */
@@ -510,7 +512,12 @@ enum {
     IBTFO_MATH_DIV_F64 = 4,     /* 1.0 / x, IEEE double division */
     IBTFO_MATH_LIBSQRT_F64 = 5, /* sqrt(x), CUDA's double square root */
     IBTFO_MATH_DIV_F32 = 6,     /* 1.0f / x, IEEE float division */
-    IBTFO_MATH_LIBSQRT_F32 = 7  /* sqrtf(x), CUDA's float square root */
+    IBTFO_MATH_LIBSQRT_F32 = 7, /* sqrtf(x), CUDA's float square root */
+    IBTFO_MATH_DIVIDE_RN_F64 = 8, /* x[i] / x[n + i], the strict sweeps' and the boundary pass's quotient */
+    IBTFO_MATH_SQRT_RN_F64 = 9,   /* sqrt(x), the strict sweeps' */
+    IBTFO_MATH_PAIR_HI = 10,      /* the (hi, lo) float pair of x: (float)x ... */
+    IBTFO_MATH_PAIR_LO = 11,      /* ... and (float)(x - hi) */
+    IBTFO_MATH_WIDEN = 12         /* (double)(float)x, the widening on the integer pipes */
 };
 ibtfo_status ibtfo_fast_math_eval(int fn, const double *x, double *y, int n);
 
