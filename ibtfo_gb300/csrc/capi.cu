@@ -722,7 +722,8 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
     return geometry_from_phi(c);
 }
 
-// Up to how many active 32x16 tiles the FP64 sweeps take 16x8 tiles.  A
+// Up to how many active 32x16 tiles the FP64 sweeps take 16x8 tiles, on this
+// part (152 SMs with three 32x16 CTAs each; another count would be measured again).  A
 // 32x16 CTA lasts 45 us, most of it latency, and few of them leave SMs idle;
 // four 16x8 CTAs in its place spread over the SMs but solve 5% more faces, in
 // 40 warp passes where it takes 35 (136 X and 144 Y faces do not fill their

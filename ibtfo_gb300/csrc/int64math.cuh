@@ -10,7 +10,7 @@
 //   * its exact residual against X is small, so the low 64 bits of an integer
 //     product give it (three 32-bit multiplies), and one more FP32 correction
 //     brings the estimate to 60 bits or more;
-//   * rounding that to 53 bits is within 0.503 ulp of the value (rcp_t and
+//   * rounding that to 53 bits is within 0.504 ulp (a root 0.508) of the value (rcp_t and
 //     sqrt_t of the fast precisions); where IEEE rounding is needed (the
 //     strict sweeps), the remainder of the rounded result, again exact in 64
 //     bits, says whether its neighbour is nearer.
@@ -82,7 +82,7 @@ IBTFO_DEVICE uint64_t reciprocal62(uint64_t X)
 // a biased exponent and a significand (2^52 ... 2^53) as a double's bits
 IBTFO_DEVICE uint64_t assemble(uint64_t sig, int ex) { return sig + ((uint64_t)(int64_t)(ex - 1) << 52); }
 
-// 1/x within 0.502 ulp; |x| in [2^-1021, 2^1020)
+// 1/x within half an ulp and two units of the estimate, 0.504 ulp (0.502 seen in 20 million); |x| in [2^-1021, 2^1020)
 IBTFO_DEVICE bool rcp_range(uint64_t bits) { return (unsigned)exponent_field(bits) - 2u < 2041u; }
 IBTFO_DEVICE double rcp_int(uint64_t bits)
 {
@@ -107,7 +107,7 @@ IBTFO_DEVICE uint64_t root60(uint64_t X, int odd)
     return (S << 14) + (uint64_t)(int64_t)round_int((y * d) * 0x1p-5f);
 }
 
-// sqrt(x) within 0.503 ulp; x positive and normal
+// sqrt(x) within half an ulp and two units, 0.508 ulp (0.503 seen); x positive and normal
 IBTFO_DEVICE bool sqrt_range(uint64_t bits) { return (uint32_t)(bits >> 32) - 0x00100000u < 0x7fe00000u; }
 IBTFO_DEVICE double sqrt_int(uint64_t bits)
 {

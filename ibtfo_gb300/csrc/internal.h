@@ -249,8 +249,8 @@ constexpr int TILE_X = 32;
 constexpr int TILE_Y = 8;
 // Rows of the FP64 sweeps' tiles (not with the PVRS solvers, whose 158
 // registers leave room for one 32x8 tile per SM at most): a 32x16 tile solves
-// 2.09 faces per cell where a 32x8 tile solves 2.28, and stages 1.41 cells
-// per cell, not 1.69.  Every sweep CTA has TILE_X x TILE_Y threads.
+// 2.09 faces per cell where a 32x8 tile solves 2.16, and stages 1.41 cells
+// per cell, not 1.69.  Their CTAs have TILE_X x TILE_Y threads.
 constexpr int FAST_TILE_Y = 16;
 // The FP64 sweeps' small tiles (capi.cu, make_tiles): a 16x8 tile's 280 faces
 // are two passes of 160 threads, five CTAs per SM in 72 registers
@@ -335,7 +335,7 @@ struct BatchProgress
     int iter, status, nan_cells, active;
 };
 
-// tile shapes of the batched sweep (cells per CTA; 256 threads)
+// tile shapes of the batched sweep (cells per CTA; 256 threads, in the FP32 difference form 160)
 enum BatchShape { SHAPE_32x8 = 0, SHAPE_32x16 = 1, SHAPE_64x8 = 2, SHAPE_COUNT = 3 };
 constexpr int shape_tx(int shape) { return shape == SHAPE_64x8 ? 64 : 32; }
 constexpr int shape_ty(int shape) { return shape == SHAPE_32x16 ? 16 : 8; }

@@ -34,13 +34,13 @@ struct GasConst
 template <>
 struct GasConst<double>
 {
-    double g, gm1, c1, c2, igm1, ig2;
+    double g, gm1, c1, c2;
     double g16, c1x8, c2x16; // gamma / 16, 8 c1, 16 c2
     double c1h, ggm1;        // c1 / 2, gamma (gamma - 1)
     double gm1x2, ig4;       // 2 (gamma - 1), 1/(4 gamma)
     template <typename G>
     __device__ __forceinline__ explicit GasConst(const G &d)
-        : g(d.gamma), gm1(d.gm1), c1(d.c1), c2(d.c2), igm1(d.igm1), ig2(d.ig2), g16(d.g16), c1x8(d.c1x8),
+        : g(d.gamma), gm1(d.gm1), c1(d.c1), c2(d.c2), g16(d.g16), c1x8(d.c1x8),
           c2x16(d.c2x16), c1h(d.c1h), ggm1(d.ggm1), gm1x2(d.gm1x2), ig4(d.ig4)
     {
     }

@@ -605,7 +605,7 @@ __device__ __forceinline__ void block_reduce_finalize32(CellStats32 cs, DevState
 }
 
 // one case: one CTA per active tile of 32x16 cells (256 threads, 5 CTAs per SM;
-// the difference form of HLL_Toro: 160 or 192, 3 CTAs per SM, its tile
+// the difference form of HLL_Toro: 160, 3 CTAs per SM, its tile
 // holding 61 KB of shared memory)
 template <int SCH, int RIE, int LIM>
 __global__ void __launch_bounds__(f32_threads<SCH, RIE, 2>(), RIE == HLLT ? F32_DELTA_CTAS : 5)

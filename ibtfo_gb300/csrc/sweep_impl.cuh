@@ -430,7 +430,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
     const long long P = g.plane;
     const int pitch = g.pitch;
     const int tid = threadIdx.x;
-    constexpr bool FASTPHYS = FAST || safeguarded(RIE); // faces evaluated by physics_fast.cuh
+    constexpr bool FASTPHYS = FAST || safeguarded(RIE); // faces evaluated by physics_fast64.cuh
     if (FASTPHYS && tid == 0)
     {
         s.sC[0] = dt * g.idx;
@@ -491,7 +491,7 @@ __device__ __forceinline__ void sweep_tile64(SweepSmem64<TX, TY> &s, const GridD
 
     const double gam = g.gamma;
     const GasConst<double> K(g);
-    const double hx2 = FASTPHYS ? s.sC[2] : 0.0, hy2 = FASTPHYS ? s.sC[3] : 0.0; // MHM predictor of physics_fast
+    const double hx2 = FASTPHYS ? s.sC[2] : 0.0, hy2 = FASTPHYS ? s.sC[3] : 0.0; // MHM predictor of physics_fast64.cuh
     // X faces of the tile's rows (sF rows 1..TY) and all Y faces; the X faces
     // of the row below the tile (sF row 0) follow below, where needed
     constexpr int NXF = TileFaces<TX, TY>::NXF;
@@ -746,8 +746,8 @@ SweepLaunch select_sweep_tile(bool vl, bool fine)
               : prepared_sweep_launcher<SCH, RIE, MINMOD, FAST, TILE_X, TY>();
 }
 
-// the sweep of one scheme in strict FP64 (FAST = 0: 32x8 tiles) or fp64_fast
-// (32x16, with PVRS 32x8), or over FINE_X x FINE_Y tiles
+// the sweep of one scheme in strict FP64 (FAST = 0) or fp64_fast over 32x16
+// tiles (with PVRS 32x8), or (fine) over FINE_X x FINE_Y tiles
 template <int SCH, int FAST>
 SweepLaunch select_sweep(int riemann, int limiter, bool fine)
 {

@@ -336,7 +336,7 @@ enum { IBTFO_TILE_32x8 = 0, IBTFO_TILE_32x16 = 1, IBTFO_TILE_64x8 = 2 };
 
 typedef struct ibtfo_batch_config {
     int scheme, riemann, limiter, precision; /* the kernel variant of every case */
-    int tile_shape;   /* IBTFO_TILE_*: interior cells per CTA (256 threads) */
+    int tile_shape;   /* IBTFO_TILE_*: interior cells per CTA */
     int ctas_per_sm;  /* resident CTAs per SM of the persistent sweep (0: the occupancy limit) */
     int graph_steps;  /* steps per captured graph (0: 16) */
     int time_advance; /* IBTFO_TIME_* of every case: RK2 steps are two sweeps, each followed by
