@@ -727,12 +727,14 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
 // 32x16 CTA lasts 45 us, most of it latency, and few of them leave SMs idle;
 // four 16x8 CTAs in its place spread over the SMs but solve 5% more faces, in
 // 40 warp passes where it takes 35 (136 X and 144 Y faces do not fill their
-// warps), and reduce four times.  Measured (GB300, 152 SMs; us per step, 32x16
-// / 16x8 tiles): fp64_fast 48x24 cells 44 / 24, 256x128 (64 tiles) 46 / 30, channel 600x300
-// (100) 50 / 43, 400x200 (169) 60 / 54, channel 777x389 (190) 58 / 58, 512x256
-// (256) 70 / 69, channel 1000x500 (300) 76 / 86, 1200x600 (1444) 287 / 311;
-// strict HLL 48x24 59 / 31, 400x200 87 / 77, channel 777x389 81 / 79, channel
-// 1000x500 106 / 118, 1200x600 442 / 479, channel 2048x1024 (1114) 326 / 369.
+// warps), and reduce four times.  Measured (us per step, 32x16 / 16x8 tiles,
+// HLL): fp64_fast 48x24 cells 44 / 24, 256x128 (64 tiles) 49 / 32, channel
+// 600x300 (100) 51 / 43, 400x200 (169) 63 / 58, channel 777x389 (190) 60 / 60,
+// 512x256 (256) 76 / 77, channel 1000x500 (300) 81 / 86, 1200x600 (1444) 313 /
+// 337; strict 48x24 58 / 31, 400x200 83 / 72, channel 777x389 80 / 74, 512x256
+// 97 / 103, channel 1000x500 107 / 119 in the first steps (in the developed
+// flow, whose dearest tile a 32x16 CTA takes alone, 180 / 121), 1200x600 411 /
+// 451, channel 2048x1024 (1114) 346 / 378.
 constexpr int FINE_PARENTS = 256;
 
 // The tile lists of a case: its tiles (c->tiles), the same in row order for

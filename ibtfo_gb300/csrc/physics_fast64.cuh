@@ -8,8 +8,8 @@
 //   * reciprocals and square roots are taken on the integer and FP32 pipes
 //     (int64math.cuh), which the faces leave idle;
 //   * comparisons and the positivity tests read bit patterns;
-//   * the HLL flux takes both sides' fluxes apart, so that each velocity is
-//     multiplied once (hll_combine64: 25 instructions, 27 before), and
+//   * the HLL flux is taken as a correction to one side's flux
+//     (hll_combine64: 22 instructions, 27 before), and
 //     Steger-Warming's sums over the three waves are regrouped around
 //     T = 2 (gamma - 1) l1 + l3 + l4 (43 per state instead of 77).
 // Channel 2048x1024, MUSCL + HLL, one sweep: 161.4 M -> 87.3 M FP64 thread
@@ -55,18 +55,19 @@ __device__ __forceinline__ void flux64(const Prim64 &s, double F[4])
     F[3] = (s.E + s.p) * s.un;
 }
 
-// The HLL combination of two states with wave speeds S_L = u_L - cL and S_R = u_R + cR:
-//   F = w_L F_L + w_R F_R + w_U (U_R - U_L)
-// with w_K u_K formed once.  F_K - S_K U_K = (u_K - S_K) U_K + p_K (0, 1, 0, u_K),
-// where u_K - S_K = +-c_K, would give F = A U_L + B U_R + ... in 17
-// instructions, but A and B are near c/2 and of opposite sign: each component
-// then rounds against c U and not against its own size (r.m.s. error of the mass
-// flux 38 times as large at a Mach number up to 0.03, 4 times up to 0.3).
-// TORO: the jump term is added last, which rounds no worse than the quotient
-// (S_R F_L - S_L F_R + S_R S_L (U_R - U_L)) / (S_R - S_L) in any component;
-// for the reference's HLL it is added first, as in hll_fast, whose errors it has
-// (tests/test_fast64_faces_cpu.py).
-template <int NRM, bool TORO>
+// The HLL combination of two states with wave speeds S_L < 0 < S_R, taken from
+// one state A towards the other, B: with S the wave speed on B's side and w the
+// magnitude of the one on A's side over S_R - S_L,
+//   F = F_A + w ((F_B - F_A) - S (U_B - U_A)).
+// A is the state of the larger weight, 1 - w >= 1/2 (a comparison of
+// magnitudes, and selections, on the integer pipe).  The correction is small in
+// smooth flow, so that a component rounds little beyond F_A itself: half the
+// r.m.s. error of the weighted form w_L F_L + w_R F_R + w_U (U_R - U_L) there,
+// no more at strong jumps (tests/test_fast64_faces_cpu.py), in 22 instructions
+// where that form takes 25 to 27.  A shorter one in 17, A U_L + B U_R + ... from
+// F_K - S_K U_K = +-c_K U_K + p_K (0, 1, 0, u_K), rounds against c U and not against
+// the flux (mass flux at a Mach number up to 0.03: 38 times the error).
+template <int NRM>
 __device__ __forceinline__ void hll_combine64(const Prim64 &L, const Prim64 &R, double S_L, double S_R, double F[4])
 {
     if (ge0(S_L))
@@ -76,15 +77,15 @@ __device__ __forceinline__ void hll_combine64(const Prim64 &L, const Prim64 &R, 
     else
     {
         const double inv = rcp_t(S_R - S_L);
-        const double wl = S_R * inv, wr = -(S_L * inv), wu = wl * S_L;
-        const double ql = wl * L.un, qr = wr * R.un;
-        const auto sum = [&](double d, double a, double fl, double b, double fr) {
-            return TORO ? fma(wu, d, fma(a, fl, b * fr)) : fma(a, fl, fma(b, fr, wu * d));
-        };
-        F[0] = sum(R.r - L.r, wl, L.mn, wr, R.mn);
-        F[NRM] = sum(R.mn - L.mn, wl, fma(L.mn, L.un, L.p), wr, fma(R.mn, R.un, R.p));
-        F[3 - NRM] = sum(R.mt - L.mt, ql, L.mt, qr, R.mt);
-        F[3] = sum(R.E - L.E, ql, L.E + L.p, qr, R.E + R.p);
+        const bool left = magnitude_bits(S_L) < magnitude_bits(S_R);
+        const Prim64 A = left ? L : R, B = left ? R : L;
+        const double S = left ? S_R : S_L, w = (left ? -S_L : S_R) * inv;
+        const double dm = B.mn - A.mn; // also the difference of the mass fluxes
+        const double FN = fma(A.mn, A.un, A.p), FT = A.mt * A.un, FE = (A.E + A.p) * A.un;
+        F[0] = fma(w, fma(-S, B.r - A.r, dm), A.mn);
+        F[NRM] = fma(w, fma(-S, dm, fma(B.mn, B.un, B.p) - FN), FN);
+        F[3 - NRM] = fma(w, fma(-S, B.mt - A.mt, fma(B.mt, B.un, -FT)), FT);
+        F[3] = fma(w, fma(-S, B.E - A.E, fma(B.E + B.p, B.un, -FE)), FE);
     }
 }
 
@@ -105,7 +106,7 @@ __device__ __forceinline__ bool hll64(const double UL[4], const double UR[4], co
     if (NRM == 2 && ge0(S_L))
         return false;
     const double cR = sqrt_t(qR * fma(K.c2x16, R.p, t));
-    hll_combine64<NRM, false>(L, R, S_L, R.un + cR, F);
+    hll_combine64<NRM>(L, R, S_L, R.un + cR, F);
     return true;
 }
 
@@ -135,7 +136,7 @@ __device__ __forceinline__ void hll_toro64(const Prim64 &L, const Prim64 &R, con
         cL = sqrt_t(gL * fma(K.c2, L.p, t));
     if (exceeds_twice(W, R.p))
         cR = sqrt_t(gR * fma(K.c2, R.p, t));
-    hll_combine64<NRM, true>(L, R, L.un - cL, R.un + cR, F);
+    hll_combine64<NRM>(L, R, L.un - cL, R.un + cR, F);
 }
 
 // Contact-restoring HLLC with Toro's wave speeds (hllc_toro), from the primitive variables

@@ -6,7 +6,8 @@ of rho c.  The yardstick is the plain form of each flux in binary64 with fused
 multiply-adds, whose terms are no larger than the flux and its jump.  A form
 with the same number of roundings of the same sizes has the same r.m.s. error;
 over 2000 pairs a ratio of two such errors scatters by about 4%, so 1.15 is
-allowed."""
+allowed; where pressures differ by factors a few pairs carry most of the error, and
+1.25 is."""
 from decimal import Decimal, getcontext
 
 import numpy as np
@@ -33,11 +34,18 @@ static void state(double *U, double r, double u, double t, double p)
 {
     U[0] = r, U[1] = r * u, U[2] = r * t, U[3] = p / (G - 1) + 0.5 * r * (u * u + t * t);
 }
-// two states of one gas: Mach numbers up to M, jumps up to the part `jump`
+// two states of one gas: Mach numbers up to M, jumps up to the part `jump`; jump >= 1: any
+// velocities up to M, pressures up to that ratio apart
 static void pair_of(double M, double jump, double *L, double *R)
 {
     const double r = 1 + pm(0.5), p = 1 + pm(0.5), a = std::sqrt(G * p / r), u = pm(M * a), t = pm(M * a);
     state(L, r, u, t, p);
+    if (jump >= 1)
+    {
+        const double pr = p * std::pow(jump, pm(1.0)), rr = r * std::pow(jump, 0.6 * pm(1.0)), ar = std::sqrt(G * pr / rr);
+        const double ur = pm(M * ar), tr = pm(M * ar);
+        return state(R, rr, ur, tr, pr);
+    }
     state(R, r * (1 + pm(jump)), u + pm(M * a * jump), t + pm(M * a * jump), p * (1 + pm(jump)));
 }
 struct P { double un, ut, p, gi, a; };
@@ -79,7 +87,9 @@ template <int RIE> static void go(double M, double jump, const GasConst<double> 
         solve64<1, RIE, false>(L, R, UL, UR, K, F);
         // the same face as a Y face: the same operations on exchanged components
         std::swap(UL[1], UL[2]), std::swap(UR[1], UR[2]);
-        if (solve64<2, RIE, false>(UL, UR, UL, UR, K, Y) && (Y[0] != F[0] || Y[2] != F[1] || Y[1] != F[2] || Y[3] != F[3]))
+        const bool defined = std::isfinite(W[0]); // the reference's HLL takes roots of negative numbers at strong jumps
+        if (solve64<2, RIE, false>(UL, UR, UL, UR, K, Y) && defined &&
+            (Y[0] != F[0] || Y[2] != F[1] || Y[1] != F[2] || Y[3] != F[3]))
             exit(2);
         put(F, 4), put(W, 4);
     }
@@ -138,11 +148,13 @@ def rms_errors(exact, forms):
 def test_hll_fluxes_carry_their_digits(tmp_path, key):
     exe = device_on_host.build(tmp_path, HLL)
     for mach in (0.003, 0.06, 0.3, 0.9, 2.0):
-        for jump in (1e-4, 0.02, 0.3):
+        for jump in (1e-4, 0.02, 0.3, 3.0, 100.0):
             rows = np.frombuffer(device_on_host.run(exe, key[0], mach, jump, PAIRS)).reshape(-1, 16)
+            assert np.array_equal(np.isfinite(rows[:, 8]), np.isfinite(rows[:, 12]))
+            rows = rows[np.isfinite(rows[:, 12])]
             exact = [hll_exact(dec(r[:4]), dec(r[4:8]), key == "Toro") for r in rows]
             now, plain = rms_errors(exact, (rows[:, 8:12], rows[:, 12:]))
-            assert (now <= 1.15 * plain).all(), (mach, jump, now / plain)
+            assert (now <= (1.15 if jump < 1 else 1.25) * plain).all(), (mach, jump, now / plain)
 
 
 SPLIT = HEAD + r"""
