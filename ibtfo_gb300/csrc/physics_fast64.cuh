@@ -79,7 +79,8 @@ __device__ __forceinline__ void hll_combine64(const Prim64 &L, const Prim64 &R, 
         const double inv = rcp_t(S_R - S_L);
         const bool left = magnitude_bits(S_L) < magnitude_bits(S_R);
         const Prim64 A = left ? L : R, B = left ? R : L;
-        const double S = left ? S_R : S_L, w = (left ? -S_L : S_R) * inv;
+        // (a selected negation would be an FP64 addition)
+        const double S = left ? S_R : S_L, w = magnitude(left ? S_L : S_R) * inv;
         const double dm = B.mn - A.mn; // also the difference of the mass fluxes
         const double FN = fma(A.mn, A.un, A.p), FT = A.mt * A.un, FE = (A.E + A.p) * A.un;
         F[0] = fma(w, fma(-S, B.r - A.r, dm), A.mn);
