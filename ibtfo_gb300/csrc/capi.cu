@@ -728,10 +728,10 @@ ibtfo_status ibtfo_setup_geometry(ibtfo_case *c, const double *phi)
 // four 16x8 CTAs in its place spread over the SMs but solve 5% more faces, in
 // 40 warp passes where it takes 35 (136 X and 144 Y faces do not fill their
 // warps), and reduce four times.  Measured (us per step, 32x16 / 16x8 tiles,
-// HLL): fp64_fast 48x24 cells 44 / 24, 256x128 (64 tiles) 49 / 32, channel
-// 600x300 (100) 51 / 43, 400x200 (169) 63 / 58, channel 777x389 (190) 60 / 60,
-// 512x256 (256) 76 / 77, channel 1000x500 (300) 81 / 86, 1200x600 (1444) 313 /
-// 337; strict 48x24 58 / 31, 400x200 83 / 72, channel 777x389 80 / 74, 512x256
+// HLL): fp64_fast 48x24 cells 43 / 24, 256x128 (64 tiles) 48 / 31, channel
+// 600x300 (100) 49 / 42, 400x200 (169) 62 / 56, channel 777x389 (190) 59 / 59,
+// 512x256 (256) 74 / 73, channel 1000x500 (300) 79 / 87, 1200x600 (1444) 302 /
+// 325; strict 48x24 58 / 31, 400x200 83 / 72, channel 777x389 80 / 74, 512x256
 // 97 / 103, channel 1000x500 107 / 119 in the first steps (in the developed
 // flow, whose dearest tile a 32x16 CTA takes alone, 180 / 121), 1200x600 411 /
 // 451, channel 2048x1024 (1114) 346 / 378.

@@ -54,7 +54,7 @@ constexpr int ccm_tile_rows()
     return PREC == 2 ? FAST_TILE_Y : TILE_Y;
 }
 
-// CTAs per SM: four in FP32; in FP64 three (80 registers, 28 bytes spilled)
+// CTAs per SM: four in FP32; in FP64 three (80 registers, a few spilled)
 // instead of two keep the FP64 unit fed (1024x512, 24 bodies, HLL_Toro: 24 steps
 // and the read-back 6.75 -> 6.33 ms, a tenth of it from calls in place of
 // if-converted rare paths)

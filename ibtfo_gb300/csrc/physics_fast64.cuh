@@ -12,8 +12,8 @@
 //     (hll_combine64: 22 instructions, 27 before), and
 //     Steger-Warming's sums over the three waves are regrouped around
 //     T = 2 (gamma - 1) l1 + l3 + l4 (43 per state instead of 77).
-// Channel 2048x1024, MUSCL + HLL, one sweep: 161.4 M -> 87.3 M FP64 thread
-// instructions, 372 -> 212 us, the unit busy for 82% of the active cycles.
+// Channel 2048x1024, MUSCL + HLL, one sweep: 161.4 M -> 92.7 M FP64 thread
+// instructions, 372 -> 223 us, the unit busy for 83% of the active cycles.
 // Also tried: the products too on the integer pipes, exactly (four 32-bit
 // multiplies and the rounding, about 40 instructions each): the same bits, but
 // the code outgrows the instruction cache (fp64_fast 7.8 -> 8.6 ms for 32

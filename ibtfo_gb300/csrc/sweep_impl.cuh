@@ -663,9 +663,9 @@ constexpr int sweep_ctas()
 // one case: one CTA per active tile of TX x TY cells.  32x16 tiles in 80
 // registers (3 CTAs per SM, 59 KB of shared memory each): with fp64_fast HLL
 // 4% faster than 512 threads per tile; HLL_Toro, which had two CTAs of 106
-// registers, spills 16 bytes and gains 3% (vortex 1024^2 MHM + RK2 9.47 ->
-// 9.15 ms for eight steps, a sixth of it from calls in place of if-converted
-// rare paths); the strict form: capi.cu, FINE_PARENTS.
+// registers, gains 3% (vortex 1024^2 MHM + RK2 9.47 -> 9.15 ms for eight steps
+// when it was changed, a sixth of it from calls in place of if-converted rare
+// paths); the strict form: capi.cu, FINE_PARENTS.
 template <int SCH, int RIE, int LIM, int FAST, int TX, int TY>
 __global__ void __launch_bounds__(sweep_threads<TX>(), sweep_ctas<RIE, FAST, TX>())
     sweep_kernel(const __grid_constant__ SweepArgs a)
